@@ -104,14 +104,13 @@ struct CaseView {
 
 // Workspace of the mesh-coordinate adjoint (residual.cu), allocated on its first use.
 struct NodeAdjoint {
-  void* dual_work = nullptr;  // forward workspace as dual numbers with zero tangents
   double* buf = nullptr;
   int* node_ptr = nullptr;    // node -> face-node entries (CSR over fn_idx positions)
   int* node_ent = nullptr;
   int* wall_ptr = nullptr;    // face -> cells whose nearest wall face it is
   int* wall_cell = nullptr;
   double* sweep = nullptr;    // corrected gradients: forward iterates, their cotangents, scratch
-  double* rec = nullptr;      // limited reconstruction: centroid and limiter partials
+  double* rec = nullptr;      // limited reconstruction: the limiters' centroid partials
 };
 
 #define FV_MAX_STAGES 12

@@ -197,12 +197,9 @@ __device__ __forceinline__ T bscalar(signed char kind, double value, T phi_owner
 // The face and cell formulas read the mesh geometry through an accessor: GeoPlain returns the
 // stored doubles; GeoSeed returns dual numbers whose tangent is 1 on one geometric input (one
 // component, on every face / cell or on one of them), which lets the mesh-coordinate adjoint
-// differentiate the same formulas with respect to the geometry by local forward mode.
-enum GeoFace {
-  GF_AREA = 0, GF_NORMAL = 1, GF_TP = 4, GF_TN = 7, GF_G = 10, GF_DVEC = 11, GF_SKEW = 14,
-  GF_NN2 = 17, GF_INV_ND = 18, GF_INV_DPN = 19, GF_DPN = 20, GF_DNN = 21, GF_NS = 22,
-  GF_COUNT = 31
-};
+// differentiate the closure, source and limiter formulas by local forward mode where it does not
+// write the reverse out.
+enum GeoFace { GF_AREA = 0 };
 enum GeoCell { GC_VOL = 0, GC_WD = 1, GC_INV_WD = 2, GC_INV_WD2 = 3, GC_WDG = 4, GC_COUNT = 7 };
 // Centroid seeds (not stored per-factor cotangent rows): face centroid component j of the seeded
 // face (fcomp = GF_XF + j), cell centroid component j of the seeded cell (ccomp = GC_XC + j).
@@ -326,40 +323,6 @@ struct GeoSeed {
   }
   __device__ __forceinline__ Dual area(const MeshView& m, int f) const {
     return {m.area[f], hf(GF_AREA, f)};
-  }
-  __device__ __forceinline__ Dual normal(const MeshView& m, int j, int f) const {
-    return {m.normal[(long)j * m.nf + f], hf(GF_NORMAL + j, f)};
-  }
-  __device__ __forceinline__ Dual tP(const MeshView& m, int j, int f) const {
-    return {m.tP[(long)j * m.nf + f], hf(GF_TP + j, f)};
-  }
-  __device__ __forceinline__ Dual tN(const MeshView& m, int j, int f) const {
-    return {m.tN[(long)j * m.nf + f], hf(GF_TN + j, f)};
-  }
-  __device__ __forceinline__ Dual g(const MeshView& m, int f) const { return {m.g[f], hf(GF_G, f)}; }
-  __device__ __forceinline__ Dual dvec(const MeshView& m, int j, int f) const {
-    return {m.dvec[(long)j * m.nf + f], hf(GF_DVEC + j, f)};
-  }
-  __device__ __forceinline__ Dual skew(const MeshView& m, int j, int f) const {
-    return {m.skew[(long)j * m.nf + f], hf(GF_SKEW + j, f)};
-  }
-  __device__ __forceinline__ Dual nn2(const MeshView& m, int f) const {
-    return {m.nn2[f], hf(GF_NN2, f)};
-  }
-  __device__ __forceinline__ Dual inv_nd(const MeshView& m, int f) const {
-    return {m.inv_nd[f], hf(GF_INV_ND, f)};
-  }
-  __device__ __forceinline__ Dual inv_dpn(const MeshView& m, int f) const {
-    return {m.inv_dpn[f], hf(GF_INV_DPN, f)};
-  }
-  __device__ __forceinline__ Dual dpn(const MeshView& m, int f) const {
-    return {m.dpn[f], hf(GF_DPN, f)};
-  }
-  __device__ __forceinline__ Dual dnn(const MeshView& m, int f) const {
-    return {m.dnn[f], hf(GF_DNN, f)};
-  }
-  __device__ __forceinline__ Dual ns(const MeshView& m, int jq, int f) const {
-    return {m.ns[(long)jq * m.nf + f], hf(GF_NS + jq, f)};
   }
   __device__ __forceinline__ Dual vol(const MeshView& m, int c) const {
     return {m.vol[c], hc(GC_VOL, c)};
@@ -611,9 +574,9 @@ void gg_sweeps(const MeshView& m, int sweeps, double rel, const T* Bg, T* G0, T*
 // ---------------------------------------------------------------- k_closure (SST)
 // The closure of cell c: out = (S, F1, nu_t, wall shear rate, k diffusivity, omega diffusivity,
 // F2), gw = the omega gradient with the wall-cell value imposed.
-template <class T, int DIM, class S_, class GV>
+template <class T, int DIM, class S_, class GV, class GP>
 __device__ __forceinline__ void closure_cell(const MeshView& m, const CaseView& cv, const S_& st,
-                                             const Par<T>& par, const T* G, int c, const GV& gv,
+                                             const Par<T>& par, const GP& G, int c, const GV& gv,
                                              T* out, T* gw) {
   using L = Layout<DIM, true>;
   using GT = decltype(gv.area(m, 0));
@@ -1316,10 +1279,10 @@ __global__ void __launch_bounds__(128) k_flux_tangent(MeshView m, CaseView cv, S
 // ---------------------------------------------------------------- k_sum
 // SST rows of cell c: k and omega source terms added to the face sums rk / rw, and the omega
 // wall-cell fixation (aquaflux/turbulence/sources.py:60-412, fixed_value.py:124-158).
-template <class T, int DIM, class Acc, class GV = typename GeoOf<T>::type>
+template <class T, int DIM, class Acc, class GP, class GV = typename GeoOf<T>::type>
 __device__ __forceinline__ void sst_rows(const MeshView& m, const CaseView& cv, const Acc& st,
-                                         const Par<T>& par, const T* cl, const T* G, const T* Gwi,
-                                         int c, T& rk, T& rw, const GV& gv = GV{}) {
+                                         const Par<T>& par, const GP& cl, const GP& G,
+                                         const GP& Gwi, int c, T& rk, T& rw, const GV& gv = GV{}) {
   using L = Layout<DIM, true>;
   using GT = decltype(gv.area(m, 0));
   const int nc = m.nc;
