@@ -719,6 +719,8 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   if (live) x[(long)i * B + a] = acc;
 }
 
+#include "ilu_narrow.inc.cuh"
+
 template <class V>
 __global__ void k_copy(long n, const V* a, V* b) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -777,6 +779,14 @@ struct FvIlu0 {
   int* rows_tbwd = nullptr;  // L^T order
   std::vector<int> lv_fwd, lv_bwd, lv_tfwd, lv_tbwd;
   void* work = nullptr;                      // (n * b) vector the captured sweeps run on
+  // (b > 1) narrow level sets: the forward / transposed solve as one launch (ilu_narrow.inc.cuh)
+  struct Run {
+    int4* row = nullptr;    // 2n rows in level order, forward sweep then backward
+    int4* col = nullptr;
+    int* bounds = nullptr;  // nlev + 1 offsets into row / col
+    void* rec = nullptr;    // records, renewed by each factorisation
+    int nlev = 0, nlev_fwd = 0, widest = 0, k = 0;
+  } run[2];
   bool fuse_fb = false;  // the last forward level's rows are the first backward level's (fused)
   cudaGraphExec_t apply_exec[2] = {nullptr, nullptr};  // forward / transposed solve
   cudaGraphExec_t factor_exec = nullptr;
@@ -818,6 +828,85 @@ void levels(int n, bool ascending, DepFn deps, std::vector<int>* rows, std::vect
 template <class V>
 IluView<V> view(FvIlu0* f) {
   return IluView<V>{f->n, f->b, f->ptr, f->idx, f->diag, (V*)f->val};
+}
+
+int upload_bytes(const void* h, size_t bytes, void** d, cudaStream_t s) {
+  FV_CUDA_TRY(cudaMalloc(d, std::max<size_t>(1, bytes)));
+  if (bytes) FV_CUDA_TRY(cudaMemcpyAsync(*d, h, bytes, cudaMemcpyHostToDevice, s));
+  return FV_OK;
+}
+
+int widest(const std::vector<int>& bounds) {
+  int w = 0;
+  for (size_t l = 0; l + 1 < bounds.size(); ++l) w = std::max(w, bounds[l + 1] - bounds[l]);
+  return w;
+}
+
+// The one-launch form of a solve (k_ilu_run), when every level set fits one block and the vector
+// its shared memory (here in single precision; checked for the factor's in `runs`).  Above that a
+// level has the rows to fill more SMs than one, a launch each.  `row` gives a forward (0) /
+// backward (1) row as RunView::row; a backward row's blocks are taken upwards (step 1) or down.
+template <class RowFn>
+int build_run(FvIlu0* f, int t, const std::vector<int>& fwd, const std::vector<int>& lv_fwd,
+              const std::vector<int>& bwd, const std::vector<int>& lv_bwd, const int* idx,
+              int back_step, RowFn row, cudaStream_t s) {
+  const int nf = (int)lv_fwd.size() - 1, nb = (int)lv_bwd.size() - 1;
+  FvIlu0::Run& run = f->run[t];
+  run.widest = std::max(widest(lv_fwd), widest(lv_bwd));
+  if (!run_block_size(f->b, sizeof(float)) || run.widest > run_capacity(f->b) ||
+      run_smem_bytes(f->n, f->b, nf + nb, sizeof(float)) > kRunSmem)
+    return FV_OK;
+  std::vector<int4> rows, cols;
+  for (int back = 0; back < 2; ++back)
+    for (int i : back ? bwd : fwd) {
+      const int4 d = row(back, i);
+      int c[kRunBlocks] = {0, 0, 0, 0};
+      for (int q = 0; q < kRunBlocks && q < d.y; ++q)
+        c[q] = idx[d.z + (back ? back_step : 1) * q] * f->b;
+      rows.push_back(d);
+      cols.push_back(make_int4(c[0], c[1], c[2], c[3]));
+      run.k = std::max(run.k, std::min(d.y, kRunBlocks));
+    }
+  std::vector<int> bounds(lv_fwd);
+  for (int l = 1; l <= nb; ++l) bounds.push_back(f->n + lv_bwd[l]);
+  run.nlev = nf + nb;
+  run.nlev_fwd = nf;
+  if (upload_bytes(rows.data(), sizeof(int4) * rows.size(), (void**)&run.row, s) ||
+      upload_bytes(cols.data(), sizeof(int4) * cols.size(), (void**)&run.col, s) ||
+      upload_bytes(bounds.data(), sizeof(int) * bounds.size(), (void**)&run.bounds, s))
+    return FV_ERR_CUDA;
+  FV_CUDA_TRY(cudaStreamSynchronize(s));  // the host copies end with this call
+  return FV_OK;
+}
+
+// The records of a one-launch solve from the present factor.
+template <class V>
+int pack_run(FvIlu0* f, int t, cudaStream_t s) {
+  FvIlu0::Run& run = f->run[t];
+  if (!run.row || !run_block_size(f->b, sizeof(V)) ||
+      run_smem_bytes(f->n, f->b, run.nlev, sizeof(V)) > kRunSmem)
+    return FV_OK;
+  const long lanes = 2L * f->n * run_lanes(f->b);
+  if (!run.rec) FV_CUDA_TRY(cudaMalloc(&run.rec, sizeof(V) * lanes * run_entries(f->b, run.k)));
+  k_run_pack<V><<<fv_blocks(lanes, kThreads), kThreads, 0, s>>>(
+      f->n, f->b, run.k, t != 0, run.row, t ? (const V*)f->tval : (const V*)f->val, (V*)run.rec);
+  FV_CUDA_TRY(cudaGetLastError());
+  return FV_OK;
+}
+
+inline bool runs(const FvIlu0* f, int t) { return f->run[t].rec != nullptr; }
+
+template <class V>
+int launch_run(FvIlu0* f, int t, const V* r, V* x, cudaStream_t s) {
+  const FvIlu0::Run& run = f->run[t];
+  const RunView<V> R{f->n,   run.nlev, run.nlev_fwd,        run.k,
+                     run.bounds, run.row, run.col,          (const V*)run.rec,
+                     t ? f->tidx : f->idx, t ? (const V*)f->tval : (const V*)f->val};
+  int rc = FV_OK;
+  with_block_size(f->b, [&](auto B) {
+    rc = launch_run_b<V, B()>(R, run.widest, t != 0, r, x, s);
+  });
+  return rc;
 }
 
 // Launch the level sequence of the factorization / a solve on `s` (captured into a graph once).
@@ -931,6 +1020,11 @@ int ilu_factor(FvIlu0* f, cudaStream_t s) {
                                                                       (const V*)f->val,
                                                                       (V*)f->tval);
   }
+  for (int t = 0; t < 2; ++t)
+    if (t == 0 || f->tval) {
+      int rc = pack_run<V>(f, t, s);
+      if (rc != FV_OK) return rc;
+    }
   FV_CUDA_TRY(cudaGetLastError());
   unsigned long long flag;
   FV_CUDA_TRY(cudaMemcpyAsync(&flag, f->zero_flag, sizeof(flag), cudaMemcpyDeviceToHost, s));
@@ -956,12 +1050,13 @@ int ensure_transpose(FvIlu0* f, cudaStream_t s) {
   const int n = f->n;
   Transpose T;
   build_transpose(n, n, f->h_ptr->data(), f->h_idx->data(), &T);
-  std::vector<int> rows;
+  std::vector<int> rows, rows_fwd;
   levels(n, true, [&](int i, auto&& use) {  // U^T: column i depends on rows j < i with (j, i)
     for (int q = T.ptr[i]; q < T.ptr[i + 1]; ++q)
       if (T.idx[q] < i) use(T.idx[q]);
   }, &rows, &f->lv_tfwd);
   if (upload(rows, &f->rows_tfwd, s)) return FV_ERR_CUDA;
+  rows_fwd = rows;
   levels(n, false, [&](int i, auto&& use) {  // L^T: column i depends on rows k > i with (k, i)
     for (int q = T.ptr[i]; q < T.ptr[i + 1]; ++q)
       if (T.idx[q] > i) use(T.idx[q]);
@@ -975,6 +1070,12 @@ int ensure_transpose(FvIlu0* f, cudaStream_t s) {
       for (int q = T.ptr[i]; q < T.ptr[i + 1]; ++q)
         if (T.idx[q] == i) td[i] = q;
     if (upload(td, &f->tdiag, s)) return FV_ERR_CUDA;
+    int rc = build_run(f, 1, rows_fwd, f->lv_tfwd, rows, f->lv_tbwd, T.idx.data(), -1,
+                       [&](int back, int i) {
+      return back ? make_int4(i, T.ptr[i + 1] - 1 - td[i], T.ptr[i + 1] - 1, td[i])
+                  : make_int4(i, td[i] - T.ptr[i], T.ptr[i], td[i]);
+    }, s);
+    if (rc != FV_OK) return rc;
     const long nv = (long)f->nnzb * f->b * f->b;
     const size_t vs = f->precision == 64 ? sizeof(double) : sizeof(float);
     FV_CUDA_TRY(cudaMalloc(&f->tval, vs * (size_t)nv));
@@ -985,6 +1086,8 @@ int ensure_transpose(FvIlu0* f, cudaStream_t s) {
       k_transpose_blocks<float><<<fv_blocks(nv, kThreads), kThreads, 0, s>>>(
           f->nnzb, f->b, f->tblk, (const float*)f->val, (float*)f->tval);
     FV_CUDA_TRY(cudaGetLastError());
+    rc = f->precision == 64 ? pack_run<double>(f, 1, s) : pack_run<float>(f, 1, s);
+    if (rc != FV_OK) return rc;
   }
   FV_CUDA_TRY(cudaStreamSynchronize(s));
   return FV_OK;
@@ -1009,6 +1112,7 @@ int ilu_apply(FvIlu0* f, const V* r, V* x, int transpose, cudaStream_t s) {
       fv_set_error("fv_ilu0_apply: under stream capture x must be 16-byte aligned");
       return FV_ERR_ARG;
     }
+    if (runs(f, t)) return launch_run<V>(f, t, r, x, s);
     if ((const void*)x != (const void*)r)
       FV_CUDA_TRY(cudaMemcpyAsync(x, r, sizeof(V) * n, cudaMemcpyDeviceToDevice, s));
     launch_apply_levels<V>(f, t, x, s);
@@ -1019,6 +1123,7 @@ int ilu_apply(FvIlu0* f, const V* r, V* x, int transpose, cudaStream_t s) {
     int rc = ensure_transpose(f, s);
     if (rc != FV_OK) return rc;
   }
+  if (runs(f, t)) return launch_run<V>(f, t, r, x, s);
   if (!f->apply_exec[t]) {
     int rc = capture([&](cudaStream_t cs) { launch_apply_levels<V>(f, t, w, cs); },
                      &f->apply_exec[t]);
@@ -1084,6 +1189,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
     for (int q = indptr[i]; q < diag[i]; ++q) use(indices[q]);
   }, &rows, &f->lv_fwd);
   if (upload(rows, &f->rows_fwd, s)) return FV_ERR_CUDA;
+  const std::vector<int> rows_fwd(rows);
   const size_t nf = f->lv_fwd.size();
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
@@ -1096,6 +1202,11 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   std::sort(fwd_last.begin(), fwd_last.end());
   std::sort(bwd_first.begin(), bwd_first.end());
   f->fuse_fb = b > 1 && nf > 2 && f->lv_bwd.size() > 2 && fwd_last == bwd_first;
+  int rc = build_run(f, 0, rows_fwd, f->lv_fwd, rows, f->lv_bwd, indices, 1, [&](int back, int i) {
+    return back ? make_int4(i, indptr[i + 1] - 1 - diag[i], diag[i] + 1, diag[i])
+                : make_int4(i, diag[i] - indptr[i], indptr[i], diag[i]);
+  }, s);
+  if (rc != FV_OK) return rc;
   f->h_ptr = std::make_shared<const std::vector<int>>(indptr, indptr + n + 1);
   f->h_idx = std::make_shared<const std::vector<int>>(indices, indices + nnzb);
   f->h_diag = std::make_shared<const std::vector<int>>(diag);
@@ -1127,6 +1238,12 @@ extern "C" int fv_ilu0_destroy(FvIlu0* f) {
   cudaFree(f->rows_tfwd);
   cudaFree(f->rows_tbwd);
   cudaFree(f->work);
+  for (const FvIlu0::Run& r : f->run) {
+    cudaFree(r.row);
+    cudaFree(r.col);
+    cudaFree(r.bounds);
+    cudaFree(r.rec);
+  }
   for (cudaGraphExec_t e : f->apply_exec)
     if (e) cudaGraphExecDestroy(e);
   if (f->factor_exec) cudaGraphExecDestroy(f->factor_exec);
@@ -1177,6 +1294,17 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
     rc |= copy_ints(src->rows_tfwd, n, &f->rows_tfwd, s);
     rc |= copy_ints(src->rows_tbwd, n, &f->rows_tbwd, s);
     rc |= copy_ints(src->tdiag, n, &f->tdiag, s);
+  }
+  for (int t = 0; t < 2; ++t) {
+    const FvIlu0::Run& r = src->run[t];
+    if (!r.row) continue;
+    f->run[t] = r;
+    f->run[t].row = f->run[t].col = nullptr;
+    f->run[t].bounds = nullptr;
+    f->run[t].rec = nullptr;
+    rc |= copy_ints((const int*)r.row, 8 * n, (int**)&f->run[t].row, s);
+    rc |= copy_ints((const int*)r.col, 8 * n, (int**)&f->run[t].col, s);
+    rc |= copy_ints(r.bounds, r.nlev + 1, &f->run[t].bounds, s);
   }
   if (rc == FV_OK && precision != 0) {
     const size_t vs = precision == 64 ? sizeof(double) : sizeof(float);
