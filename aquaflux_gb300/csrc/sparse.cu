@@ -394,10 +394,11 @@ __device__ __forceinline__ unsigned lg_mask() { return 0xffu << ((threadIdx.x & 
 // block), with a compile-time block size: the row's lower block, the pivot row's diagonal block and
 // each upper block it updates with are held in registers (vector loads), the diagonal block's pivot
 // rows are shuffled from the lane that owns them.  Every entry sees the scalar elimination of
-// k_ilu_factor_level in the same order, so the factors are bitwise the same.
+// k_ilu_factor_level in the same order, so the factors are bitwise the same.  For the widest levels
+// (kFactorWide), where rows enough are in flight and a fourth of a warp per row issues less.
 template <class V, int B>
 __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
-                                 unsigned long long* zero_flag) {
+                                 V* rp, unsigned long long* zero_flag) {
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;  // whole groups exit together
@@ -495,9 +496,290 @@ __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
     __syncwarp(mask);
   }
   if (live) {
+    V piv = Drow[0];
 #pragma unroll
-    for (int c = 0; c < B; ++c) D[(long)a * B + c] = Drow[c];
+    for (int c = 0; c < B; ++c) {
+      D[(long)a * B + c] = Drow[c];
+      if (c == a) piv = Drow[c];
+    }
+    rp[(long)i * B + a] = V(1) / piv;
   }
+}
+
+// ---- factorisation: a warp per block row, the row's blocks in shared memory.
+// What bounds it is the chain along a row's lower blocks, not bytes: with 8 lanes a row and every
+// block updated in place in global memory, each lower block cost five or six dependent memory round
+// trips and a merge of two index lists (fp32, b = 6, 9-27 blocks a row: 100-185 us a level set
+// whatever its width; fp64 cavity: 11.9 us a level set of 64 rows).  Here a row's blocks and columns
+// are copied in once and back once; the lower blocks' rows j are looked up by 32 lanes at once; the
+// columns of row j come in one load, each lane counting row i's columns below its own to find its
+// place; the next row j is fetched and the matching blocks' columns are read before the chain of
+// quotients, which hides them; and the matching blocks are updated side by side.  Pivots of finished rows come with their reciprocals
+// (`rp`): a quotient is a product and a correction, not a division on the chain (fp64: 192 cycles
+// for 321).
+// Lanes: for b <= 4 one per block entry (16 to a block, two blocks at a time), which keeps the
+// number of fp64 instructions, 64 cycles each, at one per elimination step; above, one per column
+// (8 to a block, four blocks at a time).
+// Every entry sees the scalar elimination of k_ilu_factor_level in the same order: bitwise the same.
+
+// x / piv: in fp64 through the pivot's reciprocal (see upper_block_solve) where the quotient is far
+// from under- and overflow (192 cycles of fp64 issue for a division's 321).
+__device__ __forceinline__ bool mid_range(double q) {
+  const int e = __double2hiint(q) & 0x7ff00000;
+  return e > 0x10000000 && e < 0x70000000;
+}
+__device__ __forceinline__ double quotient(double x, double piv, double rpiv) {
+  const double q = x * rpiv;
+  if ((__double_as_longlong(x) << 1) == 0 && isfinite(rpiv)) return q;
+  if (mid_range(q) && mid_range(x) && mid_range(rpiv)) return fma_rn(fma_rn(-q, piv, x), rpiv, q);
+  return x / piv;
+}
+__device__ __forceinline__ float quotient(float x, float piv, float) { return x / piv; }
+
+// Levels of at least this many rows take 8 lanes a row (fp32, b = 6: 131,072 rows of 6 lower blocks
+// 187 us, 490 us with a warp a row; 5,900 rows of 8-15 lower blocks 120 us, 45 us with a warp).
+constexpr int kFactorWide = 65536;
+constexpr size_t kFactorSmem = 96 * 1024;
+
+// Shared memory of one warp: the matches of one lower block, the row's columns (padded to a multiple
+// of four), the pivot row's diagonal block and reciprocals, the row's blocks.
+template <class V>
+__host__ __device__ constexpr size_t factor_warp_bytes(int cap, int bb) {
+  return (32 * 8 + (size_t)(cap + 7) / 4 * 16 + 72 * sizeof(V) + (size_t)cap * bb * sizeof(V) + 15) /
+         16 * 16;
+}
+
+template <class V, int B>
+__global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* rows, int count,
+                                                      int cap, V* rp,
+                                                      unsigned long long* zero_flag) {
+  constexpr int BB = B * B;
+  constexpr bool EM = B <= 4;            // a lane per entry
+  constexpr int SG = EM ? 16 : 8, NSG = 32 / SG;
+  extern __shared__ __align__(16) unsigned char factor_smem[];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int w = blockIdx.x * (blockDim.x / 32) + warp;
+  if (w >= count) return;  // whole warps exit together
+  int2* match = (int2*)(factor_smem + (size_t)warp * factor_warp_bytes<V>(cap, BB));
+  int* cols = (int*)(match + 32);
+  V* Us = (V*)(cols + (cap + 7) / 4 * 4);
+  V* blk = Us + 72;
+  const int i = rows[w], rb = F.ptr[i], nb = F.ptr[i + 1] - rb, nl = F.diag[i] - rb;
+  V* row = F.val + (long)rb * BB;
+  for (int k = lane; k < nb + 4; k += 32) cols[k] = k < nb ? F.idx[rb + k] : 0x7fffffff;
+#pragma unroll 4
+  for (int k = lane; k < nb * BB; k += 32) blk[k] = row[k];
+  const int e = lane & (SG - 1), sg = lane / SG;
+  const unsigned sgmask = (SG == 16 ? 0xffffu : 0xffu) << (sg * SG);
+  const bool live = e < (EM ? BB : B);
+  const int el = live ? e : 0;
+  const int a = EM ? el / B : el, c = EM ? el % B : el;  // EM: entry (a, c); else row a / column c
+  __syncwarp();
+
+  int jl = 0, dl = 0, rl = 0;  // lane's lower block: row j, its diagonal's position and its end
+  // the coming lower block's row: columns (one a lane), diagonal block and reciprocals
+  constexpr int PU = (BB + B + 31) / 32;
+  int j = 0, dj = 0, ej = 0, kcol = -1;
+  V pu[PU];
+  auto fetch = [&](int q) {
+    if (q >= nl) return;
+    if ((q & 31) == 0 && q + lane < nl) {
+      jl = cols[q + lane];
+      dl = F.diag[jl];
+      rl = F.ptr[jl + 1];
+    }
+    j = __shfl_sync(0xffffffffu, jl, q & 31);
+    dj = __shfl_sync(0xffffffffu, dl, q & 31);
+    ej = __shfl_sync(0xffffffffu, rl, q & 31);
+    kcol = dj + 1 + lane < ej ? F.idx[dj + 1 + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < PU; ++u) {
+      const int k = u * 32 + lane;
+      if (k < BB) pu[u] = F.val[(long)dj * BB + k];
+      else if (k < BB + B) pu[u] = rp[(long)j * B + k - BB];
+    }
+  };
+  // the lanes' columns of row j stored in row i too, as (position in row i, block of row j); their
+  // number
+  auto find = [&](int q, int key, int s) {
+    int lo = 0;
+    if (nb <= 64) {  // columns below the key, counted (no chain of dependent reads)
+      for (int k = 0; k < nb; k += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(cols + k);
+        lo += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
+      }
+    } else {
+      int hi = nb;
+      lo = q + 1;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cols[mid] < key) lo = mid + 1;
+        else hi = mid;
+      }
+      __syncwarp();
+    }
+    const bool found = key >= 0 && lo < nb && cols[lo] == key;
+    const unsigned mask = __ballot_sync(0xffffffffu, found);
+    if (found) match[__popc(mask & ((1u << lane) - 1))] = make_int2(lo, s);
+    __syncwarp();
+    return __popc(mask);
+  };
+  auto column = [&](int t, int m, V (&Mc)[B]) {  // column c of match t's block of row j
+    if (t < m) {
+      const V* M = F.val + (long)match[t].y * BB + c;
+#pragma unroll
+      for (int k = 0; k < B; ++k) Mc[k] = M[k * B];
+    }
+  };
+  auto update = [&](int t, int m, const V* Lq, const V (&Mc)[B]) {  // A_ik -= L_ij A_jk
+    if (t >= m) return;
+    V* A = blk + match[t].x * BB;
+    if constexpr (EM) {
+      V acc = A[el];
+#pragma unroll
+      for (int k = 0; k < B; ++k) acc -= Lq[a * B + k] * Mc[k];
+      if (live) A[e] = acc;
+    } else {
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        V acc = A[r * B + c], Lr[B];
+        load_seg<B>(Lq + r * B, Lr);
+#pragma unroll
+        for (int k = 0; k < B; ++k) acc -= Lr[k] * Mc[k];
+        if (live) A[r * B + c] = acc;
+      }
+    }
+  };
+  fetch(0);
+  for (int q = 0; q < nl; ++q) {
+    const int jq = j, s0 = dj + 1, eq = ej;
+#pragma unroll
+    for (int u = 0; u < PU; ++u)
+      if (u * 32 + lane < BB + B) Us[u * 32 + lane] = pu[u];
+    const int m = find(q, kcol, s0 + lane);  // (its barrier also makes Us visible)
+    V M0[B];
+    column(sg, m, M0);
+    fetch(q + 1);
+    // L_ij = A_ij U_jj^-1, scalar columns ascending
+    V* Lq = blk + q * BB;
+    if constexpr (EM) {
+      V x = Lq[el];
+#pragma unroll
+      for (int cb = 0; cb < B; ++cb) {
+        const V piv = Us[cb * B + cb];
+        if (piv == V(0) && lane == 0) note_zero_pivot(zero_flag, i * B, jq * B + cb);
+        if (c == cb) x = quotient(x, piv, Us[BB + cb]);
+        const V l = __shfl_sync(0xffffffffu, x, a * B + cb, SG);
+        if (cb < B - 1 && c > cb) x -= l * Us[cb * B + c];
+      }
+      __syncwarp();
+      if (live && sg == 0) Lq[e] = x;
+    } else {
+      V L[B];
+      load_seg<B>(Lq + a * B, L);
+#pragma unroll
+      for (int cb = 0; cb < B; ++cb) {
+        V Ur[B];
+        load_seg<B>(Us + cb * B, Ur);
+        const V piv = Ur[cb];
+        if (piv == V(0) && lane == 0) note_zero_pivot(zero_flag, i * B, jq * B + cb);
+        const V l = quotient(L[cb], piv, Us[BB + cb]);
+        L[cb] = l;
+#pragma unroll
+        for (int k = cb + 1; k < B; ++k) L[k] -= l * Ur[k];
+      }
+      __syncwarp();
+      if (live && sg == 0) {
+#pragma unroll
+        for (int k = 0; k < B; ++k) Lq[a * B + k] = L[k];
+      }
+    }
+    __syncwarp();
+    update(sg, m, Lq, M0);
+    for (int t = sg + NSG; t < m; t += NSG) {
+      column(t, m, M0);
+      update(t, m, Lq, M0);
+    }
+    __syncwarp();
+    for (int s = s0 + 32; s < eq; s += 32) {  // more than 32 columns in row j
+      const int more = find(q, s + lane < eq ? F.idx[s + lane] : -1, s + lane);
+      for (int t = sg; t < more; t += NSG) {
+        column(t, more, M0);
+        update(t, more, Lq, M0);
+      }
+      __syncwarp();
+    }
+  }
+  // the diagonal block: in-place LU (unit lower)
+  V* D = blk + nl * BB;
+  if constexpr (EM) {
+    V x = D[el];
+#pragma unroll
+    for (int cb = 0; cb < B - 1; ++cb) {
+      const V piv = __shfl_sync(0xffffffffu, x, cb * B + cb, SG);
+      if (c == cb && a > cb && live && sg == 0) {
+        if (piv == V(0)) note_zero_pivot(zero_flag, i * B + a, i * B + cb);
+      }
+      if (c == cb && a > cb) x = x / piv;
+      const V l = __shfl_sync(0xffffffffu, x, a * B + cb, SG);
+      const V p = __shfl_sync(0xffffffffu, x, cb * B + c, SG);
+      if (a > cb && c > cb) x -= l * p;
+    }
+    __syncwarp();
+    if (live && sg == 0) D[e] = x;
+  } else {
+    V x[B];
+#pragma unroll
+    for (int m = 0; m < B; ++m) x[m] = D[a * B + m];
+#pragma unroll
+    for (int cb = 0; cb < B - 1; ++cb) {
+      V p[B];
+#pragma unroll
+      for (int m = cb; m < B; ++m) p[m] = __shfl_sync(0xffffffffu, x[m], cb, SG);
+      if (a > cb) {
+        if (p[cb] == V(0) && live && sg == 0) note_zero_pivot(zero_flag, i * B + a, i * B + cb);
+        const V l = x[cb] / p[cb];
+        x[cb] = l;
+#pragma unroll
+        for (int m = cb + 1; m < B; ++m) x[m] -= l * p[m];
+      }
+    }
+    __syncwarp();
+    if (live && sg == 0) {
+#pragma unroll
+      for (int m = 0; m < B; ++m) D[a * B + m] = x[m];
+    }
+  }
+  __syncwarp();
+  if (lane < B) rp[(long)i * B + lane] = V(1) / D[lane * B + lane];
+  // the upper blocks: L_ii^-1 applied
+  for (int t = nl + 1 + sg; t < nb; t += NSG) {
+    V* U = blk + t * BB;
+    if constexpr (EM) {
+      V x = U[el];
+#pragma unroll
+      for (int cb = 0; cb < B - 1; ++cb) {
+        const V uc = __shfl_sync(sgmask, x, cb * B + c, SG);
+        if (a > cb) x -= D[a * B + cb] * uc;
+      }
+      if (live) U[e] = x;
+    } else {
+      V u[B];
+#pragma unroll
+      for (int r = 0; r < B; ++r) u[r] = U[r * B + c];
+#pragma unroll
+      for (int cb = 0; cb < B - 1; ++cb)
+#pragma unroll
+        for (int r = cb + 1; r < B; ++r) u[r] -= D[r * B + cb] * u[cb];
+      if (live) {
+#pragma unroll
+        for (int r = 0; r < B; ++r) U[r * B + c] = u[r];
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll 4
+  for (int k = lane; k < nb * BB; k += 32) row[k] = blk[k];
 }
 
 // Forward sweep of one level, a group of FV_LG lanes per block row (lane a = row a of the block).
@@ -770,6 +1052,8 @@ struct FvIlu0 {
   int *tptr = nullptr, *tidx = nullptr, *tblk = nullptr;
   int* tdiag = nullptr;   // position of the diagonal block in each row of the transpose
   void* val = nullptr;
+  void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
+  int row_cap = 0;        // most blocks in a row
   void* tval = nullptr;   // (b > 1) the factor's blocks transposed, in the transpose's order
   unsigned long long* zero_flag = nullptr;
   // level sets: rows grouped by level (device), level boundaries (host)
@@ -916,14 +1200,27 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) {
     const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
     if (cnt == 0) continue;
-    if (f->b == 1)
+    const size_t wb = factor_warp_bytes<V>(f->row_cap, f->b * f->b);
+    if (f->b == 1 || wb > kFactorSmem) {  // scalar, or hundreds of blocks in a row
       k_ilu_factor_level<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l], cnt,
                                                                 f->zero_flag);
-    else
+      continue;
+    }
+    if (cnt >= kFactorWide) {
       with_block_size(f->b, [&](auto B) {
         k_ilu_factor_lgb<V, B()><<<fv_blocks((long)cnt * FV_LG, 128), 128, 0, s>>>(
-            F, f->rows_fwd + f->lv_fwd[l], cnt, f->zero_flag);
+            F, f->rows_fwd + f->lv_fwd[l], cnt, (V*)f->rp, f->zero_flag);
       });
+      continue;
+    }
+    // a level that leaves SMs idle: a warp per block, so that no two share an SM's fp64 issue
+    const int warps = cnt <= 4 * 152 || 4 * wb > kFactorSmem ? 1 : 4;
+    with_block_size(f->b, [&](auto B) {
+      auto kern = k_ilu_factor_w<V, B()>;
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactorSmem);
+      kern<<<fv_blocks(cnt, warps), 32 * warps, warps * wb, s>>>(
+          F, f->rows_fwd + f->lv_fwd[l], cnt, f->row_cap, (V*)f->rp, f->zero_flag);
+    });
   }
 }
 
@@ -1184,6 +1481,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   f->b = b;
   f->nnzb = nnzb;
   f->precision = precision;
+  for (int i = 0; i < n; ++i) f->row_cap = std::max(f->row_cap, indptr[i + 1] - indptr[i]);
   std::vector<int> rows;
   levels(n, true, [&](int i, auto&& use) {
     for (int q = indptr[i]; q < diag[i]; ++q) use(indices[q]);
@@ -1214,6 +1512,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
     return FV_ERR_CUDA;
   size_t vs = precision == 64 ? sizeof(double) : sizeof(float);
   FV_CUDA_TRY(cudaMalloc(&f->val, vs * (size_t)nnzb * b * b));
+  FV_CUDA_TRY(cudaMalloc(&f->rp, vs * (size_t)n * b));
   FV_CUDA_TRY(cudaMalloc(&f->zero_flag, sizeof(unsigned long long)));
   FV_CUDA_TRY(cudaMalloc(&f->work, vs * (size_t)n * b));
   FV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1231,6 +1530,7 @@ extern "C" int fv_ilu0_destroy(FvIlu0* f) {
   cudaFree(f->tblk);
   cudaFree(f->tdiag);
   cudaFree(f->val);
+  cudaFree(f->rp);
   cudaFree(f->tval);
   cudaFree(f->zero_flag);
   cudaFree(f->rows_fwd);
@@ -1272,6 +1572,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->b = src->b;
   f->nnzb = src->nnzb;
   f->precision = precision;
+  f->row_cap = src->row_cap;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;
@@ -1309,6 +1610,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   if (rc == FV_OK && precision != 0) {
     const size_t vs = precision == 64 ? sizeof(double) : sizeof(float);
     if (cudaMalloc(&f->val, vs * nnzb * f->b * f->b) != cudaSuccess ||
+        cudaMalloc(&f->rp, vs * n * f->b) != cudaSuccess ||
         cudaMalloc(&f->zero_flag, sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&f->work, vs * n * f->b) != cudaSuccess)
       rc = FV_ERR_CUDA;

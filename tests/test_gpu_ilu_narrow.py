@@ -66,3 +66,40 @@ def test_narrow_level_sets_match_the_oracle(width, layers, b, links, precision):
     c = f.clone(precision)
     c.refactor(blocks.reshape(-1))
     assert np.array_equal(got, c.solve(rhs).cpu().numpy())
+
+
+# rows of the factorisation: a warp each, up to 32 columns of a finished row looked up at once, two
+# (b <= 4) or four matching blocks updated at once; more than 32 lower blocks, a row too long for
+# shared memory (one thread a row), and blocks with zeros (whose quotients are zero).
+@pytest.mark.parametrize("n,b,density", [(40, 2, 0.1), (60, 3, 0.3), (50, 4, 1.0), (48, 5, 0.5), (45, 6, 1.0),
+                                         (30, 7, 0.4), (24, 8, 1.0), (110, 4, 0.9), (400, 8, 0.02)])
+def test_factor_is_bitwise_the_oracle(n, b, density):
+    import scipy.sparse as sp
+
+    from aquaflux_gb300.ilu0 import Ilu0
+
+    rng = np.random.default_rng(n + b)
+    mask = rng.random((n, n)) < density
+    if n == 400:
+        mask[0], mask[:, 0] = True, True  # one row of 400 blocks of 512 bytes
+    mask = mask | mask.T | np.eye(n, dtype=bool)
+    pat = sp.csr_matrix(mask)
+    pat.sort_indices()
+    blocks = rng.uniform(-1, 1, (pat.nnz, b, b)) * (0.5 / (n * b))
+    blocks[rng.random(blocks.shape) < 0.2] = 0.0
+    for r in range(n):
+        blocks[pat.indptr[r] + int(np.searchsorted(pat.indices[pat.indptr[r]:pat.indptr[r + 1]], r))] += np.eye(b)
+    a = sp.bsr_matrix((blocks, pat.indices, pat.indptr), shape=(n * b,) * 2).tocsr()
+    rows = np.repeat(np.arange(n), np.diff(pat.indptr))
+    full = sp.csr_matrix(np.ones((n * b, n * b)) * np.kron(mask, np.ones((b, b))))
+    full.sort_indices()
+    dense = a.toarray()
+    ip, ix = full.indptr.astype(np.int32), full.indices.astype(np.int32)
+    vals = dense[np.repeat(np.arange(n * b), np.diff(ip)), ix]
+    _, data, _, _ = oracle_factor_solve(ip, ix, vals, np.ones(n * b))
+    f = Ilu0.from_csr(pat.indptr.astype(np.int32), pat.indices.astype(np.int32), blocks.reshape(-1), block_size=b)
+    got = f.factor_values().cpu().numpy().reshape(-1, b, b)
+    out = np.zeros((n * b, n * b))
+    for q, (r, col) in enumerate(zip(rows, pat.indices)):
+        out[r * b:(r + 1) * b, col * b:(col + 1) * b] = got[q]
+    np.testing.assert_array_equal(out[np.repeat(np.arange(n * b), np.diff(ip)), ix], data)
