@@ -13,10 +13,11 @@
 //                     with the residual's signs (whole face blocks, contiguous), then the SST
 //                     source rows, the omega wall-cell rows and the pressure-pin row.
 // Every entry is the tangent the coloured probe computes for it, by the same arithmetic in the
-// same order.
+// same order.  This is the fp32 assembly of an fp32 preconditioner; fp64 blocks come from the
+// derivatives written out (jacobian.inc.cuh).
 
-// The state with a unit tangent on one unknown (index `seed` of the field-major state); T = Dual,
-// or DualF for the fp32 assembly of an fp32 preconditioner.
+// The state with a unit tangent on one unknown (index `seed` of the field-major state); T = DualF,
+// or Dual for the wall cells' source rows of the fp64 assembly.
 template <class T>
 struct SeedSrc {
   const decltype(T::v)* v;  // the state in the pass's precision

@@ -1794,6 +1794,7 @@ int dispatch_t(FvCase* cs, const double* state, const double* tangent, int kind,
 
 #include "adjoint.inc.cuh"
 #include "assemble.inc.cuh"
+#include "jacobian.inc.cuh"
 
 template <int DIM, bool TURB>
 AdjWork adj_layout(FvCase* cs) {
@@ -2136,27 +2137,28 @@ size_t fv_residual_work_bytes(int dim, int turb, long nc, long nf, int sweeps, i
   return (size_t)n * sizeof(Dual);
 }
 
+// fp32: the face derivatives; fp64: the source rows' 4 doubles per cell (fewer: nc < nf).
 size_t fv_jac_face_bytes(int dim, int turb, long nf) {
   long nfld = dim + 1 + (turb ? 2 : 0);
-  return sizeof(double) * (size_t)(2 * nfld * nfld) * nf;
+  return sizeof(float) * (size_t)(2 * nfld * nfld) * nf;
 }
 
 int fv_case_assemble_frozen(FvCase* cs, const double* state, const int* indptr,
                             const int* indices, void* values, void* D, int fp32,
                             cudaStream_t s) {
-  const int dim = cs->mesh->dim;
-  const bool turb = cs->desc.turbulent != 0;
-  auto go = [&](auto t) {
-    using T = decltype(t);
-    GS<T>* v = (GS<T>*)values;
-    GS<T>* d = (GS<T>*)D;
-    if (dim == 2)
-      return turb ? assemble_frozen<T, 2, true>(cs, state, indptr, indices, v, d, s)
-                  : assemble_frozen<T, 2, false>(cs, state, indptr, indices, v, d, s);
-    return turb ? assemble_frozen<T, 3, true>(cs, state, indptr, indices, v, d, s)
-                : assemble_frozen<T, 3, false>(cs, state, indptr, indices, v, d, s);
+  auto go = [&](auto dim, auto turb) {
+    constexpr int DIM = decltype(dim)::value;
+    constexpr bool TURB = decltype(turb)::value;
+    if (fp32)
+      return assemble_frozen<DualF, DIM, TURB>(cs, state, indptr, indices, (float*)values,
+                                               (float*)D, s);
+    return assemble_frozen64<DIM, TURB>(cs, state, indptr, indices, (double*)values, (double*)D, s);
   };
-  return fp32 ? go(DualF{}) : go(Dual{});
+  using D2 = std::integral_constant<int, 2>;
+  using D3 = std::integral_constant<int, 3>;
+  const bool turb = cs->desc.turbulent != 0;
+  if (cs->mesh->dim == 2) return turb ? go(D2{}, std::true_type{}) : go(D2{}, std::false_type{});
+  return turb ? go(D3{}, std::true_type{}) : go(D3{}, std::false_type{});
 }
 
 int fv_gg_sweeps_scalar(const MeshView& m, int sweeps, double rel, const double* num, double* x0,
