@@ -4,7 +4,7 @@
 scipy's ``reverse_cuthill_mckee`` on the interior-face cell graph (``cell_adjacency_coo``,
 ``aquaflux/mesh/graph.py:29-56``).  Here the graph is built on the GPU (``fv_cell_graph``: sorted,
 coalesced CSR) and the breadth-first sweeps run on the GPU level by level
-(``fv_rcm_permutation``), giving the same permutation bit for bit.  The only host step is the seed
+(``fv_rcm_permutation``, one launch), giving the same permutation bit for bit.  The only host step is the seed
 order, numpy's ``argsort`` of the node degrees -- the call scipy's implementation makes, so ties
 between equal-degree seeds resolve as they do there.
 """
@@ -23,11 +23,10 @@ def _stream() -> int:
 def cell_graph(owner, neighbour, n_cells: int) -> tuple[torch.Tensor, torch.Tensor]:
     """The symmetric cell graph of the interior faces (``neighbour >= 0``) as device CSR
     ``(indptr, indices)``, neighbours ascending, repeated pairs coalesced."""
-    own = torch.as_tensor(np.asarray(owner), dtype=torch.int32)
-    nb = torch.as_tensor(np.asarray(neighbour), dtype=torch.int32)
+    own = torch.as_tensor(np.asarray(owner), dtype=torch.int32).to("cuda")
+    nb = torch.as_tensor(np.asarray(neighbour), dtype=torch.int32).to("cuda")
     keep = nb >= 0
-    own = own[keep].to("cuda").contiguous()
-    nb = nb[keep].to("cuda").contiguous()
+    own, nb = own[keep], nb[keep]
     n_pairs = int(own.numel())
     indptr = torch.empty(n_cells + 1, dtype=torch.int32, device="cuda")
     indices = torch.empty(max(2 * n_pairs, 1), dtype=torch.int32, device="cuda")
@@ -47,7 +46,7 @@ def rcm_permutation(owner, neighbour, n_cells: int) -> np.ndarray:
     work = torch.empty(3 * n_cells + 1, dtype=torch.int32, device="cuda")
     check(lib().fv_rcm_permutation(n_cells, ptr(indptr), ptr(indices), ptr(seeds), ptr(perm),
                                    ptr(work), _stream()))
-    return perm.cpu().numpy().astype(np.int64)
+    return perm.to(torch.int64).cpu().numpy()
 
 
 def mesh_rcm_permutation(mesh) -> np.ndarray:
