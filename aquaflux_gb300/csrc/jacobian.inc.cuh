@@ -177,6 +177,10 @@ __global__ void __launch_bounds__(128) k_jac_src(MeshView m, CaseView cv, const 
   src[3 * nc + c] = okw ? V * (2.0 * beta * w - cut * lw + cross * iw) : bad;
 }
 
+// -x where `neg`, by the sign bit (no fp64 instruction).
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
 template <int NF>
 __device__ __forceinline__ void store_row(double* p, const double (&x)[NF], bool vec) {
   if (NF % 2 == 0 && vec) {
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
                                                   const double* cl, const double* psi,
                                                   const double* co, const double* src,
                                                   const int* indptr, const int* indices,
-                                                  double* values, bool vec) {
+                                                  double* values, double irho, bool vec) {
   using L = Layout<DIM, TURB>;
   constexpr int NF = L::NFLD;
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -208,10 +212,12 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
   // rows without the face sum: the pinned pressure row, the omega wall-cell row
   bool skip = cont && c == cv.pin;
   if constexpr (TURB) skip = skip || (q == L::W && cv.wcell[c] != 0);
-  const double rho = cv.rho, irho = 1.0 / rho;
+  const double rho = cv.rho;
   const double* rec = mom ? (cv.rec_mom ? psi : nullptr) : (cv.rec_sca ? psi : nullptr);
   const int adv = mom ? q : q - 1;  // index among the advected fields
-  double dg[NF];
+  // the diagonal block's row; its own field's column (one fp64 addition a face, not one for every
+  // field a warp's rows hold) is added at the end
+  double dg[NF], dq = 0.0;
 #pragma unroll
   for (int r = 0; r < NF; ++r) dg[r] = 0.0;
   unsigned long long written = 0;  // slots of the block row, the first 64
@@ -235,15 +241,20 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
     for (int j = 0; j < DIM; ++j) nrm[j] = m.normal[(long)j * nf + f];
     if (f < m.nfi) {
       const int o = m.owner[f], n = m.nb[f];
-      const double sg = isnb ? -1.0 : 1.0, g = m.g[f];
-      const double ws = isnb ? g : 1.0 - g, wo = isnb ? 1.0 - g : g;  // this cell's weight, the other's
-      double up = sg;  // d flux / d mdot, with the sum's sign
+      const double g = m.g[f], h = 1.0 - g;
+      const double ws = isnb ? g : h, wo = isnb ? h : g;  // this cell's weight, the other's
+      double up = isnb ? -1.0 : 1.0;  // d flux / d mdot, with the sum's sign
       double cond = 0.0, flux = 0.0;
       if (!cont) {
         const int cu = out ? o : n;
-        const double s = mom ? sg : sg * irho;
-        up = s * upwind_rec<double, DIM>(m, G, rec, adv, q, f, cu, state[(long)q * nc + cu], gv);
-        flux = s * mdot;
+        up = upwind_rec<double, DIM>(m, G, rec, adv, q, f, cu, state[(long)q * nc + cu], gv);
+        flux = mdot;
+        if (!mom) {
+          up *= irho;
+          flux *= irho;
+        }
+        up = flip(up, isnb);
+        flux = flip(flux, isnb);
         cond = co[(mom ? 2L : (long)q - DIM + 2) * nf + f];
       }
       double oth[NF];
@@ -256,13 +267,13 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
         dg[j] = fma(ws, x, dg[j]);
         oth[j] = wo * x;
       }
-      const double x = isnb ? -(up * co[nf + f]) : up * co[nf + f];
+      const double x = flip(up * co[nf + f], isnb);
       double ps = x, po = -x;
       double nq = 0.0;
 #pragma unroll
       for (int j = 0; j < DIM; ++j) nq = q == j ? nrm[j] : nq;
       if (mom) {
-        const double y = sg * (A * nq);
+        const double y = flip(A * nq, isnb);
         ps = fma(ws, y, ps);
         po = fma(wo, y, po);
       }
@@ -271,12 +282,13 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
       const bool mine = out != isnb;  // this cell is the upwind one
       const double ds = mine ? cond + flux : cond, dn = mine ? -cond : flux - cond;
       if (!cont) {
+        dq += ds;
+        double own = oth[0];
 #pragma unroll
-        for (int r = 0; r < NF; ++r)
-          if (r == q) {
-            dg[r] += ds;
-            oth[r] += dn;
-          }
+        for (int r = 1; r < NF; ++r) own = r == q ? oth[r] : own;
+        own += dn;
+#pragma unroll
+        for (int r = 0; r < NF; ++r) oth[r] = r == q ? own : oth[r];
       }
       if (!finite_bits(co[nf + f]) ||
           (!cont && !(finite_bits(mdot) && finite_bits(cond) && finite_bits(up)))) {
@@ -315,9 +327,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
       double nq = 0.0;
 #pragma unroll
       for (int j = 0; j < DIM; ++j) nq = q == j ? nrm[j] : nq;
-#pragma unroll
-      for (int r = 0; r < DIM; ++r)
-        if (r == q) dg[r] += d;
+      dq += d;
       if (kind >= 0 && kind != 3) dg[L::P] += A * nq;
       if constexpr (TURB) {
         if ((kind == 0 || kind == 1) && cv.swall[f]) {
@@ -346,10 +356,8 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
           const Dual wt = wall_weight(Dual{par.nu, 0.0}, cv.wd[o], Dual{phi, 1.0});
           d += wt.d * cl[4L * nc + o] * (A * m.inv_dpn[f]) * (bphi - phi - cp);
         }
-#pragma unroll
-        for (int r = L::K; r <= L::W; ++r)
-          if (r == q) dg[r] += d;
       }
+      dq += d;
     }
     if (!finite_bits(co[nf + f]) ||
         (!cont && !(finite_bits(mdot) && finite_bits(up) &&
@@ -362,6 +370,9 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
       dg[L::P] = fma(up, co[nf + f], dg[L::P]);
     }
   }
+#pragma unroll
+  for (int r = 0; r < NF; ++r)
+    if (r == q) dg[r] += dq;
   if (cont && c == cv.pin) dg[L::P] = 1.0;
   if constexpr (TURB) {
     if (q >= L::K) {
@@ -378,7 +389,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
 }
 
 // The fp64 blocks of J_direct; `src` holds 4 nc doubles.
-// Measured (80 x 63 x 51 SST channel): 6.73 -> 1.26 ms, 0.76 of it k_jac_rows.
+// Measured (80 x 63 x 51 SST channel): 6.73 -> 1.13 ms, 0.62 of it k_jac_rows.
 template <int DIM, bool TURB>
 int assemble_frozen64(FvCase* cs, const double* state, const int* indptr, const int* indices,
                       double* values, double* src, cudaStream_t s) {
@@ -408,7 +419,7 @@ int assemble_frozen64(FvCase* cs, const double* state, const int* indptr, const 
     k_jac_src<DIM><<<bc, TB, 0, s>>>(m, cv, state, par, w.G, w.cl, w.Gwi, src);
   k_jac_rows<DIM, TURB><<<fv_blocks(nc * NF, TB), TB, 0, s>>>(
       m, cv, state, par, w.G, w.cl, npsi ? w.psi : nullptr, w.FL, src, indptr, indices, values,
-      (uintptr_t)values % 16 == 0);
+      1.0 / cs->desc.rho, (uintptr_t)values % 16 == 0);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
 }
