@@ -387,6 +387,16 @@ __global__ void k_ilu_lower_t(IluView<V> F, const int* tptr, const int* tidx, co
 // Element-wise operation orders are those of the one-thread kernels above, except the forward
 // solve's upper sweep, which subtracts the off-diagonal blocks before the in-block terms (the
 // reference subtracts in ascending column order); b = 1 uses the one-thread kernels.
+// A level's kernel is launched while the one before still runs (programmatic dependent launch): it
+// lets the next one start, finds its rows and asks the L2 cache for their blocks, which no sweep
+// writes, and only then waits for the level before.  Without that each level paid its launch and
+// the memory latency of rows, offsets, columns and blocks in turn.
+__device__ __forceinline__ void next_level_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_level_before() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 #define FV_LG 8
 __device__ __forceinline__ unsigned lg_mask() { return 0xffu << ((threadIdx.x & 31) & ~(FV_LG - 1)); }
 
@@ -557,6 +567,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
   constexpr bool EM = B <= 4;            // a lane per entry
   constexpr int SG = EM ? 16 : 8, NSG = 32 / SG;
   extern __shared__ __align__(16) unsigned char factor_smem[];
+  next_level_may_start();
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x / 32) + warp;
   if (w >= count) return;  // whole warps exit together
@@ -650,6 +661,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
       }
     }
   };
+  wait_level_before();  // (only the row itself, which no earlier level writes, was read so far)
   fetch(0);
   for (int q = 0; q < nl; ++q) {
     const int jq = j, s0 = dj + 1, eq = ej;
@@ -782,9 +794,66 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
   for (int k = lane; k < nb * BB; k += 32) row[k] = blk[k];
 }
 
-// Forward sweep of one level, a group of FV_LG lanes per block row (lane a = row a of the block).
+// acc minus the products of `count` blocks (positions q0, q0 + STEP, ...) with their columns' entries
+// of x, in that order (and, STEP = -1, each block's entries from the last).  U > 1: U blocks are
+// read at a time, the columns of eight by the group's lanes at once.
+template <class V, int B, int STEP, int U>
+__device__ __forceinline__ V subtract_blocks(V acc, const V* val, const int* idx, const V* x, int q0,
+                                             int count, int a, bool live, unsigned mask) {
+  constexpr long BB = (long)B * B;
+  auto block = [&](const V (&L)[B], const V (&xj)[B]) {
+#pragma unroll
+    for (int c = 0; c < B; ++c) {
+      const int e = STEP > 0 ? c : B - 1 - c;
+      acc -= L[e] * xj[e];
+    }
+  };
+  if constexpr (U == 1) {
+    if (live)
+#pragma unroll 1
+      for (int k = 0; k < count; ++k) {
+        const int q = q0 + STEP * k;
+        V L[B], xj[B];
+        load_seg<B>(val + (long)q * BB + (long)a * B, L);
+        load_seg<B>(x + (long)idx[q] * B, xj);
+        block(L, xj);
+      }
+  } else {
+    for (int k0 = 0; k0 < count; k0 += FV_LG) {
+      const int col = k0 + a < count ? idx[q0 + STEP * (k0 + a)] : 0;
+      for (int k = k0; k < count && k < k0 + FV_LG; k += U) {
+        V L[U][B], xj[U][B];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (live && k + u < count)
+            load_seg<B>(val + (long)(q0 + STEP * (k + u)) * BB + (long)a * B, L[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int j = __shfl_sync(mask, col, k - k0 + u, FV_LG);
+          if (live && k + u < count) load_seg<B>(x + (long)j * B, xj[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (live && k + u < count) block(L[u], xj[u]);
+      }
+    }
+  }
+  return acc;
+}
+
 template <class V, int B>
+__device__ __forceinline__ void ask_blocks(const V* val, int q0, int count, int a) {
+  // lane a asks for the lines at a, a + 8, ... of the blocks' contiguous range
+  const char* p = (const char*)(val + (long)q0 * B * B);
+  const long bytes = (long)count * B * B * (long)sizeof(V);
+  for (long o = 128L * a; o < bytes; o += 128L * FV_LG)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
+}
+
+// Forward sweep of one level, a group of FV_LG lanes per block row (lane a = row a of the block).
+template <class V, int B, int U>
 __global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, V* y) {
+  if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -792,17 +861,15 @@ __global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, V* y) {
   const int i = rows[gid];
   const bool live = a < B;
   constexpr long BB = (long)B * B;
+  const int q0 = F.ptr[i], di = F.diag[i];
+  if (U > 1) {
+    ask_blocks<V, B>(F.val, q0, di - q0, a);
+    wait_level_before();
+  }
   V acc = live ? y[(long)i * B + a] : V(0);
-  if (live)
-    for (int q = F.ptr[i]; q < F.diag[i]; ++q) {
-      V L[B], yj[B];
-      load_seg<B>(F.val + (long)q * BB + (long)a * B, L);
-      load_seg<B>(y + (long)F.idx[q] * B, yj);
-#pragma unroll
-      for (int c = 0; c < B; ++c) acc -= L[c] * yj[c];
-    }
+  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
-  if (live) load_seg<B>(F.val + (long)F.diag[i] * BB + (long)a * B, D);
+  if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
 #pragma unroll
   for (int c = 0; c < B; ++c) {
     const V vc = __shfl_sync(mask, acc, c, FV_LG);
@@ -847,8 +914,9 @@ __device__ __forceinline__ V upper_block_solve(V acc, const V (&D)[B], int a, bo
 }
 
 // Backward sweep of one level (U x = y).
-template <class V, int B>
+template <class V, int B, int U>
 __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
+  if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -856,17 +924,15 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
   const int i = rows[gid];
   const bool live = a < B;
   constexpr long BB = (long)B * B;
+  const int di = F.diag[i], re = F.ptr[i + 1];
+  if (U > 1) {
+    ask_blocks<V, B>(F.val, di + 1, re - di - 1, a);
+    wait_level_before();
+  }
   V acc = live ? x[(long)i * B + a] : V(0);
-  if (live)
-    for (int q = F.diag[i] + 1; q < F.ptr[i + 1]; ++q) {
-      V U[B], xk[B];
-      load_seg<B>(F.val + (long)q * BB + (long)a * B, U);
-      load_seg<B>(x + (long)F.idx[q] * B, xk);
-#pragma unroll
-      for (int c = 0; c < B; ++c) acc -= U[c] * xk[c];
-    }
+  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, x, di + 1, re - di - 1, a, live, mask);
   V D[B];
-  if (live) load_seg<B>(F.val + (long)F.diag[i] * BB + (long)a * B, D);
+  if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
   acc = upper_block_solve<V, B>(acc, D, a, live, mask);
   if (live) x[(long)i * B + a] = acc;
 }
@@ -875,8 +941,9 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
 // those rows own no upper blocks (the second colour of a two-colour order), a row's backward step
 // is the in-block upper solve of its own forward result, with the diagonal block already in
 // registers.  The same operations in the same order as the two separate sweeps.
-template <class V, int B>
+template <class V, int B, int U>
 __global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, V* y) {
+  if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -884,17 +951,15 @@ __global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, V
   const int i = rows[gid];
   const bool live = a < B;
   constexpr long BB = (long)B * B;
+  const int q0 = F.ptr[i], di = F.diag[i];
+  if (U > 1) {
+    ask_blocks<V, B>(F.val, q0, di - q0, a);
+    wait_level_before();
+  }
   V acc = live ? y[(long)i * B + a] : V(0);
-  if (live)
-    for (int q = F.ptr[i]; q < F.diag[i]; ++q) {
-      V L[B], yj[B];
-      load_seg<B>(F.val + (long)q * BB + (long)a * B, L);
-      load_seg<B>(y + (long)F.idx[q] * B, yj);
-#pragma unroll
-      for (int c = 0; c < B; ++c) acc -= L[c] * yj[c];
-    }
+  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
-  if (live) load_seg<B>(F.val + (long)F.diag[i] * BB + (long)a * B, D);
+  if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
 #pragma unroll
   for (int c = 0; c < B; ++c) {
     const V vc = __shfl_sync(mask, acc, c, FV_LG);
@@ -938,9 +1003,10 @@ __device__ __forceinline__ V lower_t_block_solve(V acc, const V (&Dc)[B], int a,
 // blocks (j, i) of U, j < i (positions tptr[i] .. tdiag[i] of the transpose, ascending j), row a
 // of each transposed block (column a of the block of U) for lane a, then the in-block lower solve
 // with D^T -- the operations and their order of the reference's transposed solve.
-template <class V, int B>
+template <class V, int B, int U>
 __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx, const int* tdiag,
                                  const V* tval, const int* rows, int count, V* z) {
+  if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -948,17 +1014,15 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const int i = rows[gid];
   const bool live = a < B;
   constexpr long BB = (long)B * B;
+  const int q0 = tptr[i], di = tdiag[i];
+  if (U > 1) {
+    ask_blocks<V, B>(tval, q0, di - q0, a);
+    wait_level_before();
+  }
   V acc = live ? z[(long)i * B + a] : V(0);
-  if (live)
-    for (int q = tptr[i]; q < tdiag[i]; ++q) {
-      V Ut[B], zj[B];
-      load_seg<B>(tval + (long)q * BB + (long)a * B, Ut);
-      load_seg<B>(z + (long)tidx[q] * B, zj);
-#pragma unroll
-      for (int c = 0; c < B; ++c) acc -= Ut[c] * zj[c];
-    }
+  acc = subtract_blocks<V, B, 1, U>(acc, tval, tidx, z, q0, di - q0, a, live, mask);
   V Dc[B];  // Dc[c] = D(c, a): row a of D^T
-  if (live) load_seg<B>(tval + (long)tdiag[i] * BB + (long)a * B, Dc);
+  if (live) load_seg<B>(tval + (long)di * BB + (long)a * B, Dc);
   else
 #pragma unroll
     for (int c = 0; c < B; ++c) Dc[c] = V(0);
@@ -969,9 +1033,10 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // Backward sweep of one level of the transposed solve, L^T x = z (unit diagonal): the blocks
 // (k, i) of L, k > i (positions tptr[i + 1] - 1 down to tdiag[i] + 1), then the in-block unit
 // upper solve.
-template <class V, int B>
+template <class V, int B, int U>
 __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx, const int* tdiag,
                                  const V* tval, const int* rows, int count, V* x) {
+  if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -979,17 +1044,15 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const int i = rows[gid];
   const bool live = a < B;
   constexpr long BB = (long)B * B;
+  const int di = tdiag[i], last = tptr[i + 1] - 1;
+  if (U > 1) {
+    ask_blocks<V, B>(tval, di + 1, last - di, a);
+    wait_level_before();
+  }
   V acc = live ? x[(long)i * B + a] : V(0);
-  if (live)
-    for (int q = tptr[i + 1] - 1; q > tdiag[i]; --q) {
-      V Lt[B], xk[B];
-      load_seg<B>(tval + (long)q * BB + (long)a * B, Lt);
-      load_seg<B>(x + (long)tidx[q] * B, xk);
-#pragma unroll
-      for (int c = B - 1; c >= 0; --c) acc -= Lt[c] * xk[c];
-    }
+  acc = subtract_blocks<V, B, -1, U>(acc, tval, tidx, x, last, last - di, a, live, mask);
   V Dc[B];
-  if (live) load_seg<B>(tval + (long)tdiag[i] * BB + (long)a * B, Dc);
+  if (live) load_seg<B>(tval + (long)di * BB + (long)a * B, Dc);
   else
 #pragma unroll
     for (int c = 0; c < B; ++c) Dc[c] = V(0);
@@ -1069,7 +1132,8 @@ struct FvIlu0 {
     int4* col = nullptr;
     int* bounds = nullptr;  // nlev + 1 offsets into row / col
     void* rec = nullptr;    // records, renewed by each factorisation
-    int nlev = 0, nlev_fwd = 0, widest = 0, k = 0;
+    int nlev = 0, nlev_fwd = 0, widest = 0;
+    int k = 0;              // blocks in a record, at most
   } run[2];
   bool fuse_fb = false;  // the last forward level's rows are the first backward level's (fused)
   cudaGraphExec_t apply_exec[2] = {nullptr, nullptr};  // forward / transposed solve
@@ -1127,8 +1191,10 @@ int widest(const std::vector<int>& bounds) {
 }
 
 // The one-launch form of a solve (k_ilu_run), when every level set fits one block and the vector
-// its shared memory (here in single precision; checked for the factor's in `runs`).  Above that a
-// level has the rows to fill more SMs than one, a launch each.  `row` gives a forward (0) /
+// its shared memory (here in single precision; checked for the factor's in pack_run).  Above that a
+// level has the rows to fill more SMs than one, a launch each: a 16-block cluster that runs levels
+// of 700 rows, the vector in global memory, took 135 us a solve against 114 (128 x 96 x 96 channel,
+// 20 levels, 15-27 blocks a row).  `row` gives a forward (0) /
 // backward (1) row as RunView::row; a backward row's blocks are taken upwards (step 1) or down.
 template <class RowFn>
 int build_run(FvIlu0* f, int t, const std::vector<int>& fwd, const std::vector<int>& lv_fwd,
@@ -1193,13 +1259,33 @@ int launch_run(FvIlu0* f, int t, const V* r, V* x, cudaStream_t s) {
   return rc;
 }
 
+// A level's kernel; `after` says that the launch before it on the stream is a level's too.
+template <class K, class... Args>
+void launch_level(K kern, int grid, cudaStream_t s, bool after, int threads, size_t smem,
+                  Args... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = after ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // Launch the level sequence of the factorization / a solve on `s` (captured into a graph once).
 template <class V>
 void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   IluView<V> F = view<V>(f);
+  bool after = false;  // the launch before on `s` lets this one start early
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) {
     const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
     if (cnt == 0) continue;
+    const bool early = after;
+    after = false;
     const size_t wb = factor_warp_bytes<V>(f->row_cap, f->b * f->b);
     if (f->b == 1 || wb > kFactorSmem) {  // scalar, or hundreds of blocks in a row
       k_ilu_factor_level<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l], cnt,
@@ -1218,65 +1304,89 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
     with_block_size(f->b, [&](auto B) {
       auto kern = k_ilu_factor_w<V, B()>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactorSmem);
-      kern<<<fv_blocks(cnt, warps), 32 * warps, warps * wb, s>>>(
-          F, f->rows_fwd + f->lv_fwd[l], cnt, f->row_cap, (V*)f->rp, f->zero_flag);
+      launch_level(kern, fv_blocks(cnt, warps), s, early, 32 * warps, warps * wb, F,
+                   (const int*)f->rows_fwd + f->lv_fwd[l], cnt, f->row_cap, (V*)f->rp,
+                   f->zero_flag);
     });
+    after = true;
   }
 }
+
+// The widest levels (590,000 rows: 140 us) are bound by bytes and want warps in flight: one block at
+// a time, a launch after the other (the registers of a deeper read made them 180-220 us).  Below
+// kWideRows a row's chain of latencies is the level's time: blocks are read several at a time and
+// the next level is launched early.  128 x 96 x 96 channel: 16 levels of 26,000 rows 176 -> 156 us.
+constexpr int kWideRows = 65536, kDeepRows = 8192;
 
 template <class V>
 void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
   IluView<V> F = view<V>(f);
   const bool lg = f->b > 1;
-  auto grid = [&](int cnt) { return lg ? fv_blocks((long)cnt * FV_LG, 128) : fv_blocks(cnt, 128); };
+  bool after = false;  // the launch before on `s` is a level of this solve
+  auto levels_of = [&](const std::vector<int>& lv, const int* order, size_t first, auto&& one) {
+    for (size_t l = first; l + 1 < lv.size(); ++l) {
+      const int cnt = lv[l + 1] - lv[l];
+      if (!cnt) continue;
+      one(l, order + lv[l], cnt);
+      after = cnt < kWideRows;
+    }
+  };
+  // the lane-group kernels of a level, by block size and depth
+  auto lane_groups = [&](int cnt, auto&& launch) {
+    const int grid = fv_blocks((long)cnt * FV_LG, 128);
+    with_block_size(f->b, [&](auto B) {
+      if (cnt >= kWideRows) launch(B, std::integral_constant<int, 1>{}, grid);
+      else if (cnt >= kDeepRows || sizeof(V) == 8) launch(B, std::integral_constant<int, 2>{}, grid);
+      else if constexpr (sizeof(V) == 4) launch(B, std::integral_constant<int, 4>{}, grid);
+    });
+  };
+  const V* tval = (const V*)f->tval;
   if (!transpose) {
     const size_t last = f->lv_fwd.size() - 2;
-    for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) {
-      const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
-      if (!cnt) continue;
-      if (lg && f->fuse_fb && l == last)
-        with_block_size(f->b, [&](auto B) {
-          k_ilu_lower_upper_lg<V, B()><<<grid(cnt), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l],
-                                                                 cnt, x);
-        });
-      else if (lg)
-        with_block_size(f->b, [&](auto B) {
-          k_ilu_lower_lg<V, B()><<<grid(cnt), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l], cnt, x);
-        });
-      else k_ilu_lower<V><<<grid(cnt), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l], cnt, x);
-    }
-    for (size_t l = f->fuse_fb ? 1 : 0; l + 1 < f->lv_bwd.size(); ++l) {
-      const int cnt = f->lv_bwd[l + 1] - f->lv_bwd[l];
-      if (!cnt) continue;
-      if (lg)
-        with_block_size(f->b, [&](auto B) {
-          k_ilu_upper_lg<V, B()><<<grid(cnt), 128, 0, s>>>(F, f->rows_bwd + f->lv_bwd[l], cnt, x);
-        });
-      else k_ilu_upper<V><<<grid(cnt), 128, 0, s>>>(F, f->rows_bwd + f->lv_bwd[l], cnt, x);
-    }
+    levels_of(f->lv_fwd, f->rows_fwd, 0, [&](size_t l, const int* rows, int cnt) {
+      if (!lg) {
+        k_ilu_lower<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, rows, cnt, x);
+        return;
+      }
+      lane_groups(cnt, [&](auto B, auto U, int grid) {
+        if (f->fuse_fb && l == last)
+          launch_level(k_ilu_lower_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+        else
+          launch_level(k_ilu_lower_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+      });
+    });
+    levels_of(f->lv_bwd, f->rows_bwd, f->fuse_fb ? 1 : 0, [&](size_t, const int* rows, int cnt) {
+      if (!lg) {
+        k_ilu_upper<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, rows, cnt, x);
+        return;
+      }
+      lane_groups(cnt, [&](auto B, auto U, int grid) {
+        launch_level(k_ilu_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+      });
+    });
   } else {
-    for (size_t l = 0; l + 1 < f->lv_tfwd.size(); ++l) {
-      const int cnt = f->lv_tfwd[l + 1] - f->lv_tfwd[l];
-      if (!cnt) continue;
-      const int* rows = f->rows_tfwd + f->lv_tfwd[l];
-      if (lg)
-        with_block_size(f->b, [&](auto B) {
-          k_ilu_upper_t_lg<V, B()><<<grid(cnt), 128, 0, s>>>(F, f->tptr, f->tidx, f->tdiag,
-                                                             (const V*)f->tval, rows, cnt, x);
-        });
-      else k_ilu_upper_t<V><<<grid(cnt), 128, 0, s>>>(F, f->tptr, f->tidx, f->tblk, rows, cnt, x);
-    }
-    for (size_t l = 0; l + 1 < f->lv_tbwd.size(); ++l) {
-      const int cnt = f->lv_tbwd[l + 1] - f->lv_tbwd[l];
-      if (!cnt) continue;
-      const int* rows = f->rows_tbwd + f->lv_tbwd[l];
-      if (lg)
-        with_block_size(f->b, [&](auto B) {
-          k_ilu_lower_t_lg<V, B()><<<grid(cnt), 128, 0, s>>>(F, f->tptr, f->tidx, f->tdiag,
-                                                             (const V*)f->tval, rows, cnt, x);
-        });
-      else k_ilu_lower_t<V><<<grid(cnt), 128, 0, s>>>(F, f->tptr, f->tidx, f->tblk, rows, cnt, x);
-    }
+    levels_of(f->lv_tfwd, f->rows_tfwd, 0, [&](size_t, const int* rows, int cnt) {
+      if (!lg) {
+        k_ilu_upper_t<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->tptr, f->tidx, f->tblk, rows,
+                                                             cnt, x);
+        return;
+      }
+      lane_groups(cnt, [&](auto B, auto U, int grid) {
+        launch_level(k_ilu_upper_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
+                     tval, rows, cnt, x);
+      });
+    });
+    levels_of(f->lv_tbwd, f->rows_tbwd, 0, [&](size_t, const int* rows, int cnt) {
+      if (!lg) {
+        k_ilu_lower_t<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->tptr, f->tidx, f->tblk, rows,
+                                                             cnt, x);
+        return;
+      }
+      lane_groups(cnt, [&](auto B, auto U, int grid) {
+        launch_level(k_ilu_lower_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
+                     tval, rows, cnt, x);
+      });
+    });
   }
 }
 

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 def layered(width, layers, b, links, seed):
-    """A symmetric block pattern of `layers` level sets of `width` rows, each row coupled to `links`
+    """A symmetric block pattern of `layers` level sets of `width` rows, each row coupled to up to `links`
     rows of the layer before; diagonally dominant blocks (condition number below 10)."""
     import scipy.sparse as sp
 
@@ -19,7 +19,7 @@ def layered(width, layers, b, links, seed):
     rows, cols = [np.arange(n)], [np.arange(n)]
     for layer in range(1, layers):
         for i in range(layer * width, (layer + 1) * width):
-            j = (layer - 1) * width + rng.choice(width, min(links, width), replace=False)
+            j = (layer - 1) * width + np.unique(rng.integers(0, width, links))
             rows += [np.full(j.size, i), j]
             cols += [j, np.full(j.size, i)]
     pat = sp.coo_matrix((np.ones(sum(r.size for r in rows)),
@@ -36,11 +36,13 @@ def layered(width, layers, b, links, seed):
 
 # a level's rows: one; a partial warp; as many as one launch takes (96 for b <= 4, 48 above) and
 # one more (a launch per level).  links: fewer than, as many as and more than a record's blocks (4),
-# with remainders of the batches of 2 behind them.
+# with remainders of the batches of 2 behind them.  Wider levels: blocks are
+# read 4 at a time below 8192 rows (fp32), 2 below 65536, one above.
 @pytest.mark.parametrize("precision", [64, 32])
 @pytest.mark.parametrize("width,layers,b,links", [
     (1, 60, 3, 1), (7, 9, 2, 2), (64, 12, 3, 3), (37, 6, 4, 4), (33, 5, 5, 7), (40, 4, 6, 8), (19, 5, 7, 9),
-    (30, 3, 8, 5), (96, 3, 3, 2), (97, 3, 3, 2), (48, 3, 6, 2), (49, 3, 6, 2)])
+    (30, 3, 8, 5), (96, 3, 3, 2), (97, 3, 3, 2), (48, 3, 6, 2), (49, 3, 6, 2),
+    (8191, 2, 2, 2), (8192, 2, 2, 2), (65535, 2, 2, 1), (65536, 2, 2, 1)])
 def test_narrow_level_sets_match_the_oracle(width, layers, b, links, precision):
     """fp64: transposed solve bitwise, forward solve to the rounding of its reordered sums (at most
     links * b + b terms of a well-conditioned row: 100 units in the last place of the largest
