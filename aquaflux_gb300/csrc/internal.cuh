@@ -140,8 +140,6 @@ struct FvCase {
   double* aux = nullptr;    // face intermediates of the double forward pass (for the adjoint)
   double* dscalar = nullptr; // (4) device scalars
   double* jac_face = nullptr; // (nf, 2, nfld, nfld) face flux derivatives of the Jacobian assembly
-  const int* jac_indptr = nullptr;  // the block pattern last assembled into, and its block count
-  long jac_nnzb = 0;
   int* wnear = nullptr;       // (nc) nearest SST wall face (internal index), turbulent cases
   bool wd_external = false;   // wd set by fv_case_set_wall_distance (wnear no longer describes it)
   bool wd_missing = false;    // turbulent, no SST wall face, distance not yet set: no evaluation
