@@ -10,9 +10,11 @@
 //                  ||w||, applies the previous Givens rotations, forms the new one, and updates
 //                  the rotated right-hand side g (residual estimate |g[j+1]|)
 //   k_scale        V[j+1] = w / ||w||
-// Every reduction is a fixed grid of kRedBlocks blocks over a grid-stride loop, block partials
-// summed in a fixed order by the last block to finish (a ticket counter), so results are bitwise
-// identical run to run.  Up to kChunk basis vectors are handled per launch; a longer basis is
+// Every reduction is a grid of kRedBlocks blocks, or one per tile of a shorter vector, over a
+// grid-stride loop, block partials summed in a fixed order by the last block to finish (a ticket
+// counter), so results are bitwise identical run to run (and the same for either grid: a block
+// without a tile would add zeros.  On 12,288 unknowns those 560 blocks' partials were most of a
+// column's time: 10-20 us a kernel, 5-15 without them).  Up to kChunk basis vectors are handled per launch; a longer basis is
 // processed chunk by chunk with the update and the projection in separate passes.
 #include <algorithm>
 #include <cmath>
@@ -23,7 +25,7 @@ namespace {
 
 constexpr int kThreads = 256;          // 8 warps
 constexpr int kWarps = kThreads / 32;
-constexpr int kRedBlocks = 4 * 152;     // fixed, so the summation order never changes
+constexpr int kRedBlocks = 4 * 152;     // most blocks of a reduction
 constexpr int kChunk = 32;              // basis vectors per launch
 constexpr int kSlots = kChunk / kWarps; // projections per warp
 
@@ -265,6 +267,10 @@ __global__ void k_combine(long n, int k, const double* __restrict__ Z, const dou
   }
 }
 
+int red_blocks(long n) {
+  return (int)std::min<long>(kRedBlocks, (n + kThreads - 1) / kThreads);
+}
+
 }  // namespace
 
 struct FvKrylov {
@@ -327,10 +333,10 @@ extern "C" int fv_krylov_start(FvKrylov* kr, long n, const double* r, double* v0
     return FV_ERR_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  k_upd_norm<<<kRedBlocks, kThreads, 0, s>>>(n, 0, nullptr, nullptr, const_cast<double*>(r),
+  k_upd_norm<<<red_blocks(n), kThreads, 0, s>>>(n, 0, nullptr, nullptr, const_cast<double*>(r),
                                               kr->part, kr->ticket, kr->red, kr->hs, NM_START, -1,
                                               nullptr, nullptr, nullptr);
-  k_scale<<<kRedBlocks, kThreads, 0, s>>>(n, r, kr->hs.inv, v0);
+  k_scale<<<red_blocks(n), kThreads, 0, s>>>(n, r, kr->hs.inv, v0);
   if (est) FV_CUDA_TRY(cudaMemcpyAsync(est, kr->hs.est, 2 * sizeof(double), cudaMemcpyDefault, s));
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
@@ -345,27 +351,27 @@ extern "C" int fv_krylov_arnoldi(FvKrylov* kr, int j, long n, double* V, double*
   cudaStream_t s = (cudaStream_t)stream;
   const int k = j + 1;  // basis vectors V[0..k)
   if (k <= kChunk) {
-    k_proj<<<kRedBlocks, kThreads, 0, s>>>(n, k, V, w, kr->part, kr->ticket, kr->h1);
-    k_upd<true><<<kRedBlocks, kThreads, 0, s>>>(n, k, V, kr->h1, w, kr->part, kr->ticket, kr->h2);
-    k_upd_norm<<<kRedBlocks, kThreads, 0, s>>>(n, k, V, kr->h2, w, kr->part, kr->ticket, kr->red,
+    k_proj<<<red_blocks(n), kThreads, 0, s>>>(n, k, V, w, kr->part, kr->ticket, kr->h1);
+    k_upd<true><<<red_blocks(n), kThreads, 0, s>>>(n, k, V, kr->h1, w, kr->part, kr->ticket, kr->h2);
+    k_upd_norm<<<red_blocks(n), kThreads, 0, s>>>(n, k, V, kr->h2, w, kr->part, kr->ticket, kr->red,
                                                 kr->hs, NM_COLUMN, j, kr->h1, kr->h2, nullptr);
   } else {
     // chunked CGS2: project all chunks, update by all chunks, twice; then the norm
     for (int pass = 0; pass < 2; ++pass) {
       double* h = pass == 0 ? kr->h1 : kr->h2;
       for (int c0 = 0; c0 < k; c0 += kChunk)
-        k_proj<<<kRedBlocks, kThreads, 0, s>>>(n, std::min(kChunk, k - c0), V + (long)c0 * n, w,
+        k_proj<<<red_blocks(n), kThreads, 0, s>>>(n, std::min(kChunk, k - c0), V + (long)c0 * n, w,
                                                kr->part, kr->ticket, h + c0);
       for (int c0 = 0; c0 < k; c0 += kChunk)
-        k_upd<false><<<kRedBlocks, kThreads, 0, s>>>(n, std::min(kChunk, k - c0),
+        k_upd<false><<<red_blocks(n), kThreads, 0, s>>>(n, std::min(kChunk, k - c0),
                                                      V + (long)c0 * n, h + c0, w, nullptr,
                                                      nullptr, nullptr);
     }
-    k_upd_norm<<<kRedBlocks, kThreads, 0, s>>>(n, 0, nullptr, nullptr, w, kr->part, kr->ticket,
+    k_upd_norm<<<red_blocks(n), kThreads, 0, s>>>(n, 0, nullptr, nullptr, w, kr->part, kr->ticket,
                                                 kr->red, kr->hs, NM_COLUMN, j, kr->h1, kr->h2,
                                                 nullptr);
   }
-  k_scale<<<kRedBlocks, kThreads, 0, s>>>(n, w, kr->hs.inv, V + (long)k * n);
+  k_scale<<<red_blocks(n), kThreads, 0, s>>>(n, w, kr->hs.inv, V + (long)k * n);
   if (est) FV_CUDA_TRY(cudaMemcpyAsync(est, kr->hs.est, 2 * sizeof(double), cudaMemcpyDefault, s));
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
@@ -381,7 +387,7 @@ extern "C" int fv_krylov_update(FvKrylov* kr, int k, long n, const double* Z, do
   cudaStream_t s = (cudaStream_t)stream;
   k_backsolve<<<1, 32, 0, s>>>(kr->hs, k, kr->y);
   for (int c0 = 0; c0 < k; c0 += kChunk)
-    k_combine<<<kRedBlocks, kThreads, 0, s>>>(n, std::min(kChunk, k - c0), Z + (long)c0 * n,
+    k_combine<<<red_blocks(n), kThreads, 0, s>>>(n, std::min(kChunk, k - c0), Z + (long)c0 * n,
                                               kr->y + c0, x);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
@@ -394,7 +400,7 @@ extern "C" int fv_krylov_norm(FvKrylov* kr, long n, const double* x, double* out
   }
   cudaStream_t s = (cudaStream_t)stream;
   // k = 0: x is only read
-  k_upd_norm<<<kRedBlocks, kThreads, 0, s>>>(n, 0, nullptr, nullptr, const_cast<double*>(x),
+  k_upd_norm<<<red_blocks(n), kThreads, 0, s>>>(n, 0, nullptr, nullptr, const_cast<double*>(x),
                                               kr->part, kr->ticket, kr->red, kr->hs, NM_ONLY, -1,
                                               nullptr, nullptr, out);
   FV_CUDA_TRY(cudaGetLastError());
