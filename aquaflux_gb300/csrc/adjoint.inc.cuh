@@ -217,6 +217,7 @@ template <int DIM, bool TURB>
 __global__ void __launch_bounds__(128) a_sum(MeshView m, CaseView cv, Src<double> st, Par<double> par,
                                              const double* W, const double* cl, const double* G,
                                              const double* Gwi, AdjWork aw) {
+  stage_begin();
   a_sum_at<DIM, TURB>(stage_cell(m, cv), m, cv, st, par, W, cl, G, Gwi, aw);
 }
 
@@ -557,6 +558,7 @@ template <int DIM, bool TURB, bool FLX = false, bool LIM = false>
 __global__ void __launch_bounds__(128) a_flux(MeshView m, CaseView cv, Src<double> st, Par<double> par,
                                               const double* G, const double* cl, const double* dco,
                                               const double* me, const double* aux, AdjWork aw) {
+  stage_begin();
   a_flux_at<DIM, TURB, FLX, LIM>(stage_cell(m, cv), m, cv, st, par, G, cl, dco, me, aux, aw);
 }
 
@@ -568,6 +570,7 @@ __global__ void __launch_bounds__(128) a_flux(MeshView m, CaseView cv, Src<doubl
 template <int DIM, bool TURB>
 __global__ void __launch_bounds__(128) a_limiter(MeshView m, Src<double> st, const double* G,
                                                  double Km, double Ks, AdjWork aw) {
+  stage_begin();
   constexpr int NA = DIM + (TURB ? 2 : 0);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nc) return;
@@ -613,6 +616,7 @@ __global__ void __launch_bounds__(128) a_limiter(MeshView m, Src<double> st, con
 
 template <int DIM, bool TURB>
 __global__ void a_limiter_gather(MeshView m, AdjWork aw) {
+  stage_begin();
   constexpr int NA = DIM + (TURB ? 2 : 0);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nc) return;
@@ -711,6 +715,7 @@ template <int DIM, bool TURB>
 __global__ void __launch_bounds__(128) a_apcoef(MeshView m, CaseView cv, Src<double> st, Par<double> par,
                                                 const double* G, const double* cl, const double* dco,
                                                 const double* me, const double* aux, AdjWork aw) {
+  stage_begin();
   a_apcoef_at<DIM, TURB>(stage_cell(m, cv), m, cv, st, par, G, cl, dco, me, aux, aw);
 }
 
@@ -889,6 +894,7 @@ __device__ __forceinline__ void a_closure_at(const int c, MeshView m, CaseView c
 template <int DIM>
 __global__ void __launch_bounds__(128) a_closure(MeshView m, CaseView cv, Src<double> st, Par<double> par,
                                                  const double* G, const double* cl, AdjWork aw) {
+  stage_begin();
   a_closure_at<DIM>(stage_cell(m, cv), m, cv, st, par, G, cl, aw);
 }
 
@@ -904,6 +910,7 @@ __global__ void __launch_bounds__(128) a_closure(MeshView m, CaseView cv, Src<do
 template <int DIM, int NQ>
 __global__ void __launch_bounds__(128) a_gg_skew(MeshView m, const double* Xb, double rel,
                                                  double* wb) {
+  stage_begin();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= m.nfi) return;
   const int nc = m.nc, nf = m.nf;
@@ -926,6 +933,7 @@ __global__ void __launch_bounds__(128) a_gg_skew(MeshView m, const double* Xb, d
 template <int DIM, int NQ>
 __global__ void __launch_bounds__(128) a_gg_sweep(MeshView m, const double* Xb, const double* wb,
                                                   double rel, bool first, double* Bb, double* Xbn) {
+  stage_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.nc) return;
   const int nc = m.nc, nf = m.nf;
@@ -971,8 +979,8 @@ const double* gg_sweeps_adjoint(const MeshView& m, int sweeps, double rel, const
   double* cur = aw.Gb;
   double* nxt = aw.Gb2;
   for (int it = 1; it < sweeps; ++it) {
-    if (m.nfi > 0) a_gg_skew<DIM, NQ><<<bfi, TB, 0, s>>>(m, cur, rel, wface);
-    a_gg_sweep<DIM, NQ><<<bc, TB, 0, s>>>(m, cur, wface, rel, it == 1, aw.Bb, nxt);
+    if (m.nfi > 0) stage(a_gg_skew<DIM, NQ>, bfi, TB, s, m, cur, rel, wface);
+    stage(a_gg_sweep<DIM, NQ>, bc, TB, s, m, cur, wface, rel, it == 1, aw.Bb, nxt);
     double* t = cur;
     cur = nxt;
     nxt = t;
@@ -1049,6 +1057,7 @@ template <int DIM, bool TURB>
 __global__ void __launch_bounds__(128) a_grad_face(MeshView m, CaseView cv, AdjWork aw,
                                                    const double* Gb0, const double* Bb, double rel,
                                                    double* pb) {
+  stage_begin();
   a_grad_face_at<DIM, TURB>(blockIdx.x * blockDim.x + threadIdx.x, m, cv, aw, Gb0, Bb, rel, pb);
 }
 
@@ -1093,5 +1102,6 @@ __device__ __forceinline__ void a_grad_at(const int c, MeshView m, CaseView cv, 
 template <int DIM, bool TURB>
 __global__ void __launch_bounds__(128) a_grad(MeshView m, CaseView cv, AdjWork aw, const double* pb,
                                               double* out) {
+  stage_begin();
   a_grad_at<DIM, TURB>(stage_cell(m, cv), m, cv, aw, pb, out);
 }
