@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(128) k_nadj_face(MeshView m, CaseView cv, cons
   double nb_[DIM], skb[DIM], xfb[DIM], xob[DIM], xnb[DIM];
 #pragma unroll
   for (int j = 0; j < DIM; ++j) nb_[j] = skb[j] = xfb[j] = xob[j] = xnb[j] = 0.0;
-  const double abo = -aw.dcob[o] * dco[o] * dco[o] * m.inv_vol[o];
+  const double abo = aw.apb[o];
   const double mest = me[f];
   // the cotangent of a limited reconstruction at upwind cell cu (psi itself: k_nadj_limiter)
   auto rec_adj = [&](int a, int q, bool own, double t) {
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(128) k_nadj_face(MeshView m, CaseView cv, cons
     const double mn_ = TURB ? par.mu + rho * cl[2L * nc + n] : mu_at(par, cv, n);
     const double dpn = m.dpn[f], dnn = m.dnn[f], inv_nd = m.inv_nd[f], nn2 = m.nn2[f];
     const double mdot = aux[f], damping = aux[1L * nf + f], dhat = aux[2L * nf + f];
-    const double abn = -aw.dcob[n] * dco[n] * dco[n] * m.inv_vol[n];
+    const double abn = aw.apb[n];
     const bool out = mdot >= 0.0;
     double dv[DIM], sk[DIM], tPb[DIM], tNb[DIM], gpfb[DIM];
 #pragma unroll

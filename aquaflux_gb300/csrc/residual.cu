@@ -610,6 +610,23 @@ void gg_sweeps(const MeshView& m, int sweeps, double rel, const T* Bg, T* G0, T*
 }
 
 // ---------------------------------------------------------------- k_closure (SST)
+// 2 s_ij s_ij of the strain rate s = sym grad u, each pair of off-diagonal entries once (10 fp64
+// instructions in 3D, 28 entry by entry).
+template <class T, int DIM>
+__device__ __forceinline__ T strain2(const T (&gu)[DIM][DIM]) {
+  T diag = cst(0.0, gu[0][0]), off = diag;
+#pragma unroll
+  for (int i = 0; i < DIM; ++i) {
+    diag += gu[i][i] * gu[i][i];
+#pragma unroll
+    for (int j = i + 1; j < DIM; ++j) {
+      const T x = gu[i][j] + gu[j][i];
+      off += x * x;
+    }
+  }
+  return 2.0 * diag + off;
+}
+
 // The closure of cell c: out = (S, F1, nu_t, wall shear rate, k diffusivity, omega diffusivity,
 // F2), gw = the omega gradient with the wall-cell value imposed.
 template <class T, int DIM, class S_, class GV, class GP>
@@ -624,15 +641,20 @@ __device__ __forceinline__ void closure_cell(const MeshView& m, const CaseView& 
   for (int i = 0; i < DIM; ++i)
 #pragma unroll
     for (int j = 0; j < DIM; ++j) gu[i][j] = G[((long)i * DIM + j) * nc + c];
-  T sum = cst(0.0, gu[0][0]);
+  T S;
+  if constexpr (!IsF32<T>::value) {
+    S = safe_sqrt(strain2<T, DIM>(gu));
+  } else {
+    T sum = cst(0.0, gu[0][0]);
 #pragma unroll
-  for (int i = 0; i < DIM; ++i)
+    for (int i = 0; i < DIM; ++i)
 #pragma unroll
-    for (int j = 0; j < DIM; ++j) {
-      T sij = 0.5 * (gu[i][j] + gu[j][i]);
-      sum += sij * sij;
-    }
-  T S = safe_sqrt(2.0 * sum);
+      for (int j = 0; j < DIM; ++j) {
+        T sij = 0.5 * (gu[i][j] + gu[j][i]);
+        sum += sij * sij;
+      }
+    S = safe_sqrt(2.0 * sum);
+  }
   const T k = st((long)L::K * nc + c);
   const T w = st((long)L::W * nc + c);
   const T nu = par.nu;
@@ -743,16 +765,33 @@ template <class T, int DIM, bool TURB, class S, class GV, class GT>
 __device__ __forceinline__ T mom_normal(const MeshView& m, const S& st, const T* G, GS<T> rho,
                                         int f, int o, int n, GT g, const GV& gv) {
   const int nc = m.nc;
-  T mn = cst(0.0, st(o));
+  if constexpr (IsF32<T>::value) {
+    T mn = cst(0.0, st(o));
+#pragma unroll
+    for (int j = 0; j < DIM; ++j) {
+      mn += gv.normal(m, j, f) * lerp(st((long)j * nc + o), st((long)j * nc + n), g);
+#pragma unroll
+      for (int q = 0; q < DIM; ++q)
+        mn += gv.ns(m, j * DIM + q, f) *
+              lerp(G[((long)j * DIM + q) * nc + o], G[((long)j * DIM + q) * nc + n], g);
+    }
+    return rho * mn;
+  }
+  // fp64: each side's sum, then one blend of the two (3D: 26 fp64 instructions for 36)
+  T mo = gv.normal(m, 0, f) * st(o), mn = gv.normal(m, 0, f) * st(n);
 #pragma unroll
   for (int j = 0; j < DIM; ++j) {
-    mn += gv.normal(m, j, f) * lerp(st((long)j * nc + o), st((long)j * nc + n), g);
+    if (j > 0) {
+      mo += gv.normal(m, j, f) * st((long)j * nc + o);
+      mn += gv.normal(m, j, f) * st((long)j * nc + n);
+    }
 #pragma unroll
-    for (int q = 0; q < DIM; ++q)
-      mn += gv.ns(m, j * DIM + q, f) *
-            lerp(G[((long)j * DIM + q) * nc + o], G[((long)j * DIM + q) * nc + n], g);
+    for (int q = 0; q < DIM; ++q) {
+      mo += gv.ns(m, j * DIM + q, f) * G[((long)j * DIM + q) * nc + o];
+      mn += gv.ns(m, j * DIM + q, f) * G[((long)j * DIM + q) * nc + n];
+    }
   }
-  return rho * mn;
+  return rho * lerp(mo, mn, g);
 }
 
 // flux-continuous conductance g_o A / (dpn - g_o / g_n dnn), one division
@@ -761,6 +800,32 @@ template <class T, class GT>
 __device__ __forceinline__ T conductance(T go, T gn, GT A, GT dpn, GT dnn) {
   return go * gn * A / (dpn * gn - go * dnn);
 }
+
+// The conductance c = g_o g_n A / den, den = dpn g_n - g_o dnn, of a flux stage, and its derivatives
+// in g_o and g_n, d c / d g_o = A dpn (g_n / den)^2 and d c / d g_n = -A dnn (g_o / den)^2: two
+// products each behind the ratios, where c's own form costs five.
+template <class T>
+struct Conduct {
+  T c, ro, rn;  // ro = g_o / den, rn = g_n / den
+  double ao, an;
+  template <class GT>
+  __device__ __forceinline__ Conduct(const T& go, const T& gn, GT A, GT dpn, GT dnn) {
+    const T iden = 1.0 / (dpn * gn - go * dnn);
+    if constexpr (IsF32<T>::value) {
+      c = go * gn * A * iden;
+    } else {
+      rn = gn * iden;
+      c = go * rn * A;
+      if constexpr (std::is_same<T, double>::value) {
+        ro = go * iden;
+        ao = A * dpn;
+        an = A * dnn;
+      }
+    }
+  }
+  __device__ __forceinline__ double d_owner() const { return ao * rn * rn; }
+  __device__ __forceinline__ double d_neighbour() const { return -(an * ro * ro); }
+};
 
 // ---------------------------------------------------------------- slope limiter
 // VenkatakrishnanLimiter.limit (aquaflux/schemes/limiter.py:78-117) of one field at cell c:
@@ -922,16 +987,20 @@ __global__ void __launch_bounds__(128) k_apcoef_tangent(MeshView m, CaseView cv,
   const long nc = m.nc, nf = m.nf;
   const int o = m.owner[f], n = m.nb[f];
   const double g = m.g[f], A = m.area[f], rho = cv.rho;
-  double mn_t = 0.0;
+  double so_t = 0.0, sn_t = 0.0;  // each side's sum (mom_normal)
 #pragma unroll
   for (int j = 0; j < DIM; ++j) {
-    mn_t += m.normal[(long)j * nf + f] * lerp(st((long)j * nc + o).d, st((long)j * nc + n).d, g);
+    const double nj = m.normal[(long)j * nf + f];
+    so_t += nj * st((long)j * nc + o).d;
+    sn_t += nj * st((long)j * nc + n).d;
 #pragma unroll
-    for (int q = 0; q < DIM; ++q)
-      mn_t += m.ns[(long)(j * DIM + q) * nf + f] *
-              lerp(G[((long)j * DIM + q) * nc + o].d, G[((long)j * DIM + q) * nc + n].d, g);
+    for (int q = 0; q < DIM; ++q) {
+      const double x = m.ns[(long)(j * DIM + q) * nf + f];
+      so_t += x * G[((long)j * DIM + q) * nc + o].d;
+      sn_t += x * G[((long)j * DIM + q) * nc + n].d;
+    }
   }
-  const double me_t = (rho * mn_t) * A;
+  const double me_t = (rho * lerp(so_t, sn_t, g)) * A;
   const double mo_t = TURB ? rho * cl[2L * nc + o].d : 0.0;
   const double mn_c = TURB ? rho * cl[2L * nc + n].d : 0.0;
   const double visc_t = aux[4L * nf + f] * mo_t + aux[5L * nf + f] * mn_c;
@@ -1082,8 +1151,8 @@ __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv,
     const T mdot = mest - (rho * A) * dhat * damping;
     const T pf = lerp(po, pn, g) + gs;
     const T mnb = mu_eff<T, TURB>(par, cv, rho, cl, nc, n);
-    const T iden = 1.0 / (gv.dpn(m, f) * mnb - mo * gv.dnn(m, f));
-    const T cmo = mo * mnb * A * iden;
+    const Conduct<T> cm(mo, mnb, A, gv.dpn(m, f), gv.dnn(m, f));
+    const T cmo = cm.c;
     const bool out = val(mdot) >= 0.0;
     const T pA = pf * A;
     using AX = Aux<DIM, TURB>;
@@ -1093,8 +1162,8 @@ __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv,
         aux[1L * nf + f] = damping;
         aux[2L * nf + f] = dhat;
         aux[3L * nf + f] = cmo;
-        aux[4L * nf + f] = (mnb * A * iden) * (1.0 + mo * m.dnn[f] * iden);
-        aux[5L * nf + f] = (mo * A * iden) * (1.0 - mnb * m.dpn[f] * iden);
+        aux[4L * nf + f] = cm.d_owner();
+        aux[5L * nf + f] = cm.d_neighbour();
       }
     }
 #pragma unroll
@@ -1125,8 +1194,8 @@ __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv,
 #pragma unroll
         for (int j = 0; j < DIM; ++j)
           cpn += G[((long)q * DIM + j) * nc + n] * tN[j] - G[((long)q * DIM + j) * nc + o] * tP[j];
-        const T idn = 1.0 / (gv.dpn(m, f) * gn - go * gv.dnn(m, f));
-        const T cs_ = go * gn * A * idn;
+        const Conduct<T> cq(go, gn, A, gv.dpn(m, f), gv.dnn(m, f));
+        const T cs_ = cq.c;
         const T* ps = cv.rec_sca ? psi : nullptr;
         const T up = vout ? upwind_rec<T, DIM>(m, G, ps, DIM + s, q, f, o, phio, gv)
                           : upwind_rec<T, DIM>(m, G, ps, DIM + s, q, f, n, phin, gv);
@@ -1135,8 +1204,8 @@ __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv,
           if (aux) {
             const long b0 = AX::S0 + 4 * s;
             aux[b0 * nf + f] = cs_;
-            aux[(b0 + 1) * nf + f] = (gn * A * idn) * (1.0 + go * m.dnn[f] * idn);
-            aux[(b0 + 2) * nf + f] = (go * A * idn) * (1.0 - gn * m.dpn[f] * idn);
+            aux[(b0 + 1) * nf + f] = cq.d_owner();
+            aux[(b0 + 2) * nf + f] = cq.d_neighbour();
             aux[(b0 + 3) * nf + f] = cpn;
           }
         }
@@ -1602,11 +1671,14 @@ __global__ void __launch_bounds__(128) k_closure_lin(MeshView m, CaseView cv, Sr
       gv[i][j] = g.v;
       gd[i][j] = g.d;
     }
-  double ss = 0.0;
+  double ss = 0.0, off = 0.0;  // s_ij (grad u)'_ij, each off-diagonal pair once
 #pragma unroll
-  for (int i = 0; i < DIM; ++i)
+  for (int i = 0; i < DIM; ++i) {
+    ss += gv[i][i] * gd[i][i];
 #pragma unroll
-    for (int j = 0; j < DIM; ++j) ss += (0.5 * (gv[i][j] + gv[j][i])) * gd[i][j];
+    for (int j = i + 1; j < DIM; ++j) off += (gv[i][j] + gv[j][i]) * (gd[i][j] + gd[j][i]);
+  }
+  ss += 0.5 * off;
   const double t[4] = {st.t ? st.t[(long)L::K * nc + c] : 0.0,
                        st.t ? st.t[(long)L::W * nc + c] : 0.0, cc[c] * ss, 0.0};
   double ddot = 0.0;
@@ -1846,6 +1918,7 @@ AdjWork adj_layout(FvCase* cs) {
   aw.sb = p; p += L::NFLD * nc;
   aw.Gb = p; p += L::NFLD * DIM * nc;
   aw.dcob = p; p += nc;
+  aw.apb = p; p += nc;
   aw.clb = p; p += 4 * nc;
   aw.Gwib = p; p += DIM * nc;
   aw.Gb2 = p; p += L::NFLD * DIM * nc;  // present when the case is swept
@@ -2054,7 +2127,7 @@ bool g_const_ready = false;
 
 size_t fv_adjoint_work_bytes(int dim, int turb, long nc, long nf, int sweeps, int advection) {
   long nfld = dim + 1 + (turb ? 2 : 0);
-  long n = 2 * nfld * nc + nfld * dim * nc + nc + 4 * nc + dim * nc;
+  long n = 2 * nfld * nc + nfld * dim * nc + 2 * nc + 4 * nc + dim * nc;
   // the sweeps' second iterate cotangent and B phi's (the limiter buffers follow them)
   if (sweeps >= 1 || advection >= 1) n += 2 * nfld * dim * nc;
   if (advection >= 1) n += (long)(dim + (turb ? 2 : 0)) * (nc + 2 * nf);
