@@ -369,11 +369,12 @@ extern "C" int fv_case_destroy(FvCase* c) {
   cudaFree(c->wnear);
   cudaFree(c->sched);
   cudaFree(c->lin_aux);
-  cudaFree(c->lin_fl);
-  cudaFree(c->lin_ac);
+  cudaFree(c->lin_me);
+  cudaFree(c->lin_d);
   cudaFree(c->lin_g);
   cudaFree(c->lin_r);
   cudaFree(c->lin_cl);
+  cudaFree(c->wall_cells);
   cudaFree(c->lin_cc);
   cudaFree(c->lin_src);
   fv_node_adjoint_free(c);

@@ -153,15 +153,17 @@ struct FvCase {
   int* sched = nullptr;         // (nc) warp-coherent cell order of the cell stages
   int n_cell_classes = 0;       // distinct face-list patterns it groups
   double* lin_aux = nullptr;    // face intermediates of the held linearisation (fv_case_linearise)
-  double* lin_fl = nullptr;     // ... and its primal face fluxes (nfld, nf)
-  double* lin_ac = nullptr;     // ... its face coefficients and mass-flux estimates (3, nf)
+  double* lin_me = nullptr;     // ... its mass-flux estimates (nf)
+  double* lin_d = nullptr;      // ... its d = V / a_P (nc)
   double* lin_g = nullptr;      // ... its gradients (nfld, dim, nc)
   double* lin_r = nullptr;      // ... its residual (nfld, nc)
   double* lin_cl = nullptr;     // ... its SST closure fields (7, nc)
-  double* lin_cc = nullptr;     // ... the off-wall closure and source forms (29, nc)
+  double* lin_cc = nullptr;     // ... the off-wall closure and source forms (21, nc)
   double* lin_src = nullptr;    // a product's off-wall k / omega source tangents (2, nc)
+  int* wall_cells = nullptr;    // the SST wall cells, listed by the first linearisation
+  int n_wall_cells = -1;        // ... their number (-1: not listed yet)
   int lin_valid = 0;            // a linearisation is held (parameter / geometry changes clear it)
-  int lin_use = 0;              // the running dual-number pass takes its flux stage from it
+  int lin_use = 0;              // the running pass is a product at it
   int fwd_valid = 0;            // work / aux hold the double forward pass of the last VJP's state
   double* mu_cell = nullptr;    // (nc) per-cell viscosity field (laminar batched instances)
   double* flx = nullptr;        // (nfld, nf) weights of a face-flux functional (internal order)

@@ -752,8 +752,8 @@ __device__ __forceinline__ Dual mu_at(const Par<Dual>& par, const CaseView& cv, 
 __device__ __forceinline__ DualF mu_at(const Par<DualF>& par, const CaseView& cv, int c) {
   return cv.mu_cell ? DualF{cv.f_mu_cell[c], par.mu.d} : par.mu;
 }
-template <class T, bool TURB>
-__device__ __forceinline__ T mu_eff(const Par<T>& par, const CaseView& cv, GS<T> rho, const T* cl,
+template <class T, bool TURB, class CP>
+__device__ __forceinline__ T mu_eff(const Par<T>& par, const CaseView& cv, GS<T> rho, const CP& cl,
                                     int nc, int c) {
   if (TURB) return par.mu + rho * cl[2L * nc + c];
   return mu_at(par, cv, c);
@@ -761,8 +761,8 @@ __device__ __forceinline__ T mu_eff(const Par<T>& par, const CaseView& cv, GS<T>
 
 // lagged advective momentum flux (rho u)_f . n with the skew-corrected face value
 // (aquaflux/flow/rhie_chow.py:220-271): rho (sum_j n_j u_j,f + sum_jq n_j skew_q (grad u)_jq,f)
-template <class T, int DIM, bool TURB, class S, class GV, class GT>
-__device__ __forceinline__ T mom_normal(const MeshView& m, const S& st, const T* G, GS<T> rho,
+template <class T, int DIM, bool TURB, class S, class GP, class GV, class GT>
+__device__ __forceinline__ T mom_normal(const MeshView& m, const S& st, const GP& G, GS<T> rho,
                                         int f, int o, int n, GT g, const GV& gv) {
   const int nc = m.nc;
   if constexpr (IsF32<T>::value) {
@@ -901,8 +901,8 @@ __global__ void __launch_bounds__(128) k_limiter(MeshView m, Src<T> st, const T*
 
 // The advected face value of field q through face f from the upwind cell cu (upwind_value, the
 // cell value; with a limiter, plus psi grad . (x_f - x_cu)).
-template <class T, int DIM, class GV>
-__device__ __forceinline__ T upwind_rec(const MeshView& m, const T* G, const T* psi, int a, int q,
+template <class T, int DIM, class GP, class GV>
+__device__ __forceinline__ T upwind_rec(const MeshView& m, const GP& G, const T* psi, int a, int q,
                                         int f, int cu, const T& value, const GV& gv) {
   if (!psi) return value;
   const int nc = m.nc;
@@ -916,9 +916,9 @@ __device__ __forceinline__ T upwind_rec(const MeshView& m, const T* G, const T* 
 // ---------------------------------------------------------------- k_apcoef
 // The momentum-diagonal face coefficients of face f (owner side, neighbour side) and the lagged
 // mass-flux estimate me.
-template <class T, int DIM, bool TURB, class S_, class GV>
+template <class T, int DIM, bool TURB, class S_, class GP, class CP, class GV>
 __device__ __forceinline__ void apcoef_face(const MeshView& m, const CaseView& cv, const S_& st,
-                                            const Par<T>& par, const T* G, const T* cl, int f,
+                                            const Par<T>& par, const GP& G, const CP& cl, int f,
                                             const GV& gv, T& ac_own, T& ac_nb, T& me) {
   using L = Layout<DIM, TURB>;
   using GT = decltype(gv.area(m, 0));
@@ -971,112 +971,6 @@ __global__ void __launch_bounds__(128) k_apcoef(MeshView m, CaseView cv, Src<T> 
   k_apcoef_at<T, DIM, TURB>(face0 + blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, ac_own, ac_nb, me);
 }
 
-// The interior faces' momentum-diagonal coefficients and mass-flux estimate of a state-tangent
-// dual-number pass at a held linearisation: the momentum-normal flux is linear in the velocities
-// and their gradients, the conductance's tangent comes from its kept partial derivatives in the
-// cell viscosities, max(., 0) follows the kept sign of the estimate (JAX's tie rule); the primal
-// values are the kept ones (lin: owner coefficient, neighbour coefficient, estimate).
-template <int DIM, bool TURB>
-__global__ void __launch_bounds__(128) k_apcoef_tangent(MeshView m, CaseView cv, Src<Dual> st,
-                                                        const Dual* G, const Dual* cl,
-                                                        const double* aux, const double* lin,
-                                                        Dual* ac_own, Dual* ac_nb, Dual* me) {
-  stage_begin();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= m.nfi) return;
-  const long nc = m.nc, nf = m.nf;
-  const int o = m.owner[f], n = m.nb[f];
-  const double g = m.g[f], A = m.area[f], rho = cv.rho;
-  double so_t = 0.0, sn_t = 0.0;  // each side's sum (mom_normal)
-#pragma unroll
-  for (int j = 0; j < DIM; ++j) {
-    const double nj = m.normal[(long)j * nf + f];
-    so_t += nj * st((long)j * nc + o).d;
-    sn_t += nj * st((long)j * nc + n).d;
-#pragma unroll
-    for (int q = 0; q < DIM; ++q) {
-      const double x = m.ns[(long)(j * DIM + q) * nf + f];
-      so_t += x * G[((long)j * DIM + q) * nc + o].d;
-      sn_t += x * G[((long)j * DIM + q) * nc + n].d;
-    }
-  }
-  const double me_t = (rho * lerp(so_t, sn_t, g)) * A;
-  const double mo_t = TURB ? rho * cl[2L * nc + o].d : 0.0;
-  const double mn_c = TURB ? rho * cl[2L * nc + n].d : 0.0;
-  const double visc_t = aux[4L * nf + f] * mo_t + aux[5L * nf + f] * mn_c;
-  const double e = lin[2L * nf + f];
-  const double pp = e > 0.0 ? me_t : (e < 0.0 ? 0.0 : 0.5 * me_t);
-  const double pm = e < 0.0 ? -me_t : (e > 0.0 ? 0.0 : 0.5 * -me_t);
-  ac_own[f] = Dual{lin[f], visc_t + pp};
-  ac_nb[f] = Dual{lin[(long)nf + f], visc_t + pm};
-  me[f] = Dual{e, me_t};
-}
-
-// The compact Green-Gauss gradients of a state-tangent dual-number pass at a held linearisation:
-// the scheme is linear, so the tangents are the face-value tangents' gradients (boundary values by
-// the dual-number closures) and the primal gradients are the kept ones.
-template <int DIM, bool TURB>
-__global__ void __launch_bounds__(128) k_grad_tangent(MeshView m, CaseView cv, Src<Dual> st,
-                                                      Par<Dual> par, const double* Gp, Dual* G) {
-  stage_begin();
-  using L = Layout<DIM, TURB>;
-  constexpr int NF = L::NFLD;
-  const int c = stage_cell<Dual>(m, cv);
-  if (c >= m.nc) return;
-  const int nc = m.nc, nf = m.nf;
-  Dual phic[NF];
-#pragma unroll
-  for (int q = 0; q < NF; ++q) phic[q] = st((long)q * nc + c);
-  double acc[NF][DIM];
-#pragma unroll
-  for (int q = 0; q < NF; ++q)
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) acc[q][j] = 0.0;
-  const int b = m.cf_ptr[c], e = m.cf_ptr[c + 1];
-  for (int i = b; i < e; ++i) {
-    const unsigned ent = m.cf_face[i];
-    const int f = (int)(ent & ~FV_NB_BIT);
-    const bool isnb = (ent & FV_NB_BIT) != 0;
-    const double af = m.area[f];
-    const double A = isnb ? -af : af;
-    double S[DIM];
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) S[j] = m.normal[(long)j * nf + f] * A;
-    double phif[NF];
-    if (f < m.nfi) {
-      const double g = m.g[f];
-      const int other = isnb ? m.owner[f] : m.nb[f];
-#pragma unroll
-      for (int q = 0; q < NF; ++q) {
-        const double po = st((long)q * nc + other).d;
-        phif[q] = lerp(isnb ? po : phic[q].d, isnb ? phic[q].d : po, g);
-      }
-    } else {
-      const signed char kind = cv.fkind[f];
-#pragma unroll
-      for (int j = 0; j < DIM; ++j) phif[j] = bvel(cv, nf, f, j, kind, phic[j], par).d;
-      phif[L::P] = bpress(cv, f, kind, phic[L::P]).d;
-      if (TURB) {
-        const Dual z = cst(0.0, phic[0]);
-        phif[L::K] = bscalar(cv.kkind[f], cv.kval[f], phic[L::K], z).d;
-        phif[L::W] = bscalar(cv.wkind[f], cv.wval[f], phic[L::W], z).d;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < NF; ++q)
-#pragma unroll
-      for (int j = 0; j < DIM; ++j) acc[q][j] += S[j] * phif[q];
-  }
-  const double inv = m.inv_vol[c];
-#pragma unroll
-  for (int q = 0; q < NF; ++q)
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) {
-      const long k = ((long)q * DIM + j) * nc + c;
-      G[k] = Dual{Gp[k], acc[q][j] * inv};
-    }
-}
-
 // ---------------------------------------------------------------- k_dcoeff
 template <class T>
 __device__ __forceinline__ void k_dcoeff_at(const int c, MeshView m, const T* ac_own, const T* ac_nb, T* dco) {
@@ -1111,9 +1005,10 @@ struct Aux {
 
 // The fluxes of face f, handed to wr(q, flux_q) for every field q.  `st` reads the state (Src, or
 // a seeded accessor in the Jacobian assembly); aux (double only) receives the face intermediates.
-template <class T, int DIM, bool TURB, class S, class Wr, class GV = typename GeoOf<T>::type>
+template <class T, int DIM, bool TURB, class S, class GP, class CP, class DP, class Wr,
+          class GV = typename GeoOf<T>::type>
 __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv, const S& st,
-                                          const Par<T>& par, const T* G, const T* cl, const T* dco,
+                                          const Par<T>& par, const GP& G, const CP& cl, const DP& dco,
                                           const T* me, const T* psi, bool recompute_me, int f,
                                           const Wr& wr, double* aux, const GV& gv = GV{}) {
   using GT = decltype(gv.area(m, 0));
@@ -1308,89 +1203,6 @@ __global__ void __launch_bounds__(128) k_flux(MeshView m, CaseView cv, Src<T> st
   k_flux_at<T, DIM, TURB>(face0 + blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, dco, me, psi, recompute_me, FL, aux);
 }
 
-// The interior face fluxes of a state-tangent dual-number pass at a held linearisation (first-order
-// upwind): the primal face intermediates the double pass kept (mass flux, pressure damping,
-// interpolated d, conductances and their partial derivatives in the cell diffusivities, the
-// cross-diffusion numerators) stand in for their recomputation, so only the tangent arithmetic of
-// flux_face runs -- the forward-mode counterpart of the adjoint's use of the same intermediates.
-// The primal fluxes are the kept ones.  Mass-flux estimate, gradients, closure and d arrive as dual
-// numbers from the pass's earlier stages.
-template <int DIM, bool TURB>
-__global__ void __launch_bounds__(128) k_flux_tangent(MeshView m, CaseView cv, Src<Dual> st,
-                                                      const Dual* G, const Dual* cl,
-                                                      const Dual* dco, const Dual* me,
-                                                      const double* aux, const double* flp,
-                                                      Dual* FL) {
-  stage_begin();
-  using L = Layout<DIM, TURB>;
-  using AX = Aux<DIM, TURB>;
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= m.nfi) return;
-  const long nc = m.nc, nf = m.nf;
-  const int o = m.owner[f], n = m.nb[f];
-  const double A = m.area[f], g = m.g[f];
-  const double rho = cv.rho, irho = 1.0 / cv.rho;
-  const double mdot = aux[0L * nf + f], damping = aux[1L * nf + f], dhat = aux[2L * nf + f];
-  const double cmo = aux[3L * nf + f], dcdo = aux[4L * nf + f], dcdn = aux[5L * nf + f];
-  double gd = 0.0, gs = 0.0;
-#pragma unroll
-  for (int j = 0; j < DIM; ++j) {
-    const double gpf = lerp(G[((long)L::P * DIM + j) * nc + o].d, G[((long)L::P * DIM + j) * nc + n].d, g);
-    gd += gpf * m.dvec[(long)j * nf + f];
-    gs += gpf * m.skew[(long)j * nf + f];
-  }
-  const double dhat_t = m.nn2[f] * lerp(dco[o].d, dco[n].d, g);
-  const Dual po = st((long)L::P * nc + o), pn = st((long)L::P * nc + n);
-  const double damp_t = ((pn.d - po.d) - gd) * m.inv_nd[f];
-  const double mdot_t = me[f].d - (rho * A) * (dhat_t * damping + dhat * damp_t);
-  const double pA_t = (lerp(po.d, pn.d, g) + gs) * A;
-  // d(mu + rho nu_t) for a state tangent (the molecular viscosity is a parameter)
-  const double mo_t = TURB ? rho * cl[2L * nc + o].d : 0.0;
-  const double mn_t = TURB ? rho * cl[2L * nc + n].d : 0.0;
-  const double cmo_t = dcdo * mo_t + dcdn * mn_t;
-  const bool out = mdot >= 0.0;
-  double tP[DIM], tN[DIM];
-#pragma unroll
-  for (int j = 0; j < DIM; ++j) {
-    tP[j] = m.tP[(long)j * nf + f];
-    tN[j] = m.tN[(long)j * nf + f];
-  }
-#pragma unroll
-  for (int i = 0; i < DIM; ++i) {
-    const Dual uo = st((long)i * nc + o), un = st((long)i * nc + n);
-    double cpn_t = un.d - uo.d;
-#pragma unroll
-    for (int j = 0; j < DIM; ++j)
-      cpn_t += G[((long)i * DIM + j) * nc + n].d * tN[j] - G[((long)i * DIM + j) * nc + o].d * tP[j];
-    const double cpn = aux[(long)(AX::CPN + i) * nf + f];
-    const double up = out ? uo.v : un.v, up_t = out ? uo.d : un.d;
-    const double ft = (pA_t * m.normal[(long)i * nf + f] - (cmo_t * cpn + cmo * cpn_t)) +
-                      (mdot_t * up + mdot * up_t);
-    FL[(long)i * nf + f] = Dual{flp[(long)i * nf + f], ft};
-  }
-  FL[(long)L::P * nf + f] = Dual{flp[(long)L::P * nf + f], mdot_t};
-  if (TURB) {
-    const double vflux = mdot * irho, vflux_t = mdot_t * irho;
-    const bool vout = vflux >= 0.0;
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int q = s == 0 ? L::K : L::W;
-      const long b0 = AX::S0 + 4 * s;
-      const double go_t = cl[(4L + s) * nc + o].d, gn_t = cl[(4L + s) * nc + n].d;
-      const Dual phio = st((long)q * nc + o), phin = st((long)q * nc + n);
-      double cpn_t = phin.d - phio.d;
-#pragma unroll
-      for (int j = 0; j < DIM; ++j)
-        cpn_t += G[((long)q * DIM + j) * nc + n].d * tN[j] - G[((long)q * DIM + j) * nc + o].d * tP[j];
-      const double cs = aux[b0 * nf + f], cpn = aux[(b0 + 3) * nf + f];
-      const double cs_t = aux[(b0 + 1) * nf + f] * go_t + aux[(b0 + 2) * nf + f] * gn_t;
-      const double up = vout ? phio.v : phin.v, up_t = vout ? phio.d : phin.d;
-      const double ft = (vflux_t * up + vflux * up_t) - (cs_t * cpn + cs * cpn_t);
-      FL[(long)q * nf + f] = Dual{flp[(long)q * nf + f], ft};
-    }
-  }
-}
-
 // ---------------------------------------------------------------- k_sum
 // SST rows of cell c: k and omega source terms added to the face sums rk / rw, and the omega
 // wall-cell fixation (aquaflux/turbulence/sources.py:60-412, fixed_value.py:124-158).
@@ -1468,284 +1280,6 @@ __global__ void __launch_bounds__(128) k_sum(MeshView m, CaseView cv, Src<T> st,
   k_sum_at<T, DIM, TURB>(stage_cell<T>(m, cv), m, cv, st, par, FL, cl, G, Gwi, R, JV);
 }
 
-// ---------------------------------------------------------------- linearised SST closure
-// Off the wall, the closure fields and the k / omega source terms of a cell depend on the state
-// through four scalars only: k, omega, the strain rate S and grad k . grad omega.  At a held
-// linearisation their tangents are therefore linear forms in those four tangents, tabulated once
-// per linearisation (k_lin_closure_coef) and applied by every Krylov product (k_closure_lin,
-// k_sum_lin) instead of the dual-number closure and source rows.  Wall cells (wall functions,
-// omega fixation) keep the dual-number path.
-
-// A value with N tangent directions, under the dual number's rules (max / min split the tangent
-// at a tie; safe_sqrt and the k >= 0 clamp give a zero tangent where they clamp).
-template <int N>
-struct DualV {
-  double v, d[N];
-};
-template <int N>
-__device__ __forceinline__ double val(const DualV<N>& x) { return x.v; }
-template <int N>
-__device__ __forceinline__ DualV<N> cst(double x, const DualV<N>&) {
-  DualV<N> r;
-  r.v = x;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = 0.0;
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualV<N> lin_comb(double v, double a, const DualV<N>& x, double b,
-                                            const DualV<N>& y) {  // value v, tangent a x' + b y'
-  DualV<N> r;
-  r.v = v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a * x.d[i] + b * y.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualV<N> scaled(double v, double a, const DualV<N>& x) {
-  DualV<N> r;
-  r.v = v;
-#pragma unroll
-  for (int i = 0; i < N; ++i) r.d[i] = a * x.d[i];
-  return r;
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator+(const DualV<N>& a, const DualV<N>& b) {
-  return lin_comb(a.v + b.v, 1.0, a, 1.0, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator-(const DualV<N>& a, const DualV<N>& b) {
-  return lin_comb(a.v - b.v, 1.0, a, -1.0, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator*(const DualV<N>& a, const DualV<N>& b) {
-  return lin_comb(a.v * b.v, b.v, a, a.v, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator/(const DualV<N>& a, const DualV<N>& b) {
-  const double r = 1.0 / b.v, q = a.v * r;
-  return lin_comb(q, r, a, -q * r, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator+(const DualV<N>& a, double b) { return scaled(a.v + b, 1.0, a); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator+(double a, const DualV<N>& b) { return scaled(a + b.v, 1.0, b); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator-(const DualV<N>& a, double b) { return scaled(a.v - b, 1.0, a); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator-(double a, const DualV<N>& b) { return scaled(a - b.v, -1.0, b); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator*(const DualV<N>& a, double b) { return scaled(a.v * b, b, a); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator*(double a, const DualV<N>& b) { return scaled(a * b.v, a, b); }
-template <int N>
-__device__ __forceinline__ DualV<N> operator/(const DualV<N>& a, double b) {
-  const double r = 1.0 / b;
-  return scaled(a.v * r, r, a);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> operator/(double a, const DualV<N>& b) {
-  const double r = 1.0 / b.v, q = a * r;
-  return scaled(q, -q * r, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> fv_max(const DualV<N>& a, const DualV<N>& b) {
-  if (a.v > b.v) return a;
-  if (a.v < b.v) return b;
-  return lin_comb(a.v, 0.5, a, 0.5, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> fv_min(const DualV<N>& a, const DualV<N>& b) {
-  if (a.v < b.v) return a;
-  if (a.v > b.v) return b;
-  return lin_comb(a.v, 0.5, a, 0.5, b);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> fv_sqrt(const DualV<N>& x) {
-  const double r = sqrt(x.v);
-  return scaled(r, 0.5 / r, x);
-}
-template <int N>
-__device__ __forceinline__ DualV<N> fv_tanh(const DualV<N>& x) {
-  const double t = tanh(x.v);
-  return scaled(t, 1.0 - t * t, x);
-}
-
-// The off-wall SST closure of closure_cell and source rows of sst_rows as functions of (S, k,
-// omega, grad k . grad omega), the same formulas: out = (F1, nu_t, k diffusivity, omega
-// diffusivity, F2, k source, omega source), the sources as they enter the face sums.
-template <class T>
-__device__ __forceinline__ void sst_off_wall(T S, T k, T w, T dot_kw, double nu, double id,
-                                             double id2, double V, T (&out)[7]) {
-  const T kp = pos(k);
-  const T iw = 1.0 / w;
-  const T cd = fv_max((2.0 * SIGMA_W2) * dot_kw * iw, cst(CROSS_FLOOR, w));
-  const T sk = safe_sqrt(kp);
-  const T vt = ((500.0 * id2) * nu) * iw;
-  const T c1 = sk * iw * (id / BETA_STAR);
-  const T arg1 = fv_min(fv_max(c1, vt), (4.0 * SIGMA_W2 * id2) * kp / cd);
-  const T a1sq = arg1 * arg1;
-  const T F1 = fv_tanh(a1sq * a1sq);
-  const T arg2 = fv_max(2.0 * c1, vt);
-  const T F2 = fv_tanh(arg2 * arg2);
-  const T nut = A1 * kp / fv_max(A1 * w, S * F2);
-  out[0] = F1;
-  out[1] = nut;
-  out[2] = nu + (SIGMA_K2 + F1 * (SIGMA_K1 - SIGMA_K2)) * nut;
-  out[3] = nu + (SIGMA_W2 + F1 * (SIGMA_W1 - SIGMA_W2)) * nut;
-  out[4] = F2;
-  const T limit = (PROD_RATIO * BETA_STAR) * kp * w;
-  const T lim = fv_min(nut * (S * S), limit);
-  out[5] = BETA_STAR * V * k * w - lim * V;
-  const T alpha = ALPHA_2 + F1 * (ALPHA_1 - ALPHA_2);
-  const T cap = limit / fv_max(nut, cst(NUT_FLOOR, nut));
-  const T beta = BETA_2 + F1 * (BETA_1 - BETA_2);
-  const T cross = (2.0 * SIGMA_W2) * (1.0 - F1) * dot_kw / w;
-  out[6] = V * (beta * (w * w) - alpha * fv_min(S * S, cap) - cross);
-}
-
-// Coefficients per cell (LIN_NCOEF rows of nc): 2 / S (the strain rate's tangent is
-// 2 / S sum_ij s_ij (grad u)'_ij, 0 where S = 0), then for each output of sst_off_wall its
-// linear form in (k', omega', S', (grad k . grad omega)').
-constexpr int LIN_NCOEF = 29;
-
-// At a held linearisation: keep the closure fields (hcl, 7 rows of nc) and tabulate the off-wall
-// cells' coefficients from the evaluation's state, gradients and closure fields.
-template <int DIM>
-__global__ void k_lin_closure_coef(MeshView m, CaseView cv, const double* state, const double* G,
-                                   const double* cl, double nu, double* hcl, double* cc) {
-  using L = Layout<DIM, true>;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.nc) return;
-  const long nc = m.nc;
-#pragma unroll
-  for (int q = 0; q < 7; ++q) hcl[q * nc + c] = cl[q * nc + c];
-  if (cv.wcell[c]) return;
-  const GeoPlain gv{};
-  const double S = cl[c];
-  cc[c] = S > 0.0 ? 2.0 / S : 0.0;
-  double dot = G[((long)L::K * DIM) * nc + c] * G[((long)L::W * DIM) * nc + c];
-#pragma unroll
-  for (int j = 1; j < DIM; ++j)
-    dot += G[((long)L::K * DIM + j) * nc + c] * G[((long)L::W * DIM + j) * nc + c];
-  DualV<4> in[4];
-  const double v0[4] = {state[(long)L::K * nc + c], state[(long)L::W * nc + c], S, dot};
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    in[a].v = v0[a];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) in[a].d[i] = a == i ? 1.0 : 0.0;
-  }
-  DualV<4> out[7];
-  sst_off_wall<DualV<4>>(in[2], in[0], in[1], in[3], nu, gv.inv_wd(cv, c), gv.inv_wd2(cv, c),
-                         gv.vol(m, c), out);
-#pragma unroll
-  for (int q = 0; q < 7; ++q)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) cc[(1L + 4 * q + i) * nc + c] = out[q].d[i];
-}
-
-// The closure stage of a Krylov product at the held linearisation: off the wall, the held fields
-// with tangents from the tabulated forms, the omega gradient passed through, and the k / omega
-// source tangents (src, 2 rows of nc) for k_sum_lin; wall cells by the dual-number closure.
-template <int DIM>
-__global__ void __launch_bounds__(128) k_closure_lin(MeshView m, CaseView cv, Src<Dual> st,
-                                                     Par<Dual> par, const Dual* G,
-                                                     const double* hcl, const double* cc, Dual* cl,
-                                                     Dual* Gwi, double* src) {
-  stage_begin();
-  using L = Layout<DIM, true>;
-  const int c = stage_cell<Dual>(m, cv);
-  if (c >= m.nc) return;
-  if (cv.wcell[c]) {
-    k_closure_at<Dual, DIM>(c, m, cv, st, par, G, cl, Gwi);
-    return;
-  }
-  const long nc = m.nc;
-  double gv[DIM][DIM], gd[DIM][DIM];
-#pragma unroll
-  for (int i = 0; i < DIM; ++i)
-#pragma unroll
-    for (int j = 0; j < DIM; ++j) {
-      const Dual g = G[((long)i * DIM + j) * nc + c];
-      gv[i][j] = g.v;
-      gd[i][j] = g.d;
-    }
-  double ss = 0.0, off = 0.0;  // s_ij (grad u)'_ij, each off-diagonal pair once
-#pragma unroll
-  for (int i = 0; i < DIM; ++i) {
-    ss += gv[i][i] * gd[i][i];
-#pragma unroll
-    for (int j = i + 1; j < DIM; ++j) off += (gv[i][j] + gv[j][i]) * (gd[i][j] + gd[j][i]);
-  }
-  ss += 0.5 * off;
-  const double t[4] = {st.t ? st.t[(long)L::K * nc + c] : 0.0,
-                       st.t ? st.t[(long)L::W * nc + c] : 0.0, cc[c] * ss, 0.0};
-  double ddot = 0.0;
-#pragma unroll
-  for (int j = 0; j < DIM; ++j) {
-    const Dual gk = G[((long)L::K * DIM + j) * nc + c], gw = G[((long)L::W * DIM + j) * nc + c];
-    ddot += gk.d * gw.v + gk.v * gw.d;
-    Gwi[(long)j * nc + c] = gw;
-  }
-  auto form = [&](int q) {
-    const double* a = cc + (1L + 4 * q) * nc + c;
-    return a[0] * t[0] + a[nc] * t[1] + a[2 * nc] * t[2] + a[3 * nc] * ddot;
-  };
-  cl[c] = Dual{hcl[c], t[2]};
-  cl[nc + c] = Dual{hcl[nc + c], form(0)};
-  cl[2 * nc + c] = Dual{hcl[2 * nc + c], form(1)};
-  cl[3 * nc + c] = Dual{hcl[3 * nc + c], 0.0};  // the wall shear rate: 0 off the wall
-  cl[4 * nc + c] = Dual{hcl[4 * nc + c], form(2)};
-  cl[5 * nc + c] = Dual{hcl[5 * nc + c], form(3)};
-  cl[6 * nc + c] = Dual{hcl[6 * nc + c], form(4)};
-  src[c] = form(5);
-  src[nc + c] = form(6);
-}
-
-// The face sums of a Krylov product at the held linearisation: tangents only (the product's
-// output), the pin row, the k / omega source tangents of k_closure_lin off the wall and the
-// dual-number source rows on it.
-template <int DIM, bool TURB>
-__global__ void __launch_bounds__(128) k_sum_lin(MeshView m, CaseView cv, Src<Dual> st,
-                                                 Par<Dual> par, const Dual* FL, const Dual* cl,
-                                                 const Dual* G, const Dual* Gwi,
-                                                 const double* src, double* JV) {
-  stage_begin();
-  using L = Layout<DIM, TURB>;
-  constexpr int NF = L::NFLD;
-  const int c = stage_cell<Dual>(m, cv);
-  if (c >= m.nc) return;
-  const long nc = m.nc, nf = m.nf;
-  double r[NF];
-  const int b = m.cf_ptr[c], e = m.cf_ptr[c + 1];
-  for (int i = b; i < e; ++i) {
-    const unsigned ent = m.cf_face[i];
-    const int f = (int)(ent & ~FV_NB_BIT);
-    const bool isnb = (ent & FV_NB_BIT) != 0;
-#pragma unroll
-    for (int q = 0; q < NF; ++q) {
-      double x = FL[(long)q * nf + f].d;
-      if (isnb) x = -x;
-      r[q] = i == b ? x : r[q] + x;
-    }
-  }
-  if (c == cv.pin) r[L::P] = st.t ? st.t[(long)L::P * nc + c] : 0.0;
-  if constexpr (TURB) {
-    if (cv.wcell[c]) {
-      Dual rk{0.0, r[L::K]}, rw{0.0, r[L::W]};
-      sst_rows<Dual, DIM>(m, cv, st, par, cl, G, Gwi, c, rk, rw);
-      r[L::K] = rk.d;
-      r[L::W] = rw.d;
-    } else {
-      r[L::K] += src[c];
-      r[L::W] += src[nc + c];
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < NF; ++q) JV[(long)q * nc + c] = r[q];
-}
-
 // Zero the tangent of n dual values (the "frozen" JVP holds gradients, closure and a_P fixed).
 __global__ void k_freeze(long n, Dual* x) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1788,57 +1322,24 @@ void gradient_stage(FvCase* cs, Src<T> st, Par<T> par, const Work<T>& w, cudaStr
 
 template <class T, int DIM, bool TURB>
 int run(FvCase* cs, Src<T> st, Par<T> par, double* R, double* JV, cudaStream_t s,
-        bool frozen = false, bool end_profile_run = true, double* aux = nullptr) {
+        bool frozen = false, bool end_profile_run = true, double* aux = nullptr,
+        const Work<T>* into = nullptr) {  // into: where its arrays go, in place of the workspace
   const MeshView& m = cs->mesh->view;
   const CaseView& cv = cs->view;
   const long nc = m.nc, nf = m.nf;
   cs->fwd_valid = 0;  // the workspace is about to hold this pass
-  Work<T> w = work_layout<T, DIM, TURB>(cs->work, nc, nf, psi_count<DIM, TURB>(cs));
+  const Work<T> w =
+      into ? *into : work_layout<T, DIM, TURB>(cs->work, nc, nf, psi_count<DIM, TURB>(cs));
   // each stage at its own block size (the index is the stage's profiling mark)
   const int* tb = cs->tbs;
   auto bc = [&](int k) { return fv_blocks(nc, tb[k]); };
   auto bf = [&](int k) { return fv_blocks(nf, tb[k]); };
-  // a held linearisation (a state-tangent dual-number pass, first-order upwind): the linear
-  // compact gradients and the interior faces' coefficient and flux stages take their primal
-  // values from it and compute only tangents
-  bool lin = false;
-  if constexpr (std::is_same<T, Dual>::value) lin = cs->lin_use && !frozen && !psi_count<DIM, TURB>(cs);
-  // ... and the closure and face-sum stages from its tabulated closure forms (the product only:
-  // fv_jvp_linearised returns the residual the linearisation held)
-  const bool lin_sum = lin && R == nullptr && (!TURB || cs->lin_cc != nullptr);
   fv_prof_mark(cs, 0, s);
-  if constexpr (std::is_same<T, Dual>::value) {
-    if (lin && cs->desc.gradient_sweeps == 0)  // the compact scheme (no relaxation factor)
-      stage(k_grad_tangent<DIM, TURB>, bc(0), tb[0], s, m, cv, st, par, cs->lin_g, w.G);
-    else
-      gradient_stage<T, DIM, TURB>(cs, st, par, w, s);
-  } else {
-    gradient_stage<T, DIM, TURB>(cs, st, par, w, s);
-  }
+  gradient_stage<T, DIM, TURB>(cs, st, par, w, s);
   fv_prof_mark(cs, 1, s);
-  if (TURB) {
-    bool done = false;
-    if constexpr (std::is_same<T, Dual>::value) {
-      if (lin_sum) {
-        stage(k_closure_lin<DIM>, bc(1), tb[1], s, m, cv, st, par, w.G, cs->lin_cl, cs->lin_cc, w.cl, w.Gwi, cs->lin_src);
-        done = true;
-      }
-    }
-    if (!done) stage(k_closure<T, DIM>, bc(1), tb[1], s, m, cv, st, par, w.G, w.cl, w.Gwi);
-  }
+  if (TURB) stage(k_closure<T, DIM>, bc(1), tb[1], s, m, cv, st, par, w.G, w.cl, w.Gwi);
   fv_prof_mark(cs, 2, s);
-  if constexpr (std::is_same<T, Dual>::value) {
-    if (lin) {
-      if (m.nfi > 0)
-        stage(k_apcoef_tangent<DIM, TURB>, fv_blocks(m.nfi, tb[2]), tb[2], s, m, cv, st, w.G, w.cl, cs->lin_aux, cs->lin_ac, w.acown, w.acnb, w.me);
-      if (nf > m.nfi)
-        stage(k_apcoef<T, DIM, TURB>, fv_blocks(nf - m.nfi, tb[2]), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me, m.nfi);
-    } else {
-      stage(k_apcoef<T, DIM, TURB>, bf(2), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me, 0);
-    }
-  } else {
-    stage(k_apcoef<T, DIM, TURB>, bf(2), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me, 0);
-  }
+  stage(k_apcoef<T, DIM, TURB>, bf(2), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me, 0);
   fv_prof_mark(cs, 3, s);
   stage(k_dcoeff<T>, bc(3), tb[3], s, m, w.acown, w.acnb, w.dco);
   const long npsi = psi_count<DIM, TURB>(cs);
@@ -1847,35 +1348,20 @@ int run(FvCase* cs, Src<T> st, Par<T> par, double* R, double* JV, cudaStream_t s
   // G, closure, Gwi, a_P, d and the slope limiters
   if (frozen) freeze<T>(w.G, (long)(w.psi + npsi - w.G), s);
   fv_prof_mark(cs, 4, s);
-  bool flux_done = false;
-  if constexpr (std::is_same<T, Dual>::value) {
-    if (lin) {
-      // a held linearisation: the interior faces' tangent fluxes from its kept intermediates, the
-      // boundary faces by the full dual-number flux
-      if (m.nfi > 0)
-        stage(k_flux_tangent<DIM, TURB>, fv_blocks(m.nfi, tb[4]), tb[4], s, m, cv, st, w.G, w.cl, w.dco, w.me, cs->lin_aux, cs->lin_fl, w.FL);
-      if (nf > m.nfi)
-        stage(k_flux<T, DIM, TURB>, fv_blocks(nf - m.nfi, tb[4]), tb[4], s, m, cv, st, par, w.G, w.cl, w.dco, w.me, nullptr, false, w.FL, nullptr, m.nfi);
-      flux_done = true;
-    }
-  }
-  if (!flux_done)
-    stage(k_flux<T, DIM, TURB>, bf(4), tb[4], s, m, cv, st, par, w.G, w.cl, w.dco, w.me, npsi ? w.psi : nullptr, frozen, w.FL, aux, 0);
+  stage(k_flux<T, DIM, TURB>, bf(4), tb[4], s, m, cv, st, par, w.G, w.cl, w.dco, w.me,
+        npsi ? w.psi : nullptr, frozen, w.FL, aux, 0);
   fv_prof_mark(cs, 5, s);
-  bool summed = false;
-  if constexpr (std::is_same<T, Dual>::value) {
-    if (lin_sum) {
-      stage(k_sum_lin<DIM, TURB>, bc(5), tb[5], s, m, cv, st, par, w.FL, w.cl, w.G, w.Gwi, cs->lin_src, JV);
-      summed = true;
-    }
-  }
-  if (!summed)
-    stage(k_sum<T, DIM, TURB>, bc(5), tb[5], s, m, cv, st, par, w.FL, w.cl, w.G, w.Gwi, R, JV);
+  stage(k_sum<T, DIM, TURB>, bc(5), tb[5], s, m, cv, st, par, w.FL, w.cl, w.G, w.Gwi, R, JV);
   fv_prof_mark(cs, 6, s);
   if (end_profile_run) fv_prof_end_run(cs);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
 }
+
+#include "adjoint.inc.cuh"
+#include "assemble.inc.cuh"
+#include "jacobian.inc.cuh"
+#include "linearised.inc.cuh"
 
 template <int DIM, bool TURB>
 int dispatch_t(FvCase* cs, const double* state, const double* tangent, int kind, double* R,
@@ -1897,6 +1383,9 @@ int dispatch_t(FvCase* cs, const double* state, const double* tangent, int kind,
     return run<DualF, DIM, TURB>(cs, Src<DualF>{cs->f_state, tangent ? cs->f_tangent : nullptr},
                                  pf, R, JV, s, kind == FV_TAN_FROZEN32);
   }
+  if (kind == FV_TAN_STATE && cs->lin_use) {
+    return run_linearised<DIM, TURB>(cs, state, tangent, JV, s);
+  }
   const double dmu = kind == FV_TAN_MU ? 1.0 : 0.0;
   Par<Dual> par{{cs->mu, dmu}, {cs->inlet_scale, kind == FV_TAN_INLET ? 1.0 : 0.0},
                 {cs->mu * irho, dmu * irho}};
@@ -1904,9 +1393,6 @@ int dispatch_t(FvCase* cs, const double* state, const double* tangent, int kind,
   return run<Dual, DIM, TURB>(cs, st, par, R, JV, s, kind == FV_TAN_FROZEN);
 }
 
-#include "adjoint.inc.cuh"
-#include "assemble.inc.cuh"
-#include "jacobian.inc.cuh"
 
 template <int DIM, bool TURB>
 AdjWork adj_layout(FvCase* cs) {
@@ -2190,34 +1676,45 @@ int linearise(FvCase* cs, const double* state, double* R, cudaStream_t s) {
     fv_set_error("fv_case_linearise: the linearised JVP covers first-order upwind advection only");
     return FV_ERR_ARG;
   }
-  if (!cs->lin_aux) FV_CUDA_TRY(cudaMalloc(&cs->lin_aux, fv_aux_bytes(DIM, TURB, nf)));
-  if (!cs->lin_fl) FV_CUDA_TRY(cudaMalloc(&cs->lin_fl, sizeof(double) * NF * nf));
-  if (!cs->lin_ac) FV_CUDA_TRY(cudaMalloc(&cs->lin_ac, sizeof(double) * 3 * nf));
-  if (!cs->lin_g) FV_CUDA_TRY(cudaMalloc(&cs->lin_g, sizeof(double) * NF * DIM * nc));
+  auto ensure = [](double** p, long n) {
+    return *p || cudaMalloc(p, sizeof(double) * (size_t)n) == cudaSuccess;
+  };
+  if ((!cs->lin_aux && cudaMalloc(&cs->lin_aux, fv_aux_bytes(DIM, TURB, nf)) != cudaSuccess) ||
+      !ensure(&cs->lin_me, nf) || !ensure(&cs->lin_d, nc) || !ensure(&cs->lin_g, NF * DIM * nc) ||
+      !ensure(&cs->lin_r, NF * nc) || !ensure(&cs->lin_cl, 7 * nc) ||
+      (TURB && (!ensure(&cs->lin_cc, LIN_NCOEF * nc) || !ensure(&cs->lin_src, 2 * nc)))) {
+    fv_set_error("fv_case_linearise: %s", cudaGetErrorString(cudaGetLastError()));
+    return FV_ERR_CUDA;
+  }
+  if (TURB && cs->n_wall_cells < 0) {  // the wall cells, listed once a case
+    std::vector<unsigned char> wall(nc);
+    FV_CUDA_TRY(cudaMemcpyAsync(wall.data(), cs->wcell, nc, cudaMemcpyDeviceToHost, s));
+    FV_CUDA_TRY(cudaStreamSynchronize(s));
+    std::vector<int> cells;
+    for (long c = 0; c < nc; ++c)
+      if (wall[c]) cells.push_back((int)c);
+    FV_CUDA_TRY(cudaMalloc(&cs->wall_cells, sizeof(int) * (cells.size() + 1)));
+    FV_CUDA_TRY(cudaMemcpyAsync(cs->wall_cells, cells.data(), sizeof(int) * cells.size(),
+                                cudaMemcpyHostToDevice, s));
+    FV_CUDA_TRY(cudaStreamSynchronize(s));
+    cs->n_wall_cells = (int)cells.size();
+  }
   cs->lin_valid = 0;
   const double irho = 1.0 / cs->desc.rho;
+  // the pass writes what is held where it stays
+  Work<double> w = work_layout<double, DIM, TURB>(cs->work, nc, nf, psi_count<DIM, TURB>(cs));
+  w.G = cs->lin_g;
+  w.cl = cs->lin_cl;
+  w.me = cs->lin_me;
+  w.dco = cs->lin_d;
   int rc = run<double, DIM, TURB>(cs, Src<double>{state},
                                   Par<double>{cs->mu, cs->inlet_scale, cs->mu * irho}, R, nullptr,
-                                  s, false, true, cs->lin_aux);
+                                  s, false, true, cs->lin_aux, &w);
   if (rc != FV_OK) return rc;
-  Work<double> w = work_layout<double, DIM, TURB>(cs->work, nc, nf, psi_count<DIM, TURB>(cs));
-  FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_fl, w.FL, sizeof(double) * NF * nf,
-                              cudaMemcpyDeviceToDevice, s));
-  FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_ac, w.acown, sizeof(double) * nf, cudaMemcpyDeviceToDevice, s));
-  FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_ac + nf, w.acnb, sizeof(double) * nf,
-                              cudaMemcpyDeviceToDevice, s));
-  FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_ac + 2 * nf, w.me, sizeof(double) * nf,
-                              cudaMemcpyDeviceToDevice, s));
-  FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_g, w.G, sizeof(double) * NF * DIM * nc,
-                              cudaMemcpyDeviceToDevice, s));
-  if (!cs->lin_r) FV_CUDA_TRY(cudaMalloc(&cs->lin_r, sizeof(double) * NF * nc));
   FV_CUDA_TRY(cudaMemcpyAsync(cs->lin_r, R, sizeof(double) * NF * nc, cudaMemcpyDeviceToDevice, s));
   if constexpr (TURB) {
-    if (!cs->lin_cl) FV_CUDA_TRY(cudaMalloc(&cs->lin_cl, sizeof(double) * 7 * nc));
-    if (!cs->lin_cc) FV_CUDA_TRY(cudaMalloc(&cs->lin_cc, sizeof(double) * LIN_NCOEF * nc));
-    if (!cs->lin_src) FV_CUDA_TRY(cudaMalloc(&cs->lin_src, sizeof(double) * 2 * nc));
     k_lin_closure_coef<DIM><<<fv_blocks(nc, 128), 128, 0, s>>>(
-        cs->mesh->view, cs->view, state, w.G, w.cl, cs->mu * irho, cs->lin_cl, cs->lin_cc);
+        cs->mesh->view, cs->view, state, w.G, w.cl, cs->mu * irho, cs->lin_cc);
     FV_CUDA_TRY(cudaGetLastError());
   }
   cs->lin_valid = 1;
