@@ -30,11 +30,16 @@
 namespace {
 
 // The stages of a pass are launched with programmatic dependent launch: a stage's blocks may be
-// placed while the stage before drains, and wait for it before their first read.  On small meshes a
-// pass is a dozen kernels of 2-6 us with 1-3 us between them (64 x 64 cavity, residual + VJP: 79 ->
-// 61 us).
+// placed before the stage before has ended, and wait for it before their first read.  On small
+// meshes a pass is a dozen kernels of 2-6 us with 1-3 us between them (64 x 64 cavity, residual +
+// VJP: 79 -> 61 us).  The next stage is let in at once where its blocks find SMs of their own
+// beside this one's, or where there are many waves of them; between, blocks placed around a stage
+// that still runs would crowd the SMs it left free (10,000-cell JVP: 41 -> 43 us), so the next
+// stage comes as this one's blocks end.
 __device__ __forceinline__ void stage_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const unsigned threads = gridDim.x * blockDim.x;
+  if (threads <= 8192u || threads >= 262144u)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class K, class... Args>
