@@ -256,7 +256,7 @@ __device__ __forceinline__ void a_flux_at(const int c, MeshView m, CaseView cv, 
   constexpr int NF = L::NFLD;
   if (c >= m.nc) return;
   const int nc = m.nc, nf = m.nf;
-  const double rho = cv.rho, irho = 1.0 / cv.rho;
+  const double rho = cv.rho, irho = cv.irho;
   const double nu = par.nu;
   double sb[NF], Gb[NF][DIM];
 #pragma unroll

@@ -323,6 +323,7 @@ extern "C" int fv_case_create(const FvMesh* mesh, const FvCaseDesc* desc,
   v.lim_ks = (desc->turbulent && sadv == 2) ? sK : 0.0;
   v.turb = desc->turbulent;
   v.rho = desc->rho;
+  v.irho = 1.0 / desc->rho;
   v.pin = desc->pressure_pin;
   v.pin_value = desc->pressure_pin_value;
   v.fkind = c->fkind;

@@ -76,7 +76,7 @@ int fv_mesh_compute_geometry(FvMesh* m, cudaStream_t s);
 // Device case tables (internal face order) and the residual workspace (residual.cu).
 struct CaseView {
   int turb;
-  double rho;
+  double rho, irho;           // density and its reciprocal
   int pin;
   double pin_value;
   const signed char* fkind;   // (nf) flow boundary kind

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
                                                   const double* cl, const double* psi,
                                                   const double* co, const double* src,
                                                   const int* indptr, const int* indices,
-                                                  double* values, double irho, bool vec) {
+                                                  double* values, bool vec) {
   using L = Layout<DIM, TURB>;
   constexpr int NF = L::NFLD;
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
   // rows without the face sum: the pinned pressure row, the omega wall-cell row
   bool skip = cont && c == cv.pin;
   if constexpr (TURB) skip = skip || (q == L::W && cv.wcell[c] != 0);
-  const double rho = cv.rho;
+  const double rho = cv.rho, irho = cv.irho;
   const double* rec = mom ? (cv.rec_mom ? psi : nullptr) : (cv.rec_sca ? psi : nullptr);
   const int adv = mom ? q : q - 1;  // index among the advected fields
   // the diagonal block's row; its own field's column (one fp64 addition a face, not one for every
@@ -419,7 +419,7 @@ int assemble_frozen64(FvCase* cs, const double* state, const int* indptr, const 
     k_jac_src<DIM><<<bc, TB, 0, s>>>(m, cv, state, par, w.G, w.cl, w.Gwi, src);
   k_jac_rows<DIM, TURB><<<fv_blocks(nc * NF, TB), TB, 0, s>>>(
       m, cv, state, par, w.G, w.cl, npsi ? w.psi : nullptr, w.FL, src, indptr, indices, values,
-      1.0 / cs->desc.rho, (uintptr_t)values % 16 == 0);
+      (uintptr_t)values % 16 == 0);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
 }

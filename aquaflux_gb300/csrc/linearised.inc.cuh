@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(128) k_flux_tangent(MeshView m, CaseView cv, S
   const long nc = m.nc, nf = m.nf;
   const int o = m.owner[f], n = m.nb[f];
   const double A = m.area[f], g = m.g[f];
-  const double rho = cv.rho, irho = 1.0 / cv.rho;
+  const double rho = cv.rho, irho = cv.irho;
   const double mdot = aux[0L * nf + f], damping = aux[1L * nf + f], dhat = aux[2L * nf + f];
   const double cmo = aux[3L * nf + f];
   double gd = 0.0, gs = 0.0;

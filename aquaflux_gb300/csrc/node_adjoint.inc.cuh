@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(128) k_nadj_face(MeshView m, CaseView cv, cons
   const int o = m.owner[f];
   const bool interior = f < m.nfi;
   const int n = interior ? m.nb[f] : o;
-  const double A = m.area[f], rho = cv.rho, irho = 1.0 / cv.rho, nu = par.nu;
+  const double A = m.area[f], rho = cv.rho, irho = cv.irho, nu = par.nu;
   auto st = [&](int q, int c) { return state[(long)q * nc + c]; };
   auto gr = [&](int q, int j, int c) { return G[((long)q * DIM + j) * nc + c]; };
   double nrm[DIM], dp[DIM], FLb[NF];

@@ -1022,7 +1022,10 @@ __device__ __forceinline__ void flux_face(const MeshView& m, const CaseView& cv,
   const int nc = m.nc, nf = m.nf;
   const int o = m.owner[f];
   const GT A = gv.area(m, f);
-  const GS<T> rho = rho_of<T>(cv), irho = GS<T>(1) / rho;
+  const GS<T> rho = rho_of<T>(cv);
+  GS<T> irho;
+  if constexpr (IsF32<T>::value) irho = 1.0f / rho;
+  else irho = cv.irho;
   GT nrm[DIM], tP[DIM];
 #pragma unroll
   for (int j = 0; j < DIM; ++j) {
