@@ -80,7 +80,8 @@ void with_block_size(int b, Fn&& fn) {
 // ------------------------------------------------------------------------------ BSR SpMV
 template <class V>
 __global__ void k_bsr_spmv(int nbr, int b, const int* __restrict__ ptr, const int* __restrict__ idx,
-                           const V* __restrict__ val, const V* __restrict__ x, V* __restrict__ y) {
+                           const V* __restrict__ val, const V* __restrict__ x,
+                           const V* __restrict__ rhs, V* __restrict__ y) {
   // one thread per scalar row: row r = (block row i, component a)
   long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= (long)nbr * b) return;
@@ -92,15 +93,16 @@ __global__ void k_bsr_spmv(int nbr, int b, const int* __restrict__ ptr, const in
     const V* xs = x + (long)idx[q] * b;
     for (int c = 0; c < b; ++c) acc += blk[c] * xs[c];
   }
-  y[r] = acc;
+  y[r] = rhs ? rhs[r] - acc : acc;
 }
 
 // The same product with a compile-time block size and vector loads of each row segment (every
 // block row segment and x segment starts at a multiple of B values from 16-byte aligned bases).
-template <class V, int B>
+// RES: y = rhs - A x, the product rounded before the difference, as two passes give it.
+template <class V, int B, bool RES>
 __global__ void k_bsr_spmv_b(int nbr, const int* __restrict__ ptr, const int* __restrict__ idx,
                              const V* __restrict__ val, const V* __restrict__ x,
-                             V* __restrict__ y) {
+                             const V* __restrict__ rhs, V* __restrict__ y) {
   const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= (long)nbr * B) return;
   const int i = (int)(r / B), a = (int)(r % B);
@@ -113,7 +115,7 @@ __global__ void k_bsr_spmv_b(int nbr, const int* __restrict__ ptr, const int* __
 #pragma unroll
     for (int c = 0; c < B; ++c) acc += m[c] * xs[c];
   }
-  y[r] = acc;
+  y[r] = RES ? rhs[r] - acc : acc;
 }
 
 // Transposed product through the precomputed transpose map: for block row j of A^T, gather
@@ -523,8 +525,9 @@ __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
 // whatever its width; fp64 cavity: 11.9 us a level set of 64 rows).  Here a row's blocks and columns
 // are copied in once and back once; the lower blocks' rows j are looked up by 32 lanes at once; the
 // columns of row j come in one load, each lane counting row i's columns below its own to find its
-// place; the next row j is fetched and the matching blocks' columns are read before the chain of
-// quotients, which hides them; and the matching blocks are updated side by side.  Pivots of finished rows come with their reciprocals
+// place; what the pattern alone gives is found before the level before is waited for; the next row
+// j is fetched and the matching blocks' columns are read before the chain of quotients, which hides
+// them; and the matching blocks are updated side by side.  Pivots of finished rows come with their reciprocals
 // (`rp`): a quotient is a product and a correction, not a division on the chain (fp64: 192 cycles
 // for 321).
 // Lanes: for b <= 4 one per block entry (16 to a block, two blocks at a time), which keeps the
@@ -592,8 +595,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
   constexpr int PU = (BB + B + 31) / 32;
   int j = 0, dj = 0, ej = 0, kcol = -1;
   V pu[PU];
-  auto fetch = [&](int q) {
-    if (q >= nl) return;
+  auto place = [&](int q) {  // (the pattern only)
     if ((q & 31) == 0 && q + lane < nl) {
       jl = cols[q + lane];
       dl = F.diag[jl];
@@ -603,6 +605,8 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
     dj = __shfl_sync(0xffffffffu, dl, q & 31);
     ej = __shfl_sync(0xffffffffu, rl, q & 31);
     kcol = dj + 1 + lane < ej ? F.idx[dj + 1 + lane] : -1;
+  };
+  auto fetch = [&] {
 #pragma unroll
     for (int u = 0; u < PU; ++u) {
       const int k = u * 32 + lane;
@@ -661,17 +665,26 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
       }
     }
   };
-  wait_level_before();  // (only the row itself, which no earlier level writes, was read so far)
-  fetch(0);
+  int m = 0;
+  if (nl > 0) {
+    place(0);
+    m = find(0, kcol, dj + 1 + lane);
+  }
+  // only the pattern and the row itself, which no earlier level writes, were read so far
+  wait_level_before();
+  if (nl > 0) fetch();
   for (int q = 0; q < nl; ++q) {
     const int jq = j, s0 = dj + 1, eq = ej;
+    V M0[B];
+    column(sg, m, M0);
 #pragma unroll
     for (int u = 0; u < PU; ++u)
       if (u * 32 + lane < BB + B) Us[u * 32 + lane] = pu[u];
-    const int m = find(q, kcol, s0 + lane);  // (its barrier also makes Us visible)
-    V M0[B];
-    column(sg, m, M0);
-    fetch(q + 1);
+    __syncwarp();
+    if (q + 1 < nl) {
+      place(q + 1);
+      fetch();
+    }
     // L_ij = A_ij U_jj^-1, scalar columns ascending
     V* Lq = blk + q * BB;
     if constexpr (EM) {
@@ -721,6 +734,7 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
       }
       __syncwarp();
     }
+    if (q + 1 < nl) m = find(q + 1, kcol, dj + 1 + lane);
   }
   // the diagonal block: in-place LU (unit lower)
   V* D = blk + nl * BB;
@@ -1882,12 +1896,12 @@ int spmv(int nbr, int b, const int* indptr, const int* indices, const V* values,
     const bool aligned = ((uintptr_t)values % 16 == 0) && ((uintptr_t)x % 16 == 0);
     if (aligned && b >= 2 && b <= 8)
       with_block_size(b, [&](auto B) {
-        k_bsr_spmv_b<V, B()><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(nbr, indptr, indices,
-                                                                           values, x, y);
+        k_bsr_spmv_b<V, B(), false><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(
+            nbr, indptr, indices, values, x, nullptr, y);
       });
     else
       k_bsr_spmv<V><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
-                                                                   values, x, y);
+                                                                   values, x, nullptr, y);
     FV_CUDA_TRY(cudaGetLastError());
     return FV_OK;
   }
@@ -1994,6 +2008,38 @@ extern "C" int fv_bsr_spmv_f32(int nbr, int b, const int* indptr, const int* ind
                                const float* values, const float* x, float* y, int transpose,
                                void* stream) {
   return spmv<float>(nbr, b, indptr, indices, values, x, y, transpose, (cudaStream_t)stream);
+}
+
+namespace {
+template <class V>
+int bsr_residual(int nbr, int b, const int* indptr, const int* indices, const V* values, const V* x,
+                 const V* rhs, V* r, cudaStream_t s) {
+  if (nbr <= 0 || b <= 0 || !indptr || !indices || !values || !x || !rhs || !r) {
+    fv_set_error("fv_bsr_residual: bad arguments");
+    return FV_ERR_ARG;
+  }
+  const long rows = (long)nbr * b;
+  const int grid = fv_blocks(rows, kThreads);
+  if (((uintptr_t)values | (uintptr_t)x) % 16 == 0 && b >= 2 && b <= 8)
+    with_block_size(b, [&](auto B) {
+      k_bsr_spmv_b<V, B(), true><<<grid, kThreads, 0, s>>>(nbr, indptr, indices, values, x, rhs, r);
+    });
+  else
+    k_bsr_spmv<V><<<grid, kThreads, 0, s>>>(nbr, b, indptr, indices, values, x, rhs, r);
+  FV_CUDA_TRY(cudaGetLastError());
+  return FV_OK;
+}
+}  // namespace
+
+extern "C" int fv_bsr_residual_f64(int nbr, int b, const int* indptr, const int* indices,
+                                   const double* values, const double* x, const double* rhs,
+                                   double* r, void* stream) {
+  return bsr_residual<double>(nbr, b, indptr, indices, values, x, rhs, r, (cudaStream_t)stream);
+}
+extern "C" int fv_bsr_residual_f32(int nbr, int b, const int* indptr, const int* indices,
+                                   const float* values, const float* x, const float* rhs, float* r,
+                                   void* stream) {
+  return bsr_residual<float>(nbr, b, indptr, indices, values, x, rhs, r, (cudaStream_t)stream);
 }
 
 // out[i] = sum over fields q and cells c in [seg[i], seg[i + 1]) of a[q nc + c] b[q nc + c]: one
