@@ -70,12 +70,11 @@ class _Level:
                                                 ptr(self.values), ptr(self._tvals),
                                                 int(self.sfx == "f64"), _stream()))
 
-    def spmv(self, x, y, transpose: bool = False):
+    def _operator(self, transpose: bool):
+        """Pattern and blocks of ``A``, or of ``A^T``: its blocks transposed, so that the transposed
+        product is the forward kernel's (the mapped transposed products in the same order)."""
         if not transpose:
-            check(getattr(lib(), "fv_bsr_spmv_" + self.sfx)(
-                self.n, self.b, ptr(self.d_indptr), ptr(self.d_indices), ptr(self.values), ptr(x),
-                ptr(y), 0, _stream()))
-            return
+            return self.d_indptr, self.d_indices, self.values
         if self._tmap is None:
             tp = np.empty(self.n + 1, dtype=np.int32)
             ti = np.empty(self.nnzb, dtype=np.int32)
@@ -85,11 +84,18 @@ class _Level:
             self._tmap = [torch.tensor(a, device="cuda") for a in (tp, ti, tb)]
             self._tvals = torch.empty_like(self.values)
             self.transpose_values()
-        # A^T x as the forward product on A^T's pattern and transposed blocks: the products of
-        # the mapped transposed kernel in the same order, read row-wise
-        tp, ti, _ = self._tmap
+        return self._tmap[0], self._tmap[1], self._tvals
+
+    def spmv(self, x, y, transpose: bool = False):
+        ip, ix, values = self._operator(transpose)
         check(getattr(lib(), "fv_bsr_spmv_" + self.sfx)(
-            self.n, self.b, ptr(tp), ptr(ti), ptr(self._tvals), ptr(x), ptr(y), 0, _stream()))
+            self.n, self.b, ptr(ip), ptr(ix), ptr(values), ptr(x), ptr(y), 0, _stream()))
+
+    def residual(self, rhs, x, r, transpose: bool = False):
+        """``r = rhs - A x`` (``A^T x``)."""
+        ip, ix, values = self._operator(transpose)
+        check(getattr(lib(), "fv_bsr_residual_" + self.sfx)(
+            self.n, self.b, ptr(ip), ptr(ix), ptr(values), ptr(x), ptr(rhs), ptr(r), _stream()))
 
 
 def plan_hierarchy(n, indptr, indices, *, min_cells: int = 4000, max_levels: int = 10,
@@ -266,8 +272,7 @@ class AmgHierarchy:
             lv.ilu.solve(b_vec, transpose=transpose, out=x)
             sweeps -= 1
         for _ in range(sweeps):
-            lv.spmv(x, lv.t, transpose)
-            torch.sub(b_vec, lv.t, out=lv.r)
+            lv.residual(b_vec, x, lv.r, transpose)
             lv.ilu.solve(lv.r, transpose=transpose, out=lv.t)
             x.add_(lv.t)
 
@@ -285,8 +290,7 @@ class AmgHierarchy:
                 self._smooth(lv, b_vec, x, self.coarse_sweeps, True, transpose)
             return x
         self._smooth(lv, b_vec, x, self.sweeps, True, transpose)
-        lv.spmv(x, lv.t, transpose)
-        torch.sub(b_vec, lv.t, out=lv.r)
+        lv.residual(b_vec, x, lv.r, transpose)
         coarse = self.levels[level + 1]
         t = lv.coarse
         bc = coarse.rhs

@@ -314,6 +314,14 @@ int fv_bsr_spmv_t_f64_noalloc(int n_block_rows, long nnzb, int b, const int* ind
 /* fp32 values and vectors. */
 int fv_bsr_spmv_f32(int n_block_rows, int b, const int* indptr, const int* indices,
                     const float* values, const float* x, float* y, int transpose, void* stream);
+/* r = rhs - A x in one pass (device; r overlaps no input): bitwise the difference of rhs and the product of
+ * fv_bsr_spmv (the defect of a V-cycle's smoother, aquaflux/solve/multigrid.py:1510-1864). */
+int fv_bsr_residual_f64(int n_block_rows, int b, const int* indptr, const int* indices,
+                        const double* values, const double* x, const double* rhs, double* r,
+                        void* stream);
+int fv_bsr_residual_f32(int n_block_rows, int b, const int* indptr, const int* indices,
+                        const float* values, const float* x, const float* rhs, float* r,
+                        void* stream);
 /* Transpose map of a square BSR pattern (host): tptr (n + 1) / tidx (nnzb) list, for block row j
  * of A^T, the rows i of A holding a block (i, j); tblk (nnzb) that block's index in A. */
 int fv_bsr_transpose_map(int n, const int* indptr, const int* indices, int* tptr, int* tidx,
