@@ -208,6 +208,7 @@ class AmgHierarchy:
             self.levels.append(_Level(step["n_coarse"], b, step["indptr"], step["indices"],
                                       precision, kl(i + 1)))
         last = self.levels[-1]
+        self._sides = [torch.cuda.Stream() for _ in self.levels]  # where each level is factored
         nd = last.n * b
         self.dense = None
         if len(self.levels) > 1 and (coarse_solve == "dense"
@@ -253,17 +254,32 @@ class AmgHierarchy:
             lv0.values = fine_values  # the fine operator itself (no copy)
         else:
             lv0.values.copy_(fine_values)
-        lv0.ilu.refactor(lv0.values)
+        # The levels' factors hang on the values only, and the coarse ones are chains of a few rows
+        # a level set that leave most SMs idle: each is factored on a stream of its own, the next
+        # level's Galerkin sums queued before it, and the zero pivots are read at the end.  64^3 SST
+        # channel: 3044 us a refresh and cycle, one after the other with a host round trip each 3334.
         galerkin = getattr(lib(), "fv_galerkin_" + self.sfx)
-        for fine, coarse in zip(self.levels[:-1], self.levels[1:]):
-            t = fine.coarse
-            check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
-                           ptr(fine.values), int(fine.values.dtype == torch.float64),
-                           ptr(coarse.values), _stream()))
-            if coarse is self.levels[-1] and self.dense is not None:
-                self._invert_coarsest()
-            else:
-                coarse.ilu.refactor(coarse.values)
+        main = torch.cuda.current_stream()
+        started = []
+        try:
+            for fine, coarse, side in zip(self.levels, self.levels[1:] + [None], self._sides):
+                if coarse is not None:
+                    values_ready = main.record_event()
+                    t = fine.coarse
+                    check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
+                                   ptr(fine.values), int(fine.values.dtype == torch.float64),
+                                   ptr(coarse.values), _stream()))
+                    started.append((fine, side, fine.ilu.start_factor(fine.values, side, values_ready)))
+                elif self.dense is None:
+                    started.append((fine, None, fine.ilu.start_factor(fine.values)))
+                else:
+                    self._invert_coarsest()
+        finally:
+            for _, side, _ in started:
+                if side is not None:
+                    main.wait_stream(side)
+            for lv, _, factor in started:  # (an error is the finest level's)
+                lv.ilu.finish_factor(*factor)
         for lv in self.levels:
             lv.transpose_values()
 

@@ -1427,9 +1427,8 @@ int capture(Body body, cudaGraphExec_t* out) {
 }
 
 template <class V>
-int ilu_factor(FvIlu0* f, cudaStream_t s) {
-  unsigned long long init = ~0ull;
-  FV_CUDA_TRY(cudaMemcpyAsync(f->zero_flag, &init, sizeof(init), cudaMemcpyHostToDevice, s));
+int ilu_factor_start(FvIlu0* f, cudaStream_t s) {
+  FV_CUDA_TRY(cudaMemsetAsync(f->zero_flag, 0xff, sizeof(unsigned long long), s));
   if (!f->factor_exec) {
     int rc = capture([&](cudaStream_t cs) { launch_factor_levels<V>(f, cs); }, &f->factor_exec);
     if (rc != FV_OK) return rc;
@@ -1447,6 +1446,10 @@ int ilu_factor(FvIlu0* f, cudaStream_t s) {
       if (rc != FV_OK) return rc;
     }
   FV_CUDA_TRY(cudaGetLastError());
+  return FV_OK;
+}
+
+int ilu_factor_finish(FvIlu0* f, cudaStream_t s) {
   unsigned long long flag;
   FV_CUDA_TRY(cudaMemcpyAsync(&flag, f->zero_flag, sizeof(flag), cudaMemcpyDeviceToHost, s));
   FV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1752,7 +1755,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   return FV_OK;
 }
 
-extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream) {
+extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, void* stream) {
   if (!f || !values || !f->val) {
     fv_set_error("fv_ilu0_factor: bad arguments");
     return FV_ERR_ARG;
@@ -1761,13 +1764,26 @@ extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, voi
   const long n = (long)f->nnzb * f->b * f->b;
   if (f->precision == 64) {
     FV_CUDA_TRY(cudaMemcpyAsync(f->val, values, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    return ilu_factor<double>(f, s);
+    return ilu_factor_start<double>(f, s);
   }
   if (values_f64)
     k_to_f32<<<fv_blocks(n, kThreads), kThreads, 0, s>>>(n, (const double*)values, (float*)f->val);
   else
     FV_CUDA_TRY(cudaMemcpyAsync(f->val, values, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-  return ilu_factor<float>(f, s);
+  return ilu_factor_start<float>(f, s);
+}
+
+extern "C" int fv_ilu0_factor_finish(FvIlu0* f, void* stream) {
+  if (!f || !f->val) {
+    fv_set_error("fv_ilu0_factor: bad arguments");
+    return FV_ERR_ARG;
+  }
+  return ilu_factor_finish(f, (cudaStream_t)stream);
+}
+
+extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream) {
+  const int rc = fv_ilu0_factor_start(f, values, values_f64, stream);
+  return rc == FV_OK ? fv_ilu0_factor_finish(f, stream) : rc;
 }
 
 extern "C" int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, void* stream) {

@@ -103,6 +103,11 @@ class Ilu0:
         return self._n * self._b
 
     def refactor(self, values) -> None:
+        self.finish_factor(*self.start_factor(values))
+
+    def start_factor(self, values, stream: torch.cuda.Stream | None = None, after=None):
+        """Enqueue the factorization of new values on the current stream, or on ``stream`` behind
+        the event ``after`` (when the values are there and earlier solves with this factor done).  Gives what :meth:`finish_factor`, which has to follow, takes."""
         v = torch.as_tensor(values)
         if v.numel() != self._nvals:
             raise ValueError(f"expected {self._nvals} values for this pattern, got {v.numel()}.")
@@ -113,7 +118,22 @@ class Ilu0:
         if self._precision == 32 and v.dtype not in (torch.float32, torch.float64):
             v = v.to(torch.float64)
         try:
-            check(lib().fv_ilu0_factor(self._h, ptr(v), int(v.dtype == torch.float64), _stream()))
+            if stream is not None:
+                if v is values:
+                    stream.wait_event(after)
+                else:  # converted on the current stream
+                    stream.wait_stream(torch.cuda.current_stream())
+            s = _stream() if stream is None else int(stream.cuda_stream)
+            check(lib().fv_ilu0_factor_start(self._h, ptr(v), int(v.dtype == torch.float64), s))
+        except FvError as e:
+            _raise(e)
+        return v, s
+
+    def finish_factor(self, values, stream: int) -> None:
+        """Wait for a started factorization (``values``: held until then) and report its zero
+        pivot."""
+        try:
+            check(lib().fv_ilu0_factor_finish(self._h, stream))
         except FvError as e:
             _raise(e)
 

@@ -361,6 +361,10 @@ int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvIlu0** out);
 /* Numeric factorization of new values (device, nnzb * b * b, same dtype as `precision`, or
  * float64 when values_f64 != 0 and precision == 32: converted on the fly). */
 int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream);
+/* Its two halves, to factor several matrices side by side on streams of their own: start enqueues
+ * the factorization, finish (same stream) waits for it and reports a zero pivot. */
+int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, void* stream);
+int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
 /* x = (LU)^-1 r, or (LU)^-T r when transpose != 0.  Device vectors of `precision`.  On a stream
  * under capture the level kernels are recorded into the caller's graph (x may alias r, and must be
  * 16-byte aligned: FV_ERR_ARG otherwise); a transposed solve needs one uncaptured transposed solve
