@@ -71,7 +71,9 @@ __global__ void __launch_bounds__(128) k_grad_tangent(MeshView m, CaseView cv, S
   if (c >= m.nc) return;
   const int nc = m.nc, nf = m.nf;
   const double* t = st.t;
-  double phic[NF], acc[NF][DIM];
+  double phic[NF], acc[NF][DIM], own[DIM];  // own (SST): as in k_grad
+#pragma unroll
+  for (int j = 0; j < DIM; ++j) own[j] = 0.0;
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     phic[q] = t[(long)q * nc + c];
@@ -94,7 +96,16 @@ __global__ void __launch_bounds__(128) k_grad_tangent(MeshView m, CaseView cv, S
 #pragma unroll
       for (int q = 0; q < NF; ++q) {
         const double po = t[(long)q * nc + other];
-        phif[q] = lerp(isnb ? po : phic[q], isnb ? phic[q] : po, g);
+        if constexpr (TURB) phif[q] = po;
+        else phif[q] = lerp(isnb ? po : phic[q], isnb ? phic[q] : po, g);
+      }
+      if constexpr (TURB) {
+        const double h = 1.0 - g, wo = isnb ? h : g, wc = isnb ? g : h;
+#pragma unroll
+        for (int j = 0; j < DIM; ++j) {
+          own[j] += S[j] * wc;
+          S[j] *= wo;
+        }
       }
     } else {
       const signed char kind = cv.fkind[f];
@@ -119,8 +130,9 @@ __global__ void __launch_bounds__(128) k_grad_tangent(MeshView m, CaseView cv, S
 #pragma unroll
     for (int j = 0; j < DIM; ++j) {
       const long k = ((long)q * DIM + j) * nc + c;
-      G[k] = acc[q][j] * inv;
-      if (Bg) Bg[k] = acc[q][j];
+      const double x = TURB ? acc[q][j] + own[j] * phic[q] : acc[q][j];
+      G[k] = x * inv;
+      if (Bg) Bg[k] = x;
     }
 }
 
