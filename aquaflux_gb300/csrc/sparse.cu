@@ -281,15 +281,15 @@ __global__ void k_ilu_factor_level(IluView<V> F, const int* rows, int count,
   }
 }
 
-// Forward sweep (L y = r, unit lower) for one level; y holds r on entry.
+// Forward sweep (L y = r, unit lower) for one level; y may be r.
 template <class V>
-__global__ void k_ilu_lower(IluView<V> F, const int* rows, int count, V* y) {
+__global__ void k_ilu_lower(IluView<V> F, const int* rows, int count, const V* r, V* y) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const int i = rows[t], b = F.b;
   const long bb = (long)b * b;
   V acc[8];
-  for (int a = 0; a < b; ++a) acc[a] = y[(long)i * b + a];
+  for (int a = 0; a < b; ++a) acc[a] = r[(long)i * b + a];
   for (int q = F.ptr[i]; q < F.diag[i]; ++q) {
     const V* L = F.val + (long)q * bb;
     const V* yj = y + (long)F.idx[q] * b;
@@ -333,13 +333,13 @@ __global__ void k_ilu_upper(IluView<V> F, const int* rows, int count, V* x) {
 // U^T z = r: forward over block columns; z_i = U_ii^-T (r_i - sum_{j<i} U_ji^T z_j).
 template <class V>
 __global__ void k_ilu_upper_t(IluView<V> F, const int* tptr, const int* tidx, const int* tblk,
-                              const int* rows, int count, V* z) {
+                              const int* rows, int count, const V* r, V* z) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const int i = rows[t], b = F.b;
   const long bb = (long)b * b;
   V acc[8];
-  for (int a = 0; a < b; ++a) acc[a] = z[(long)i * b + a];
+  for (int a = 0; a < b; ++a) acc[a] = r[(long)i * b + a];
   for (int q = tptr[i]; q < tptr[i + 1]; ++q) {
     const int j = tidx[q];
     if (j >= i) continue;
@@ -866,7 +866,7 @@ __device__ __forceinline__ void ask_blocks(const V* val, int q0, int count, int 
 
 // Forward sweep of one level, a group of FV_LG lanes per block row (lane a = row a of the block).
 template <class V, int B, int U>
-__global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, V* y) {
+__global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, const V* r, V* y) {
   if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
@@ -880,7 +880,7 @@ __global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, V* y) {
     ask_blocks<V, B>(F.val, q0, di - q0, a);
     wait_level_before();
   }
-  V acc = live ? y[(long)i * B + a] : V(0);
+  V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
   if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
@@ -956,7 +956,7 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
 // is the in-block upper solve of its own forward result, with the diagonal block already in
 // registers.  The same operations in the same order as the two separate sweeps.
 template <class V, int B, int U>
-__global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, V* y) {
+__global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, const V* r, V* y) {
   if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
@@ -970,7 +970,7 @@ __global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, V
     ask_blocks<V, B>(F.val, q0, di - q0, a);
     wait_level_before();
   }
-  V acc = live ? y[(long)i * B + a] : V(0);
+  V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
   if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
@@ -1019,7 +1019,7 @@ __device__ __forceinline__ V lower_t_block_solve(V acc, const V (&Dc)[B], int a,
 // with D^T -- the operations and their order of the reference's transposed solve.
 template <class V, int B, int U>
 __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx, const int* tdiag,
-                                 const V* tval, const int* rows, int count, V* z) {
+                                 const V* tval, const int* rows, int count, const V* r, V* z) {
   if (U > 1) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
@@ -1033,7 +1033,7 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
     ask_blocks<V, B>(tval, q0, di - q0, a);
     wait_level_before();
   }
-  V acc = live ? z[(long)i * B + a] : V(0);
+  V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, tval, tidx, z, q0, di - q0, a, live, mask);
   V Dc[B];  // Dc[c] = D(c, a): row a of D^T
   if (live) load_seg<B>(tval + (long)di * BB + (long)a * B, Dc);
@@ -1076,6 +1076,137 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
     if (live && a < c) acc -= Dc[c] * vc;
   }
   if (live) x[(long)i * B + a] = acc;
+}
+
+// ---- fp32 levels of fewer than kDeepRows rows: a warp per block row, its blocks in shared memory.
+// Such a level's time is its longest row's chain, and a coarse Galerkin row holds 20 to 40 blocks:
+// with 8 lanes reading four blocks at a time from L2 the chain paid a memory latency or two every
+// four blocks (10 level sets of 720 rows: 6 us each).  Here a row's columns, blocks, diagonal block
+// and, going forward, right-hand side are in place before the level before is waited for; all its x
+// entries then come in one round of loads, a block's by a lane, and what is left is the subtractions
+// one after the other: 2 us a level set.  fp32 V-cycle of the 128 x 96 x 96 channel 2083 -> 1868 us,
+// of 40^3 cells 607 -> 345; from kDeepRows on, where the lanes and not a row's chain run out, the
+// lane groups are faster (levels of 26,000 rows: 1943 us with a warp a row).
+// The operations and their order are the lane-group kernels'.
+enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
+
+constexpr int kSweepBlocks = 32;  // blocks in shared memory at a time: a column a lane
+template <int B>
+__host__ __device__ constexpr int sweep_warp_entries(int cap) {
+  return (cap * B * (B + 1) + 3) / 4 * 4;
+}
+
+// x is written by other blocks while this one runs: read past the L1 cache
+template <int B>
+__device__ __forceinline__ void load_x(const float* p, float (&o)[B]) {
+  if constexpr (B % 4 == 0) {
+#pragma unroll
+    for (int k = 0; k < B / 4; ++k) {
+      const float4 t = __ldcg(reinterpret_cast<const float4*>(p) + k);
+      o[4 * k] = t.x;
+      o[4 * k + 1] = t.y;
+      o[4 * k + 2] = t.z;
+      o[4 * k + 3] = t.w;
+    }
+  } else if constexpr (B % 2 == 0) {
+#pragma unroll
+    for (int k = 0; k < B / 2; ++k) {
+      const float2 t = __ldcg(reinterpret_cast<const float2*>(p) + k);
+      o[2 * k] = t.x;
+      o[2 * k + 1] = t.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < B; ++k) o[k] = __ldcg(p + k);
+  }
+}
+
+// ptr / idx / diag / val: the factor's, or the transpose map's and its transposed blocks; cap: the
+// most blocks of a row beside its diagonal, at most kSweepBlocks.
+template <int B, int MODE>
+__global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* idx,
+                                                     const int* diag, const float* val,
+                                                     const int* rows, int count, int cap,
+                                                     const float* r, float* x) {
+  constexpr int BB = B * B;
+  constexpr bool kAfter = MODE == kUpper || MODE == kLowerT;  // the blocks after the diagonal one
+  constexpr bool kDown = MODE == kLowerT;                     // from the last
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  next_level_may_start();
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int w = blockIdx.x * (blockDim.x / 32) + warp;
+  if (w >= count) return;  // whole warps exit together
+  float* blk = (float*)sweep_smem + (long)warp * sweep_warp_entries<B>(cap);
+  float* xs = blk + cap * BB;
+  const int i = rows[w], di = diag[i];
+  const int first = kAfter ? di + 1 : ptr[i], n = (kAfter ? ptr[i + 1] : di) - first;
+  const int a = lane & (FV_LG - 1), al = a < B ? a : 0;
+  const bool live = a < B;
+  int col = 0;
+  // blocks k0 .. k0 + m of the row's order, and the lane's column
+  auto stage = [&](int k0, int m) {
+    const int q = kDown ? first + n - k0 - m : first + k0;
+    if (lane < m) col = idx[kDown ? q + m - 1 - lane : q + lane];
+    const float* p = val + (long)q * BB;
+    if constexpr (BB % 4 == 0) {
+#pragma unroll 4
+      for (int e = lane; e < m * (BB / 4); e += 32)
+        reinterpret_cast<float4*>(blk)[e] = reinterpret_cast<const float4*>(p)[e];
+    } else {
+#pragma unroll 4
+      for (int e = lane; e < m * BB; e += 32) blk[e] = p[e];
+    }
+  };
+  stage(0, min(n, cap));
+  float D[B], acc = 0.0f;
+  load_seg<B>(val + (long)di * BB + al * B, D);
+  if (!kAfter) acc = __ldcg(r + (long)i * B + al);
+  wait_level_before();
+  if (kAfter) acc = __ldcg(x + (long)i * B + al);
+  for (int k0 = 0; k0 < n; k0 += cap) {
+    const int m = min(n - k0, cap);
+    if (k0) {
+      __syncwarp();  // (the blocks before have been used)
+      stage(k0, m);
+    }
+    if (lane < m) {
+      float t[B];
+      load_x<B>(x + (long)col * B, t);
+#pragma unroll
+      for (int c = 0; c < B; ++c) xs[lane * B + c] = t[c];
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      float L[B], xj[B];
+      load_seg<B>(blk + (kDown ? m - 1 - k : k) * BB + al * B, L);
+      load_seg<B>(xs + k * B, xj);
+#pragma unroll
+      for (int c = 0; c < B; ++c) {
+        const int e = kDown ? B - 1 - c : c;
+        acc -= L[e] * xj[e];
+      }
+    }
+  }
+  const unsigned mask = 0xffffffffu;
+  if constexpr (MODE == kLower || MODE == kLowerUpper) {
+#pragma unroll
+    for (int c = 0; c < B; ++c) {
+      const float vc = __shfl_sync(mask, acc, c, FV_LG);
+      if (live && a > c) acc -= D[c] * vc;
+    }
+  }
+  if constexpr (MODE == kUpper || MODE == kLowerUpper)
+    acc = upper_block_solve<float, B>(acc, D, a, live, mask);
+  if constexpr (MODE == kUpperT) acc = lower_t_block_solve<float, B>(acc, D, a, live, mask);
+  if constexpr (MODE == kLowerT) {
+#pragma unroll
+    for (int c = B - 1; c >= 0; --c) {
+      const float vc = __shfl_sync(mask, acc, c, FV_LG);
+      if (live && a < c) acc -= D[c] * vc;
+    }
+  }
+  if (lane < B) x[(long)i * B + lane] = acc;
 }
 
 #include "ilu_narrow.inc.cuh"
@@ -1328,12 +1459,13 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
 
 // The widest levels (590,000 rows: 140 us) are bound by bytes and want warps in flight: one block at
 // a time, a launch after the other (the registers of a deeper read made them 180-220 us).  Below
-// kWideRows a row's chain of latencies is the level's time: blocks are read several at a time and
-// the next level is launched early.  128 x 96 x 96 channel: 16 levels of 26,000 rows 176 -> 156 us.
+// kWideRows a row's chain of latencies is the level's time: blocks are read two at a time and the
+// next level is launched early (16 levels of 26,000 rows 176 -> 156 us); fp32 below kDeepRows takes
+// a warp a row.
 constexpr int kWideRows = 65536, kDeepRows = 8192;
 
 template <class V>
-void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
+void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_t s) {
   IluView<V> F = view<V>(f);
   const bool lg = f->b > 1;
   bool after = false;  // the launch before on `s` is a level of this solve
@@ -1350,23 +1482,42 @@ void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
     const int grid = fv_blocks((long)cnt * FV_LG, 128);
     with_block_size(f->b, [&](auto B) {
       if (cnt >= kWideRows) launch(B, std::integral_constant<int, 1>{}, grid);
-      else if (cnt >= kDeepRows || sizeof(V) == 8) launch(B, std::integral_constant<int, 2>{}, grid);
-      else if constexpr (sizeof(V) == 4) launch(B, std::integral_constant<int, 4>{}, grid);
+      else launch(B, std::integral_constant<int, 2>{}, grid);
     });
+  };
+  // an fp32 level of few rows by k_ilu_sweep_w; false: not one
+  auto warp_rows = [&](auto mode, const int* rows, int cnt) {
+    if constexpr (sizeof(V) == 4) {
+      if (cnt >= kDeepRows) return false;
+      const bool T = mode() == kUpperT || mode() == kLowerT;
+      const int cap = std::max(1, std::min(f->row_cap - 1, kSweepBlocks));
+      with_block_size(f->b, [&](auto B) {
+        launch_level(k_ilu_sweep_w<B(), mode()>, fv_blocks(cnt, 4), s, after, 128,
+                     4 * sizeof(float) * sweep_warp_entries<B()>(cap), T ? (const int*)f->tptr : F.ptr,
+                     T ? (const int*)f->tidx : F.idx, T ? (const int*)f->tdiag : F.diag,
+                     T ? (const float*)f->tval : (const float*)F.val, rows, cnt, cap, r, x);
+      });
+      return true;
+    } else {
+      return false;
+    }
   };
   const V* tval = (const V*)f->tval;
   if (!transpose) {
     const size_t last = f->lv_fwd.size() - 2;
     levels_of(f->lv_fwd, f->rows_fwd, 0, [&](size_t l, const int* rows, int cnt) {
       if (!lg) {
-        k_ilu_lower<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, rows, cnt, x);
+        k_ilu_lower<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, rows, cnt, r, x);
         return;
       }
+      if (f->fuse_fb && l == last ? warp_rows(std::integral_constant<int, kLowerUpper>{}, rows, cnt)
+                                  : warp_rows(std::integral_constant<int, kLower>{}, rows, cnt))
+        return;
       lane_groups(cnt, [&](auto B, auto U, int grid) {
         if (f->fuse_fb && l == last)
-          launch_level(k_ilu_lower_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+          launch_level(k_ilu_lower_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, r, x);
         else
-          launch_level(k_ilu_lower_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+          launch_level(k_ilu_lower_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, r, x);
       });
     });
     levels_of(f->lv_bwd, f->rows_bwd, f->fuse_fb ? 1 : 0, [&](size_t, const int* rows, int cnt) {
@@ -1374,6 +1525,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
         k_ilu_upper<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, rows, cnt, x);
         return;
       }
+      if (warp_rows(std::integral_constant<int, kUpper>{}, rows, cnt)) return;
       lane_groups(cnt, [&](auto B, auto U, int grid) {
         launch_level(k_ilu_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
       });
@@ -1382,12 +1534,13 @@ void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
     levels_of(f->lv_tfwd, f->rows_tfwd, 0, [&](size_t, const int* rows, int cnt) {
       if (!lg) {
         k_ilu_upper_t<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->tptr, f->tidx, f->tblk, rows,
-                                                             cnt, x);
+                                                             cnt, r, x);
         return;
       }
+      if (warp_rows(std::integral_constant<int, kUpperT>{}, rows, cnt)) return;
       lane_groups(cnt, [&](auto B, auto U, int grid) {
         launch_level(k_ilu_upper_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
-                     tval, rows, cnt, x);
+                     tval, rows, cnt, r, x);
       });
     });
     levels_of(f->lv_tbwd, f->rows_tbwd, 0, [&](size_t, const int* rows, int cnt) {
@@ -1396,6 +1549,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, V* x, cudaStream_t s) {
                                                              cnt, x);
         return;
       }
+      if (warp_rows(std::integral_constant<int, kLowerT>{}, rows, cnt)) return;
       lane_groups(cnt, [&](auto B, auto U, int grid) {
         launch_level(k_ilu_lower_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
                      tval, rows, cnt, x);
@@ -1526,7 +1680,7 @@ int ilu_apply(FvIlu0* f, const V* r, V* x, int transpose, cudaStream_t s) {
   FV_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) {
     // inside a caller's stream capture (a whole V-cycle as one graph): the level kernels go
-    // straight into the caller's graph and run in place on x; nothing is allocated or built here
+    // straight into the caller's graph; nothing is allocated or built here
     if (t && !f->tptr) {
       fv_set_error("fv_ilu0_apply: the transposed-solve structures are built by a transposed "
                    "solve outside stream capture first");
@@ -1537,9 +1691,7 @@ int ilu_apply(FvIlu0* f, const V* r, V* x, int transpose, cudaStream_t s) {
       return FV_ERR_ARG;
     }
     if (runs(f, t)) return launch_run<V>(f, t, r, x, s);
-    if ((const void*)x != (const void*)r)
-      FV_CUDA_TRY(cudaMemcpyAsync(x, r, sizeof(V) * n, cudaMemcpyDeviceToDevice, s));
-    launch_apply_levels<V>(f, t, x, s);
+    launch_apply_levels<V>(f, t, r, x, s);
     FV_CUDA_TRY(cudaGetLastError());
     return FV_OK;
   }
@@ -1549,7 +1701,7 @@ int ilu_apply(FvIlu0* f, const V* r, V* x, int transpose, cudaStream_t s) {
   }
   if (runs(f, t)) return launch_run<V>(f, t, r, x, s);
   if (!f->apply_exec[t]) {
-    int rc = capture([&](cudaStream_t cs) { launch_apply_levels<V>(f, t, w, cs); },
+    int rc = capture([&](cudaStream_t cs) { launch_apply_levels<V>(f, t, w, w, cs); },
                      &f->apply_exec[t]);
     if (rc != FV_OK) return rc;
   }
