@@ -83,6 +83,7 @@ SIGNATURES = {
     "fv_ilu0_create": (c_int, [c_int, c_int, P, P, c_int, P, P]),
     "fv_ilu0_clone": (c_int, [P, c_int, P, P]),
     "fv_ilu0_destroy": (c_int, [P]),
+    "fv_ilu0_factor": (c_int, [P, P, c_int, P]),
     "fv_ilu0_factor_start": (c_int, [P, P, c_int, P]),
     "fv_ilu0_factor_finish": (c_int, [P, P]),
     "fv_ilu0_apply": (c_int, [P, P, P, c_int, P]),
