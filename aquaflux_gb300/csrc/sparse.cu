@@ -876,10 +876,8 @@ __global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, const V
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = F.ptr[i], di = F.diag[i];
-  if (U > 1) {
-    ask_blocks<V, B>(F.val, q0, di - q0, a);
-    wait_level_before();
-  }
+  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a);
+  if (U > 1) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
@@ -939,10 +937,8 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int di = F.diag[i], re = F.ptr[i + 1];
-  if (U > 1) {
-    ask_blocks<V, B>(F.val, di + 1, re - di - 1, a);
-    wait_level_before();
-  }
+  ask_blocks<V, B>(F.val, di, re - di, a);
+  if (U > 1) wait_level_before();
   V acc = live ? x[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, x, di + 1, re - di - 1, a, live, mask);
   V D[B];
@@ -966,10 +962,8 @@ __global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, c
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = F.ptr[i], di = F.diag[i];
-  if (U > 1) {
-    ask_blocks<V, B>(F.val, q0, di - q0, a);
-    wait_level_before();
-  }
+  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a);
+  if (U > 1) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
@@ -1029,10 +1023,8 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = tptr[i], di = tdiag[i];
-  if (U > 1) {
-    ask_blocks<V, B>(tval, q0, di - q0, a);
-    wait_level_before();
-  }
+  ask_blocks<V, B>(tval, q0, di - q0 + 1, a);
+  if (U > 1) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, 1, U>(acc, tval, tidx, z, q0, di - q0, a, live, mask);
   V Dc[B];  // Dc[c] = D(c, a): row a of D^T
@@ -1059,10 +1051,8 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int di = tdiag[i], last = tptr[i + 1] - 1;
-  if (U > 1) {
-    ask_blocks<V, B>(tval, di + 1, last - di, a);
-    wait_level_before();
-  }
+  ask_blocks<V, B>(tval, di, last - di + 1, a);
+  if (U > 1) wait_level_before();
   V acc = live ? x[(long)i * B + a] : V(0);
   acc = subtract_blocks<V, B, -1, U>(acc, tval, tidx, x, last, last - di, a, live, mask);
   V Dc[B];
@@ -1457,8 +1447,9 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   }
 }
 
-// The widest levels (590,000 rows: 140 us) are bound by bytes and want warps in flight: one block at
-// a time, a launch after the other (the registers of a deeper read made them 180-220 us).  Below
+// The widest levels (590,000 rows: 120 us) are bound by bytes and want warps in flight: one block at
+// a time, a launch after the other (the registers of a deeper read made them 180-220 us), and all
+// lines of a row asked of the L2 cache first (125 -> 120 us, a 1.2M-row V-cycle 1870 -> 1844).  Below
 // kWideRows a row's chain of latencies is the level's time: blocks are read two at a time and the
 // next level is launched early (16 levels of 26,000 rows 176 -> 156 us); fp32 below kDeepRows takes
 // a warp a row.
