@@ -1368,8 +1368,11 @@ int build_run(FvIlu0* f, int t, const std::vector<int>& fwd, const std::vector<i
 template <class V>
 int pack_run(FvIlu0* f, int t, cudaStream_t s) {
   FvIlu0::Run& run = f->run[t];
+  // fp32 rows of more blocks than the records hold go by k_ilu_sweep_w, which has all of them in
+  // place (212 coarse rows of 20 to 40 blocks: 22 us a solve, 40 us by k_ilu_run)
   if (!run.row || !run_block_size(f->b, sizeof(V)) ||
-      run_smem_bytes(f->n, f->b, run.nlev, sizeof(V)) > kRunSmem)
+      run_smem_bytes(f->n, f->b, run.nlev, sizeof(V)) > kRunSmem ||
+      (sizeof(V) == 4 && f->row_cap > 2 * kRunBlocks + 1))
     return FV_OK;
   const long lanes = 2L * f->n * run_lanes(f->b);
   if (!run.rec) FV_CUDA_TRY(cudaMalloc(&run.rec, sizeof(V) * lanes * run_entries(f->b, run.k)));
