@@ -1079,6 +1079,7 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // lane groups are faster (levels of 26,000 rows: 1943 us with a warp a row).
 // The operations and their order are the lane-group kernels'.
 enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
+constexpr int kDeepRows = 8192;
 
 constexpr int kSweepBlocks = 32;  // blocks in shared memory at a time: a column a lane
 template <int B>
@@ -1197,6 +1198,77 @@ __global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* 
     }
   }
   if (lane < B) x[(long)i * B + lane] = acc;
+}
+
+// fp32 y = A x or, RES, rhs - A x of fewer than kWarpProduct block rows: a warp per row as above,
+// which pays the memory's latency once a row instead of once a block; k_bsr_spmv_b's operations in
+// its order.  b = 6, coarse Galerkin rows: 5,370 of them 15.0 -> 8.3 us (7.5 -> 6.5 from L2), 212 of
+// them 13.6 -> 4.3 (6.0 -> 2.8).  The line: rows of a few blocks gain from one round of loads only
+// where the chip is not full of them (7 blocks, b = 6: 1,000 rows 2.6 -> 2.3 us, 8,000 rows 3.4 ->
+// 4.9; 5 blocks, b = 3: 4,096 rows 2.4 either way).
+constexpr int kWarpProduct = 6144;
+template <int B, bool RES>
+__global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restrict__ ptr,
+                                                    const int* __restrict__ idx,
+                                                    const float* __restrict__ val,
+                                                    const float* __restrict__ x,
+                                                    const float* __restrict__ rhs, float* y) {
+  constexpr int BB = B * B;
+  __shared__ __align__(16) float smem[4 * sweep_warp_entries<B>(kSweepBlocks)];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 4 + warp;
+  if (i >= nbr) return;  // whole warps exit together
+  float* blk = smem + warp * sweep_warp_entries<B>(kSweepBlocks);
+  float* xs = blk + kSweepBlocks * BB;
+  const int q0 = ptr[i], n = ptr[i + 1] - q0, al = lane < B ? lane : 0;
+  const float own = RES ? rhs[(long)i * B + al] : 0.0f;
+  float acc = 0.0f;
+  for (int k0 = 0; k0 < n; k0 += kSweepBlocks) {
+    const int m = min(n - k0, kSweepBlocks);
+    __syncwarp();  // (the blocks before have been used)
+    const float* p = val + (long)(q0 + k0) * BB;
+    if constexpr (BB % 4 == 0) {
+#pragma unroll 4
+      for (int e = lane; e < m * (BB / 4); e += 32)
+        reinterpret_cast<float4*>(blk)[e] = reinterpret_cast<const float4*>(p)[e];
+    } else {
+#pragma unroll 4
+      for (int e = lane; e < m * BB; e += 32) blk[e] = p[e];
+    }
+    if (lane < m) {
+      float t[B];
+      load_seg<B>(x + (long)idx[q0 + k0 + lane] * B, t);
+#pragma unroll
+      for (int c = 0; c < B; ++c) xs[lane * B + c] = t[c];
+    }
+    __syncwarp();
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      float L[B], xj[B];
+      load_seg<B>(blk + k * BB + al * B, L);
+      load_seg<B>(xs + k * B, xj);
+#pragma unroll
+      for (int c = 0; c < B; ++c) acc += L[c] * xj[c];
+    }
+  }
+  if (lane < B) y[(long)i * B + lane] = RES ? own - acc : acc;
+}
+
+// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8)
+template <class V, bool RES>
+void launch_spmv_b(int nbr, int b, const int* indptr, const int* indices, const V* values,
+                   const V* x, const V* rhs, V* y, cudaStream_t s) {
+  with_block_size(b, [&](auto B) {
+    if constexpr (sizeof(V) == 4) {
+      if (nbr < kWarpProduct) {
+        k_bsr_spmv_w<B(), RES><<<fv_blocks(nbr, 4), 128, 0, s>>>(nbr, indptr, indices, values, x,
+                                                                 rhs, y);
+        return;
+      }
+    }
+    k_bsr_spmv_b<V, B(), RES><<<fv_blocks((long)nbr * b, kThreads), kThreads, 0, s>>>(
+        nbr, indptr, indices, values, x, rhs, y);
+  });
 }
 
 #include "ilu_narrow.inc.cuh"
@@ -1456,7 +1528,7 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
 // kWideRows a row's chain of latencies is the level's time: blocks are read two at a time and the
 // next level is launched early (16 levels of 26,000 rows 176 -> 156 us); fp32 below kDeepRows takes
 // a warp a row.
-constexpr int kWideRows = 65536, kDeepRows = 8192;
+constexpr int kWideRows = 65536;
 
 template <class V>
 void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_t s) {
@@ -2057,10 +2129,7 @@ int spmv(int nbr, int b, const int* indptr, const int* indices, const V* values,
   if (!transpose) {
     const bool aligned = ((uintptr_t)values % 16 == 0) && ((uintptr_t)x % 16 == 0);
     if (aligned && b >= 2 && b <= 8)
-      with_block_size(b, [&](auto B) {
-        k_bsr_spmv_b<V, B(), false><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(
-            nbr, indptr, indices, values, x, nullptr, y);
-      });
+      launch_spmv_b<V, false>(nbr, b, indptr, indices, values, x, (const V*)nullptr, y, s);
     else
       k_bsr_spmv<V><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
                                                                    values, x, nullptr, y);
@@ -2180,14 +2249,10 @@ int bsr_residual(int nbr, int b, const int* indptr, const int* indices, const V*
     fv_set_error("fv_bsr_residual: bad arguments");
     return FV_ERR_ARG;
   }
-  const long rows = (long)nbr * b;
-  const int grid = fv_blocks(rows, kThreads);
   if (((uintptr_t)values | (uintptr_t)x) % 16 == 0 && b >= 2 && b <= 8)
-    with_block_size(b, [&](auto B) {
-      k_bsr_spmv_b<V, B(), true><<<grid, kThreads, 0, s>>>(nbr, indptr, indices, values, x, rhs, r);
-    });
+    launch_spmv_b<V, true>(nbr, b, indptr, indices, values, x, rhs, r, s);
   else
-    k_bsr_spmv<V><<<grid, kThreads, 0, s>>>(nbr, b, indptr, indices, values, x, rhs, r);
+    k_bsr_spmv<V><<<fv_blocks((long)nbr * b, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices, values, x, rhs, r);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
 }
