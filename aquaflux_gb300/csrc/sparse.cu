@@ -552,6 +552,15 @@ __device__ __forceinline__ float quotient(float x, float piv, float) { return x 
 // Levels of at least this many rows take 8 lanes a row (fp32, b = 6: 131,072 rows of 6 lower blocks
 // 187 us, 490 us with a warp a row; 5,900 rows of 8-15 lower blocks 120 us, 45 us with a warp).
 constexpr int kFactorWide = 65536;
+// fp64 issue is four times scarcer for a warp a row than for four rows a warp, so there the line is
+// where the warps' rows fill the SMs' fp64 units; with a lane an entry (b <= 4) it lies higher
+// (3D 48^3, 142 level sets of up to 1,728 rows: b = 6 lane groups 6.55 ms, warps 5.9 ms, warps below
+// 1,024 rows 5.15; b = 4 3.91, 2.46, 2.79.  80^3, up to 4,800 rows, b = 6: 13.0, 20.7 and 11.6).
+// And a level launched early is placed where it finds room, not where fp64 units are free: it pays
+// only while a level has no more rows than there are SMs (64 x 64 cavity 793 us, 1026 without; the
+// 48^3 b = 6 factor 8.4 ms with every level early, 6.2 with none).
+constexpr int kFactorWide64(int b) { return b <= 4 ? 2048 : 1024; }
+constexpr int kEarly64 = 152;
 constexpr size_t kFactorSmem = 96 * 1024;
 
 // Shared memory of one warp: the matches of one lower block, the row's columns (padded to a multiple
@@ -1494,7 +1503,7 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) {
     const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
     if (cnt == 0) continue;
-    const bool early = after;
+    const bool early = after && (sizeof(V) == 4 || cnt <= kEarly64);
     after = false;
     const size_t wb = factor_warp_bytes<V>(f->row_cap, f->b * f->b);
     if (f->b == 1 || wb > kFactorSmem) {  // scalar, or hundreds of blocks in a row
@@ -1502,7 +1511,7 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
                                                                 f->zero_flag);
       continue;
     }
-    if (cnt >= kFactorWide) {
+    if (cnt >= (sizeof(V) == 4 ? kFactorWide : kFactorWide64(f->b))) {
       with_block_size(f->b, [&](auto B) {
         k_ilu_factor_lgb<V, B()><<<fv_blocks((long)cnt * FV_LG, 128), 128, 0, s>>>(
             F, f->rows_fwd + f->lv_fwd[l], cnt, (V*)f->rp, f->zero_flag);
@@ -1518,7 +1527,7 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
                    (const int*)f->rows_fwd + f->lv_fwd[l], cnt, f->row_cap, (V*)f->rp,
                    f->zero_flag);
     });
-    after = true;
+    after = sizeof(V) == 4 || cnt <= kEarly64;
   }
 }
 
@@ -1528,7 +1537,10 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
 // kWideRows a row's chain of latencies is the level's time: blocks are read two at a time and the
 // next level is launched early (16 levels of 26,000 rows 176 -> 156 us); fp32 below kDeepRows takes
 // a warp a row.
-constexpr int kWideRows = 65536;
+// fp64 levels of kDeep64 rows and more are bound by fp64 issue and read like the widest: a solve in
+// 3D with b = 6, 48^3 (levels of up to 1,728 rows) 2.34 -> 1.75 ms; 24^3 (432 rows) 671 us two
+// blocks at a time with an early launch, 686 one at a time.
+constexpr int kWideRows = 65536, kDeep64 = 512;
 
 template <class V>
 void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_t s) {
@@ -1547,7 +1559,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
   auto lane_groups = [&](int cnt, auto&& launch) {
     const int grid = fv_blocks((long)cnt * FV_LG, 128);
     with_block_size(f->b, [&](auto B) {
-      if (cnt >= kWideRows) launch(B, std::integral_constant<int, 1>{}, grid);
+      if (cnt >= (sizeof(V) == 4 ? kWideRows : kDeep64)) launch(B, std::integral_constant<int, 1>{}, grid);
       else launch(B, std::integral_constant<int, 2>{}, grid);
     });
   };
