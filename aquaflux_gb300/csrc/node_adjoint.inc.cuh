@@ -18,7 +18,8 @@
 // dual-number evaluation of the forward formula per geometric input (GeoSeed).
 // The reverse pass costs a face about one flux evaluation; seeding every geometric input of every
 // face cost 31 dual-number flux evaluations per face, FP64-bound (48^3 SST channel, GB300: the
-// whole node VJP 21.9 ms seeded, 1.82 ms written out).  Every scatter is a gather over a precomputed incidence list: deterministic.
+// whole node VJP 21.9 ms seeded, 1.73 ms written out).  Every scatter is a gather over a precomputed
+// incidence list: deterministic.
 // Advection: first-order upwind and the limited linear upwind reconstruction (the centroids it
 // reads, and the Venkatakrishnan limiters' geometry by seeded dual evaluations, k_nadj_limiter).
 // Gradients: the compact scheme (with its relaxation) and the corrected scheme's swept solve
