@@ -208,7 +208,8 @@ class AmgHierarchy:
             self.levels.append(_Level(step["n_coarse"], b, step["indptr"], step["indices"],
                                       precision, kl(i + 1)))
         last = self.levels[-1]
-        self._sides = [torch.cuda.Stream() for _ in self.levels]  # where each level is factored
+        # where each level is factored
+        self._sides = [torch.cuda.Stream(priority=-1 if i else 0) for i in range(len(self.levels))]
         nd = last.n * b
         self.dense = None
         if len(self.levels) > 1 and (coarse_solve == "dense"
@@ -255,31 +256,36 @@ class AmgHierarchy:
         else:
             lv0.values.copy_(fine_values)
         # The levels' factors hang on the values only, and the coarse ones are chains of a few rows
-        # a level set that leave most SMs idle: each is factored on a stream of its own, the next
-        # level's Galerkin sums queued before it, and the zero pivots are read at the end.  64^3 SST
-        # channel: 3044 us a refresh and cycle, one after the other with a host round trip each 3334.
+        # a level set that leave most SMs idle: each is factored on a stream of its own behind its
+        # values, the coarse ones before the fine one, which fills the chip (streams of higher
+        # priority, and the fine one behind all sums), and the zero pivots are read at the end.
+        # SST channel, a refresh and a cycle: 64^3 3334 -> 3044 us for factors side by side instead of
+        # one after the other with a host round trip each, and 2698 -> 2624 for the coarse ones first;
+        # 30^3 645 -> 581 for the latter.
         galerkin = getattr(lib(), "fv_galerkin_" + self.sfx)
         main = torch.cuda.current_stream()
-        started = []
+        ready = []  # when a level's values are there
+        for fine, coarse in zip(self.levels, self.levels[1:]):
+            ready.append(main.record_event())
+            t = fine.coarse
+            check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
+                           ptr(fine.values), int(fine.values.dtype == torch.float64),
+                           ptr(coarse.values), _stream()))
+        ready.append(main.record_event())
+        ready[0] = ready[-1]
+        n_factors = len(self.levels) - (self.dense is not None)
+        started = {}
         try:
-            for fine, coarse, side in zip(self.levels, self.levels[1:] + [None], self._sides):
-                if coarse is not None:
-                    values_ready = main.record_event()
-                    t = fine.coarse
-                    check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
-                                   ptr(fine.values), int(fine.values.dtype == torch.float64),
-                                   ptr(coarse.values), _stream()))
-                    started.append((fine, side, fine.ilu.start_factor(fine.values, side, values_ready)))
-                elif self.dense is None:
-                    started.append((fine, None, fine.ilu.start_factor(fine.values)))
-                else:
-                    self._invert_coarsest()
+            for i in [*range(1, n_factors), 0]:
+                lv = self.levels[i]
+                started[i] = lv.ilu.start_factor(lv.values, self._sides[i], ready[i])
+            if self.dense is not None:
+                self._invert_coarsest()
         finally:
-            for _, side, _ in started:
-                if side is not None:
-                    main.wait_stream(side)
-            for lv, _, factor in started:  # (an error is the finest level's)
-                lv.ilu.finish_factor(*factor)
+            for i in started:
+                main.wait_stream(self._sides[i])
+            for i in sorted(started):  # (an error is the finest level's)
+                self.levels[i].ilu.finish_factor(*started[i])
         for lv in self.levels:
             lv.transpose_values()
 
