@@ -84,7 +84,7 @@ SIGNATURES = {
     "fv_ilu0_clone": (c_int, [P, c_int, P, P]),
     "fv_ilu0_destroy": (c_int, [P]),
     "fv_ilu0_factor": (c_int, [P, P, c_int, P]),
-    "fv_ilu0_factor_start": (c_int, [P, P, c_int, P]),
+    "fv_ilu0_factor_start": (c_int, [P, P, c_int, c_int, P]),
     "fv_ilu0_factor_finish": (c_int, [P, P]),
     "fv_ilu0_apply": (c_int, [P, P, P, c_int, P]),
     "fv_ilu0_factor_values": (c_int, [P, P, P]),

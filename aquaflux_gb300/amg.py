@@ -208,8 +208,6 @@ class AmgHierarchy:
             self.levels.append(_Level(step["n_coarse"], b, step["indptr"], step["indices"],
                                       precision, kl(i + 1)))
         last = self.levels[-1]
-        # where each level is factored
-        self._sides = [torch.cuda.Stream(priority=-1 if i else 0) for i in range(len(self.levels))]
         nd = last.n * b
         self.dense = None
         if len(self.levels) > 1 and (coarse_solve == "dense"
@@ -263,29 +261,28 @@ class AmgHierarchy:
         # one after the other with a host round trip each, and 2698 -> 2624 for the coarse ones first;
         # 30^3 645 -> 581 for the latter.
         galerkin = getattr(lib(), "fv_galerkin_" + self.sfx)
-        main = torch.cuda.current_stream()
-        ready = []  # when a level's values are there
-        for fine, coarse in zip(self.levels, self.levels[1:]):
-            ready.append(main.record_event())
-            t = fine.coarse
-            check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
-                           ptr(fine.values), int(fine.values.dtype == torch.float64),
-                           ptr(coarse.values), _stream()))
-        ready.append(main.record_event())
-        ready[0] = ready[-1]
         n_factors = len(self.levels) - (self.dense is not None)
-        started = {}
+        started = []  # (level, values)
         try:
-            for i in [*range(1, n_factors), 0]:
-                lv = self.levels[i]
-                started[i] = lv.ilu.start_factor(lv.values, self._sides[i], ready[i])
+            for i, (fine, coarse) in enumerate(zip(self.levels, self.levels[1:]), 1):
+                t = fine.coarse
+                check(galerkin(t["n_coarse_blocks"], self.b, ptr(t["gptr"]), ptr(t["glist"]),
+                               ptr(fine.values), int(fine.values.dtype == torch.float64),
+                               ptr(coarse.values), _stream()))
+                if i < n_factors:
+                    started.append((coarse, coarse.ilu.start_factor(coarse.values, urgent=True)))
+            started.insert(0, (lv0, lv0.ilu.start_factor(lv0.values)))
             if self.dense is not None:
                 self._invert_coarsest()
         finally:
-            for i in started:
-                main.wait_stream(self._sides[i])
-            for i in sorted(started):  # (an error is the finest level's)
-                self.levels[i].ilu.finish_factor(*started[i])
+            failed = None
+            for lv, _ in started:
+                try:
+                    lv.ilu.finish_factor()
+                except (ZeroDivisionError, FvError) as e:
+                    failed = failed or e  # (the finest level's)
+            if failed is not None:
+                raise failed
         for lv in self.levels:
             lv.transpose_values()
 

@@ -1333,6 +1333,8 @@ struct FvIlu0 {
   void* val = nullptr;
   void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
   int row_cap = 0;        // most blocks in a row
+  cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
+  cudaEvent_t side_event = nullptr;
   void* tval = nullptr;   // (b > 1) the factor's blocks transposed, in the transpose's order
   unsigned long long* zero_flag = nullptr;
   // level sets: rows grouped by level (device), level boundaries (host)
@@ -1879,6 +1881,8 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
 
 extern "C" int fv_ilu0_destroy(FvIlu0* f) {
   if (!f) return FV_OK;
+  if (f->side) cudaStreamDestroy(f->side);
+  if (f->side_event) cudaEventDestroy(f->side_event);
   cudaFree(f->ptr);
   cudaFree(f->idx);
   cudaFree(f->diag);
@@ -1985,12 +1989,8 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   return FV_OK;
 }
 
-extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, void* stream) {
-  if (!f || !values || !f->val) {
-    fv_set_error("fv_ilu0_factor: bad arguments");
-    return FV_ERR_ARG;
-  }
-  cudaStream_t s = (cudaStream_t)stream;
+namespace {
+int factor_start(FvIlu0* f, const void* values, int values_f64, cudaStream_t s) {
   const long n = (long)f->nnzb * f->b * f->b;
   if (f->precision == 64) {
     FV_CUDA_TRY(cudaMemcpyAsync(f->val, values, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
@@ -2002,18 +2002,51 @@ extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f6
     FV_CUDA_TRY(cudaMemcpyAsync(f->val, values, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
   return ilu_factor_start<float>(f, s);
 }
+}  // namespace
 
-extern "C" int fv_ilu0_factor_finish(FvIlu0* f, void* stream) {
-  if (!f || !f->val) {
+extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream) {
+  if (!f || !values || !f->val) {
     fv_set_error("fv_ilu0_factor: bad arguments");
     return FV_ERR_ARG;
   }
-  return ilu_factor_finish(f, (cudaStream_t)stream);
+  const int rc = factor_start(f, values, values_f64, (cudaStream_t)stream);
+  return rc == FV_OK ? ilu_factor_finish(f, (cudaStream_t)stream) : rc;
 }
 
-extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream) {
-  const int rc = fv_ilu0_factor_start(f, values, values_f64, stream);
-  return rc == FV_OK ? fv_ilu0_factor_finish(f, stream) : rc;
+extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, int urgent,
+                                    void* stream) {
+  if (!f || !values || !f->val) {
+    fv_set_error("fv_ilu0_factor_start: bad arguments");
+    return FV_ERR_ARG;
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  FV_CUDA_TRY(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) {
+    fv_set_error("fv_ilu0_factor_start: a factorisation cannot be captured (its zero pivots are read "
+                 "by the host)");
+    return FV_ERR_CUDA;
+  }
+  if (!f->side) {
+    int least = 0, greatest = 0;
+    FV_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    if (!f->side_event)
+      FV_CUDA_TRY(cudaEventCreateWithFlags(&f->side_event, cudaEventDisableTiming));
+    FV_CUDA_TRY(cudaStreamCreateWithPriority(&f->side, cudaStreamNonBlocking,
+                                             urgent ? greatest : least));
+  }
+  FV_CUDA_TRY(cudaEventRecord(f->side_event, (cudaStream_t)stream));
+  FV_CUDA_TRY(cudaStreamWaitEvent(f->side, f->side_event, 0));
+  return factor_start(f, values, values_f64, f->side);
+}
+
+extern "C" int fv_ilu0_factor_finish(FvIlu0* f, void* stream) {
+  if (!f || !f->side) {
+    fv_set_error("fv_ilu0_factor_finish: no factorisation was started");
+    return FV_ERR_ARG;
+  }
+  FV_CUDA_TRY(cudaEventRecord(f->side_event, f->side));
+  FV_CUDA_TRY(cudaStreamWaitEvent((cudaStream_t)stream, f->side_event, 0));
+  return ilu_factor_finish(f, f->side);
 }
 
 extern "C" int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, void* stream) {

@@ -103,11 +103,32 @@ class Ilu0:
         return self._n * self._b
 
     def refactor(self, values) -> None:
-        self.finish_factor(*self.start_factor(values))
+        v = self._device_values(values)
+        try:
+            check(lib().fv_ilu0_factor(self._h, ptr(v), int(v.dtype == torch.float64), _stream()))
+        except FvError as e:
+            _raise(e)
 
-    def start_factor(self, values, stream: torch.cuda.Stream | None = None, after=None):
-        """Enqueue the factorization of new values on the current stream, or on ``stream`` behind
-        the event ``after`` (when the values are there and earlier solves with this factor done).  Gives what :meth:`finish_factor`, which has to follow, takes."""
+    def start_factor(self, values, urgent: bool = False):
+        """Enqueue the factorization of new values on a stream of this factor's own, behind what the
+        current stream holds by now; gives the values it reads, to be kept until
+        :meth:`finish_factor`, which has to follow."""
+        v = self._device_values(values)
+        try:
+            check(lib().fv_ilu0_factor_start(self._h, ptr(v), int(v.dtype == torch.float64),
+                                             int(urgent), _stream()))
+        except FvError as e:
+            _raise(e)
+        return v
+
+    def finish_factor(self) -> None:
+        """Wait for a started factorization and report its zero pivot."""
+        try:
+            check(lib().fv_ilu0_factor_finish(self._h, _stream()))
+        except FvError as e:
+            _raise(e)
+
+    def _device_values(self, values) -> torch.Tensor:
         v = torch.as_tensor(values)
         if v.numel() != self._nvals:
             raise ValueError(f"expected {self._nvals} values for this pattern, got {v.numel()}.")
@@ -117,25 +138,7 @@ class Ilu0:
             v = v.to(torch.float64)
         if self._precision == 32 and v.dtype not in (torch.float32, torch.float64):
             v = v.to(torch.float64)
-        try:
-            if stream is not None:
-                if v is values:
-                    stream.wait_event(after)
-                else:  # converted on the current stream
-                    stream.wait_stream(torch.cuda.current_stream())
-            s = _stream() if stream is None else int(stream.cuda_stream)
-            check(lib().fv_ilu0_factor_start(self._h, ptr(v), int(v.dtype == torch.float64), s))
-        except FvError as e:
-            _raise(e)
-        return v, s
-
-    def finish_factor(self, values, stream: int) -> None:
-        """Wait for a started factorization (``values``: held until then) and report its zero
-        pivot."""
-        try:
-            check(lib().fv_ilu0_factor_finish(self._h, stream))
-        except FvError as e:
-            _raise(e)
+        return v
 
     def factor_values(self) -> torch.Tensor:
         out = torch.empty(self._nvals, dtype=self._dtype, device="cuda")

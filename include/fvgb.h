@@ -361,9 +361,11 @@ int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvIlu0** out);
 /* Numeric factorization of new values (device, nnzb * b * b, same dtype as `precision`, or
  * float64 when values_f64 != 0 and precision == 32: converted on the fly). */
 int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream);
-/* Its two halves, to factor several matrices side by side on streams of their own: start enqueues
- * the factorization, finish (same stream) waits for it and reports a zero pivot. */
-int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, void* stream);
+/* Its two halves, to factor several matrices side by side: start enqueues the factorization on a
+ * stream of the factor's own (of higher priority if `urgent`; fixed by the first call) behind what
+ * `stream` holds by then; finish waits for it, also on `stream`, and reports a zero pivot.  `values`
+ * stay untouched in between.  Not under stream capture. */
+int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, int urgent, void* stream);
 int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
 /* x = (LU)^-1 r, or (LU)^-T r when transpose != 0.  Device vectors of `precision`.  On a stream
  * under capture the level kernels are recorded into the caller's graph (x may alias r, and must be
