@@ -176,8 +176,9 @@ __device__ __forceinline__ void cluster_sync() {
 
 // Cuthill-McKee sweeps from `placed` placed nodes on: from node `seed` alone, or (seeds given) from
 // every unplaced node of seeds in turn until all are placed.  order and mark change under the
-// other blocks' hands, so they are read past the L1 cache.  result: placed nodes, the position of
-// a seed out of range or -1.
+// other blocks' hands, so they are read past the L1 cache.  result: placed nodes and -1, or the
+// position of a seed out of range; -1 and the level's size where a level would place more nodes
+// than are left (a row lists a node twice), before anything of it is written.
 __global__ void __launch_bounds__(1024)
     k_rcm_sweep(int n, const int* __restrict__ ptr, const int* __restrict__ idx, int seed,
                 const long* __restrict__ seeds, int placed, int* order, int* mark, int* result) {
@@ -284,6 +285,11 @@ __global__ void __launch_bounds__(1024)
           sum += totals[parity][k];
         }
         parity ^= 1;
+        if (base + sum > n) {  // (the same in every block)
+          bad = 2;
+          seed = base + sum - le;
+          break;
+        }
         if (c > 0) {  // the neighbours won, by (degree, index), and mark them placed
           int kid[kMaxDegree], kdeg[kMaxDegree];
           int m = 0;
@@ -307,14 +313,16 @@ __global__ void __launch_bounds__(1024)
         base += sum;
       }
       cluster_sync();
+      if (bad) break;
       ls = le;
       le = base;
     }
+    if (bad) break;
     placed = le;
     if (!seeds) break;
   }
   if (gid == 0) {
-    result[0] = placed;
+    result[0] = bad == 2 ? -1 : placed;
     result[1] = bad ? seed : -1;
   }
   cluster_sync();  // no block leaves while another may still write to its shared memory
@@ -426,7 +434,7 @@ extern "C" int fv_rcm_permutation(int n, const int* indptr, const int* indices,
   };
   k_fill_int<<<blocks_of(n), kThreads, 0, s>>>(n, mark, INT_MAX);
   int rc = sweep(0);
-  if (rc == FV_OK && h[0] < n) {  // the other components, from the seed order
+  if (rc == FV_OK && h[0] >= 0 && h[0] < n) {  // the other components, from the seed order
     rc = cudaMalloc(&seeds, sizeof(long) * (size_t)n) == cudaSuccess &&
                  cudaMemcpyAsync(seeds, seed_order, sizeof(long) * (size_t)n,
                                  cudaMemcpyHostToDevice, s) == cudaSuccess
@@ -435,6 +443,10 @@ extern "C" int fv_rcm_permutation(int n, const int* indptr, const int* indices,
   }
   cudaFree(seeds);
   if (rc != FV_OK) return rc;
+  if (h[0] < 0) {
+    fv_set_error("fv_rcm_permutation: inconsistent level size %d", h[1]);
+    return FV_ERR_ARG;
+  }
   if (h[1] >= 0) return bad_seed(seed_order[h[1]]);
   if (h[0] < n) {
     fv_set_error("fv_rcm_permutation: seed order is not a permutation");
