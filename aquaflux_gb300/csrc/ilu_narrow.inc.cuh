@@ -268,8 +268,9 @@ int launch_run_b(const RunView<V>& R, int widest, bool transpose, const V* r, V*
     auto kern = R.k <= 2 ? (transpose ? k_ilu_run<V, B, 2, true> : k_ilu_run<V, B, 2, false>)
                          : (transpose ? k_ilu_run<V, B, kRunBlocks, true>
                                       : k_ilu_run<V, B, kRunBlocks, false>);
+    // the limit belongs to the function, which other threads launch with other sizes: one value
     FV_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
+                                     (int)kRunSmem));
     kern<<<1, threads, smem, s>>>(R, r, x);
     FV_CUDA_TRY(cudaGetLastError());
   }
