@@ -67,8 +67,20 @@ __device__ __forceinline__ V pivot_quotient(V acc, V piv, V rpiv) {
   return acc / piv;
 }
 
+// A quotient by a pivot that may stand in a record: between 2^-256 and 2^256.
+__device__ __forceinline__ bool scalable(double q) {
+  const int e = (__double2hiint(q) >> 20 & 0x7ff) - 1023;
+  return e >= -256 && e < 256;
+}
+__device__ __forceinline__ bool finite_hi(double x) {  // no fp64 comparison
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+
 // The records of a solve from the factor's blocks (val: transposed blocks for the transposed solve,
-// whose backward sweep takes a row's blocks from the last one down).
+// whose backward sweep takes a row's blocks from the last one down).  A row of the fp64 forward
+// solve whose pivot's reciprocal or scaled entries would be large or small enough for a product with
+// them to leave the range of doubles stays as it is, marked by a NaN for the reciprocal, and is
+// divided last.
 template <class V>
 __global__ void k_run_pack(int n, int b, int k, bool transposed, const int4* row, const V* val,
                            V* rec) {
@@ -77,13 +89,19 @@ __global__ void k_run_pack(int n, int b, int k, bool transposed, const int4* row
   const int s = (int)(t / lg), a = (int)(t % lg);
   if (s >= 2 * n || a >= b) return;
   const int4 d = row[s];
-  const bool scaled = sizeof(V) == 8 && !transposed;
   const int step = transposed && s >= n ? -1 : 1;
   V* o = rec + (long)s * run_entries(b, k) * lg + a;
   const V* D = val + ((long)d.w * b + a) * b;
   const V piv = D[a];
+  V rpiv = V(1) / piv;
+  bool scaled = sizeof(V) == 8 && !transposed;
+  if (scaled) {
+    scaled = scalable(rpiv);
+    for (int c = a + 1; c < b; ++c) scaled = scaled && (D[c] == V(0) || scalable(D[c] / piv));
+    if (!scaled) rpiv = (V)__longlong_as_double(0x7ff8000000000000LL);
+  }
   for (int c = 0; c < b; ++c) o[(long)c * lg] = scaled && c > a ? D[c] / piv : D[c];
-  o[(long)b * lg] = V(1) / piv;
+  o[(long)b * lg] = rpiv;
   for (int q = 0; q < k && q < d.y; ++q) {
     const V* L = val + ((long)(d.z + step * q) * b + a) * b;
     for (int c = 0; c < b; ++c) o[(long)(b + 1 + q * b + c) * lg] = L[c];
@@ -195,13 +213,30 @@ __device__ __forceinline__ void run_level(const RunView<V>& R, int l, const RunR
       }
     }
   } else {
-    if (kFused) acc = pivot_quotient(acc, piv, w.rpiv);
+    bool scaled = true;
+    if constexpr (kFused) {
+      scaled = finite_hi(w.rpiv);
+      if (scaled) {
+        const V q = acc * w.rpiv;
+        acc = fma_rn(fma_rn(-q, piv, acc), w.rpiv, q);
+      }
+    }
+    if (kFused && __any_sync(0xffffffffu, on && live && !scaled)) {
+      // a row left unscaled (k_run_pack) takes the launch-per-level kernel's operations
 #pragma unroll
-    for (int c = B - 1; c >= 0; --c) {
-      if (!T && !kFused && a == c) acc = pivot_quotient(acc, piv, w.rpiv);
-      if (c > 0) {
+      for (int c = B - 1; c >= 0; --c) {
+        if (a == c && !scaled) acc = acc / piv;
         const V vc = __shfl_sync(0xffffffffu, acc, c, LG);
-        if (live && a < c) acc = msub<kFused>(acc, w.D[c], vc);
+        if (live && a < c) acc = scaled ? msub<kFused>(acc, w.D[c], vc) : acc - w.D[c] * vc;
+      }
+    } else {
+#pragma unroll
+      for (int c = B - 1; c >= 0; --c) {
+        if (!T && !kFused && a == c) acc = pivot_quotient(acc, piv, w.rpiv);
+        if (c > 0) {
+          const V vc = __shfl_sync(0xffffffffu, acc, c, LG);
+          if (live && a < c) acc = msub<kFused>(acc, w.D[c], vc);
+        }
       }
     }
   }
