@@ -1334,6 +1334,7 @@ struct FvIlu0 {
   void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
   int row_cap = 0;        // most blocks in a row
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
+  bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
   void* tval = nullptr;   // (b > 1) the factor's blocks transposed, in the transpose's order
   unsigned long long* zero_flag = nullptr;
@@ -1881,6 +1882,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
 
 extern "C" int fv_ilu0_destroy(FvIlu0* f) {
   if (!f) return FV_OK;
+  if (f->open) cudaStreamSynchronize(f->side);
   if (f->side) cudaStreamDestroy(f->side);
   if (f->side_event) cudaEventDestroy(f->side_event);
   cudaFree(f->ptr);
@@ -2002,6 +2004,12 @@ int factor_start(FvIlu0* f, const void* values, int values_f64, cudaStream_t s) 
     FV_CUDA_TRY(cudaMemcpyAsync(f->val, values, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
   return ilu_factor_start<float>(f, s);
 }
+
+// A factorisation started and not finished runs on its own stream: nothing else may use the factor.
+bool refuse_open(const FvIlu0* f, const char* what) {
+  if (f->open) fv_set_error("%s: fv_ilu0_factor_finish has to follow fv_ilu0_factor_start first", what);
+  return f->open;
+}
 }  // namespace
 
 extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream) {
@@ -2009,6 +2017,7 @@ extern "C" int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, voi
     fv_set_error("fv_ilu0_factor: bad arguments");
     return FV_ERR_ARG;
   }
+  if (refuse_open(f, "fv_ilu0_factor")) return FV_ERR_ARG;
   const int rc = factor_start(f, values, values_f64, (cudaStream_t)stream);
   return rc == FV_OK ? ilu_factor_finish(f, (cudaStream_t)stream) : rc;
 }
@@ -2019,6 +2028,7 @@ extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f6
     fv_set_error("fv_ilu0_factor_start: bad arguments");
     return FV_ERR_ARG;
   }
+  if (refuse_open(f, "fv_ilu0_factor_start")) return FV_ERR_ARG;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   FV_CUDA_TRY(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) {
@@ -2036,14 +2046,18 @@ extern "C" int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f6
   }
   FV_CUDA_TRY(cudaEventRecord(f->side_event, (cudaStream_t)stream));
   FV_CUDA_TRY(cudaStreamWaitEvent(f->side, f->side_event, 0));
-  return factor_start(f, values, values_f64, f->side);
+  const int rc = factor_start(f, values, values_f64, f->side);
+  f->open = rc == FV_OK;
+  if (rc != FV_OK) cudaStreamSynchronize(f->side);  // what was queued reads the caller's values
+  return rc;
 }
 
 extern "C" int fv_ilu0_factor_finish(FvIlu0* f, void* stream) {
-  if (!f || !f->side) {
+  if (!f || !f->open) {
     fv_set_error("fv_ilu0_factor_finish: no factorisation was started");
     return FV_ERR_ARG;
   }
+  f->open = false;
   FV_CUDA_TRY(cudaEventRecord(f->side_event, f->side));
   FV_CUDA_TRY(cudaStreamWaitEvent((cudaStream_t)stream, f->side_event, 0));
   return ilu_factor_finish(f, f->side);
@@ -2054,6 +2068,7 @@ extern "C" int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, v
     fv_set_error("fv_ilu0_apply: bad arguments");
     return FV_ERR_ARG;
   }
+  if (refuse_open(f, "fv_ilu0_apply")) return FV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (f->precision == 64) return ilu_apply<double>(f, (const double*)r, (double*)x, transpose, s);
   return ilu_apply<float>(f, (const float*)r, (float*)x, transpose, s);
@@ -2064,6 +2079,7 @@ extern "C" int fv_ilu0_factor_values(const FvIlu0* f, void* out, void* stream) {
     fv_set_error("fv_ilu0_factor_values: bad arguments");
     return FV_ERR_ARG;
   }
+  if (refuse_open(f, "fv_ilu0_factor_values")) return FV_ERR_ARG;
   size_t vs = f->precision == 64 ? sizeof(double) : sizeof(float);
   FV_CUDA_TRY(cudaMemcpyAsync(out, f->val, vs * (size_t)f->nnzb * f->b * f->b,
                               cudaMemcpyDeviceToDevice, (cudaStream_t)stream));

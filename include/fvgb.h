@@ -363,8 +363,10 @@ int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvIlu0** out);
 int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream);
 /* Its two halves, to factor several matrices side by side: start enqueues the factorization on a
  * stream of the factor's own (of higher priority if `urgent`; fixed by the first call) behind what
- * `stream` holds by then; finish waits for it, also on `stream`, and reports a zero pivot.  `values`
- * stay untouched in between.  Not under stream capture. */
+ * `stream` holds by then; finish waits for it, also on `stream`, and reports a zero pivot.  In between
+ * `values` stay untouched, and the factor's other calls but clone and destroy, which waits, are refused
+ * (FV_ERR_ARG).  A start that fails has waited for what it queued and needs no finish.  Not under stream
+ * capture. */
 int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, int urgent, void* stream);
 int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
 /* x = (LU)^-1 r, or (LU)^-T r when transpose != 0.  Device vectors of `precision`.  On a stream
