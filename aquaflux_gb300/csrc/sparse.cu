@@ -1333,6 +1333,7 @@ struct FvIlu0 {
   void* val = nullptr;
   void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
   int row_cap = 0;        // most blocks in a row
+  std::vector<int> lv_cap;  // ... of each forward level
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
   bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
@@ -1508,13 +1509,16 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
     if (cnt == 0) continue;
     const bool early = after && (sizeof(V) == 4 || cnt <= kEarly64);
     after = false;
-    const size_t wb = factor_warp_bytes<V>(f->row_cap, f->b * f->b);
-    if (f->b == 1 || wb > kFactorSmem) {  // scalar, or hundreds of blocks in a row
+    if (f->b == 1) {
       k_ilu_factor_level<V><<<fv_blocks(cnt, 128), 128, 0, s>>>(F, f->rows_fwd + f->lv_fwd[l], cnt,
                                                                 f->zero_flag);
       continue;
     }
-    if (cnt >= (sizeof(V) == 4 ? kFactorWide : kFactorWide64(f->b))) {
+    // a level with a row of hundreds of blocks takes lane groups too, which hold no row, and keeps the
+    // other levels to itself (96 x 96 grid, fp64: b = 6 3.1 ms, 4.1 with the first cell coupled to 400
+    // more and 34.9 with every level at a thread a row then; b = 8 4.8, 6.5, 87)
+    const size_t wb = factor_warp_bytes<V>(f->lv_cap[l], f->b * f->b);
+    if (wb > kFactorSmem || cnt >= (sizeof(V) == 4 ? kFactorWide : kFactorWide64(f->b))) {
       with_block_size(f->b, [&](auto B) {
         k_ilu_factor_lgb<V, B()><<<fv_blocks((long)cnt * FV_LG, 128), 128, 0, s>>>(
             F, f->rows_fwd + f->lv_fwd[l], cnt, (V*)f->rp, f->zero_flag);
@@ -1527,7 +1531,7 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
       auto kern = k_ilu_factor_w<V, B()>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactorSmem);
       launch_level(kern, fv_blocks(cnt, warps), s, early, 32 * warps, warps * wb, F,
-                   (const int*)f->rows_fwd + f->lv_fwd[l], cnt, f->row_cap, (V*)f->rp,
+                   (const int*)f->rows_fwd + f->lv_fwd[l], cnt, f->lv_cap[l], (V*)f->rp,
                    f->zero_flag);
     });
     after = sizeof(V) == 4 || cnt <= kEarly64;
@@ -1849,6 +1853,10 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   if (upload(rows, &f->rows_fwd, s)) return FV_ERR_CUDA;
   const std::vector<int> rows_fwd(rows);
   const size_t nf = f->lv_fwd.size();
+  f->lv_cap.assign(nf - 1, 0);
+  for (size_t l = 0; l + 1 < nf; ++l)
+    for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k)
+      f->lv_cap[l] = std::max(f->lv_cap[l], indptr[rows[k] + 1] - indptr[rows[k]]);
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
     for (int q = diag[i] + 1; q < indptr[i + 1]; ++q) use(indices[q]);
@@ -1936,6 +1944,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->nnzb = src->nnzb;
   f->precision = precision;
   f->row_cap = src->row_cap;
+  f->lv_cap = src->lv_cap;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;
