@@ -406,8 +406,8 @@ __device__ __forceinline__ unsigned lg_mask() { return 0xffu << ((threadIdx.x & 
 // block), with a compile-time block size: the row's lower block, the pivot row's diagonal block and
 // each upper block it updates with are held in registers (vector loads), the diagonal block's pivot
 // rows are shuffled from the lane that owns them.  Every entry sees the scalar elimination of
-// k_ilu_factor_level in the same order, so the factors are bitwise the same.  For the widest levels
-// (kFactorWide), where rows enough are in flight and a fourth of a warp per row issues less.
+// k_ilu_factor_level in the same order, so the factors are bitwise the same.  For the wider levels
+// (factor_wide), where rows enough are in flight and a fourth of a warp per row issues less.
 template <class V, int B>
 __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
                                  V* rp, unsigned long long* zero_flag) {
@@ -514,7 +514,7 @@ __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
       D[(long)a * B + c] = Drow[c];
       if (c == a) piv = Drow[c];
     }
-    rp[(long)i * B + a] = V(1) / piv;
+    if (rp) rp[(long)i * B + a] = V(1) / piv;  // (a level by warps follows)
   }
 }
 
@@ -549,9 +549,17 @@ __device__ __forceinline__ double quotient(double x, double piv, double rpiv) {
 }
 __device__ __forceinline__ float quotient(float x, float piv, float) { return x / piv; }
 
-// Levels of at least this many rows take 8 lanes a row (fp32, b = 6: 131,072 rows of 6 lower blocks
-// 187 us, 490 us with a warp a row; 5,900 rows of 8-15 lower blocks 120 us, 45 us with a warp).
-constexpr int kFactorWide = 65536;
+// Levels of at least this many rows take 8 lanes a row, whose time is a chain along a row's lower
+// blocks while the lanes last; a warp a row shortens the chain and takes four times the lanes, so the
+// line lies higher the longer the rows (`lower`: most lower blocks of a row in the level).  fp32, us a
+// factor of four level sets, lane groups / warps, by lower blocks and rows:
+//   b = 6   3:  5,000  98 /  99   6:  5,000 142 / 129,  8,191 162 / 187   16:  8,191 448 / 411, 12,000 490 / 562
+//   b = 4   3:  5,000  78 /  81   6:  5,000 112 / 113,  8,191 116 / 125   16: 12,000 345 / 347
+//   b = 2   3:  3,000  63 /  65   6:  8,192  97 / 100                     16: 12,000 270 / 255
+// and at 65,535 rows of 6 lower blocks 622 / 1,171, 342 / 737, 184 / 484.
+constexpr int factor_wide(int b, int lower) {
+  return b <= 4 ? 512 * lower + 2048 : 256 * lower + 3072;
+}
 // fp64 issue is four times scarcer for a warp a row than for four rows a warp, so there the line is
 // where the warps' rows fill the SMs' fp64 units; with a lane an entry (b <= 4) it lies higher
 // (3D 48^3, 142 level sets of up to 1,728 rows: b = 6 lane groups 6.55 ms, warps 5.9 ms, warps below
@@ -1333,7 +1341,7 @@ struct FvIlu0 {
   void* val = nullptr;
   void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
   int row_cap = 0;        // most blocks in a row
-  std::vector<int> lv_cap;  // ... of each forward level
+  std::vector<int> lv_cap, lv_low;  // ... of each forward level, and most lower blocks
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
   bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
@@ -1503,6 +1511,14 @@ void launch_level(K kern, int grid, cudaStream_t s, bool after, int threads, siz
 template <class V>
 void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   IluView<V> F = view<V>(f);
+  const int bb = f->b * f->b;
+  auto lane_groups = [&](size_t l) {
+    const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
+    return factor_warp_bytes<V>(f->lv_cap[l], bb) > kFactorSmem ||
+           cnt >= (sizeof(V) == 4 ? factor_wide(f->b, f->lv_low[l]) : kFactorWide64(f->b));
+  };
+  bool warps = false;  // a level takes warps, which read the pivots' reciprocals
+  for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) warps = warps || !lane_groups(l);
   bool after = false;  // the launch before on `s` lets this one start early
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) {
     const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
@@ -1517,14 +1533,14 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
     // a level with a row of hundreds of blocks takes lane groups too, which hold no row, and keeps the
     // other levels to itself (96 x 96 grid, fp64: b = 6 3.1 ms, 4.1 with the first cell coupled to 400
     // more and 34.9 with every level at a thread a row then; b = 8 4.8, 6.5, 87)
-    const size_t wb = factor_warp_bytes<V>(f->lv_cap[l], f->b * f->b);
-    if (wb > kFactorSmem || cnt >= (sizeof(V) == 4 ? kFactorWide : kFactorWide64(f->b))) {
+    if (lane_groups(l)) {
       with_block_size(f->b, [&](auto B) {
         k_ilu_factor_lgb<V, B()><<<fv_blocks((long)cnt * FV_LG, 128), 128, 0, s>>>(
-            F, f->rows_fwd + f->lv_fwd[l], cnt, (V*)f->rp, f->zero_flag);
+            F, f->rows_fwd + f->lv_fwd[l], cnt, warps ? (V*)f->rp : nullptr, f->zero_flag);
       });
       continue;
     }
+    const size_t wb = factor_warp_bytes<V>(f->lv_cap[l], bb);
     // a level that leaves SMs idle: a warp per block, so that no two share an SM's fp64 issue
     const int warps = cnt <= 4 * 152 || 4 * wb > kFactorSmem ? 1 : 4;
     with_block_size(f->b, [&](auto B) {
@@ -1854,9 +1870,13 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   const std::vector<int> rows_fwd(rows);
   const size_t nf = f->lv_fwd.size();
   f->lv_cap.assign(nf - 1, 0);
+  f->lv_low.assign(nf - 1, 0);
   for (size_t l = 0; l + 1 < nf; ++l)
-    for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k)
-      f->lv_cap[l] = std::max(f->lv_cap[l], indptr[rows[k] + 1] - indptr[rows[k]]);
+    for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k) {
+      const int i = rows[k];
+      f->lv_cap[l] = std::max(f->lv_cap[l], indptr[i + 1] - indptr[i]);
+      f->lv_low[l] = std::max(f->lv_low[l], diag[i] - indptr[i]);
+    }
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
     for (int q = diag[i] + 1; q < indptr[i + 1]; ++q) use(indices[q]);
@@ -1945,6 +1965,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->precision = precision;
   f->row_cap = src->row_cap;
   f->lv_cap = src->lv_cap;
+  f->lv_low = src->lv_low;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;

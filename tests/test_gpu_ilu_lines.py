@@ -41,6 +41,25 @@ def _factor(a, b, precision, v):
                          precision=precision)
 
 
+def _layered(width, layers, links):
+    """`layers` level sets of `width` rows, each row coupled to `links` rows of the one before."""
+    n, off = width * layers, np.arange(links) * 7
+    i = np.repeat(np.arange(width, n), links)
+    j = (i // width - 1) * width + (i % width + np.tile(off, n - width)) % width
+    a = sp.coo_matrix((np.ones(2 * i.size + n), (np.r_[i, j, np.arange(n)], np.r_[j, i, np.arange(n)])),
+                      (n, n)).tocsr()
+    a.sum_duplicates()
+    a.sort_indices()
+    return a
+
+
+def _copies(a, k):
+    """`k` copies of the pattern that do not couple: level sets k times as wide."""
+    c = sp.block_diag([a] * k, format="csr")
+    c.sort_indices()
+    return c
+
+
 @pytest.mark.parametrize("b,precision", [(6, 64), (8, 64), (8, 32)])
 def test_one_long_row_costs_the_factor_its_own_level_only(b, precision):
     """A 96 x 96 grid, and the same with the first cell coupled to 400 others (a row of more blocks than
@@ -57,3 +76,31 @@ def test_one_long_row_costs_the_factor_its_own_level_only(b, precision):
         f = _factor(a, b, precision, v)
         times.append(_time(lambda: f.refactor(v)))
     assert times[1] <= 2.0 * times[0], times
+
+
+# fp32 b, links: what the line between a warp and 8 lanes a row of the factor sees
+@pytest.mark.parametrize("b,links", [(2, 3), (3, 6), (4, 6), (4, 12), (5, 6), (6, 3), (6, 6), (6, 12), (8, 6)])
+def test_a_factor_of_narrower_levels_is_not_the_slower_one(b, links):
+    """fp32, three level sets from 2,000 to 70,000 rows: no width takes more than 1.2 times what a
+    larger one takes."""
+    times = []
+    for width in (2000, 4000, 6000, 9000, 14000, 22000, 40000, 65000, 70000):
+        a = _layered(width, 3, links)
+        v = _blocks(a, b, torch.float32)
+        f = _factor(a, b, 32, v)
+        times.append(_time(lambda: f.refactor(v)))
+    for k, t in enumerate(times):
+        assert t <= 1.2 * min(times[k:]), (k, times)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("b,links", [(2, 3), (3, 6), (4, 16), (5, 1), (6, 3), (6, 12), (7, 6), (8, 3)])
+def test_a_factor_is_the_same_at_every_width(b, links, precision):
+    """Copies side by side, so that a row's level and with it the kernel is another one: bitwise."""
+    dtype = torch.float64 if precision == 64 else torch.float32
+    a = _layered(500, 3, links)
+    v = _blocks(a, b, dtype, seed=b)
+    want = _factor(a, b, precision, v).factor_values()
+    for k in (7, 12, 24):  # 3,500, 6,000 and 12,000 rows a level set
+        got = _factor(_copies(a, k), b, precision, v.repeat(k)).factor_values()
+        assert torch.equal(got, want.repeat(k)), k
