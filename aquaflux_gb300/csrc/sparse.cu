@@ -551,8 +551,9 @@ __device__ __forceinline__ float quotient(float x, float piv, float) { return x 
 
 // Levels of at least this many rows take 8 lanes a row, whose time is a chain along a row's lower
 // blocks while the lanes last; a warp a row shortens the chain and takes four times the lanes, so the
-// line lies higher the longer the rows (`lower`: most lower blocks of a row in the level).  fp32, us a
-// factor of four level sets, lane groups / warps, by lower blocks and rows:
+// line lies higher the longer the rows (`lower`: most lower blocks of a row in the level), and in a level
+// of uneven rows, whose longest is the lanes' chain and whose mean the warps' work, by their ratio.
+// fp32, us a factor of four level sets, lane groups / warps, by lower blocks and rows:
 //   b = 6   3:  5,000  98 /  99   6:  5,000 142 / 129,  8,191 162 / 187   16:  8,191 448 / 411, 12,000 490 / 562
 //   b = 4   3:  5,000  78 /  81   6:  5,000 112 / 113,  8,191 116 / 125   16: 12,000 345 / 347
 //   b = 2   3:  3,000  63 /  65   6:  8,192  97 / 100                     16: 12,000 270 / 255
@@ -1342,6 +1343,7 @@ struct FvIlu0 {
   void* rp = nullptr;     // (n * b) reciprocals of the factor's pivots
   int row_cap = 0;        // most blocks in a row
   std::vector<int> lv_cap, lv_low;  // ... of each forward level, and most lower blocks
+  std::vector<long> lv_sum;         // ... and its lower blocks together
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
   bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
@@ -1513,9 +1515,10 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   IluView<V> F = view<V>(f);
   const int bb = f->b * f->b;
   auto lane_groups = [&](size_t l) {
-    const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l];
-    return factor_warp_bytes<V>(f->lv_cap[l], bb) > kFactorSmem ||
-           cnt >= (sizeof(V) == 4 ? factor_wide(f->b, f->lv_low[l]) : kFactorWide64(f->b));
+    const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l], low = f->lv_low[l];
+    if (factor_warp_bytes<V>(f->lv_cap[l], bb) > kFactorSmem) return true;
+    if (sizeof(V) == 8) return cnt >= kFactorWide64(f->b);
+    return low ? f->lv_sum[l] >= (long)factor_wide(f->b, low) * low : cnt >= factor_wide(f->b, 0);
   };
   bool warps = false;  // a level takes warps, which read the pivots' reciprocals
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) warps = warps || !lane_groups(l);
@@ -1871,11 +1874,13 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   const size_t nf = f->lv_fwd.size();
   f->lv_cap.assign(nf - 1, 0);
   f->lv_low.assign(nf - 1, 0);
+  f->lv_sum.assign(nf - 1, 0);
   for (size_t l = 0; l + 1 < nf; ++l)
     for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k) {
       const int i = rows[k];
       f->lv_cap[l] = std::max(f->lv_cap[l], indptr[i + 1] - indptr[i]);
       f->lv_low[l] = std::max(f->lv_low[l], diag[i] - indptr[i]);
+      f->lv_sum[l] += diag[i] - indptr[i];
     }
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
@@ -1966,6 +1971,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->row_cap = src->row_cap;
   f->lv_cap = src->lv_cap;
   f->lv_low = src->lv_low;
+  f->lv_sum = src->lv_sum;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;
