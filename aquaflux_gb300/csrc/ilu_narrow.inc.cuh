@@ -33,6 +33,16 @@ __host__ __device__ constexpr bool run_block_size(int b, size_t vs) {
 }
 // Rows a level may hold: one per lane group of the block.
 inline int run_capacity(int b) { return kRunThreads / run_lanes(b); }
+// ... and of the fp64 transposed solve, `most` blocks in a row: its operations, twice the fused forward
+// solve's, bind one block where a launch per level spreads them over the SMs.  us a solve of 60 level
+// sets, one launch / a launch per level, by rows and blocks a row (the forward solve in one launch is
+// the faster one throughout but for 4 blocks of b = 4 in 96 rows, 514 / 475):
+//   b = 4   48 rows  4: 457 / 473, 8: 696 / 658, 20: 1,313 / 1,164   96 rows  1: 373 / 372, 2: 509 / 375, 4: 883 / 475
+//   b = 3   56 rows  4: 370 / 415, 8: 611 / 570, 20: 1,169 / 989     96 rows  2: 381 / 332, 4: 598 / 415
+//   b = 2   64 rows  4: 292 / 356, 8: 488 / 487, 20: 971 / 871       96 rows  2: 257 / 296, 4: 398 / 361, 8: 627 / 498
+inline int run_widest_t64(int b, int most) {
+  return 48 - 2 * b + (450 - 62 * b) / (b * std::max(most, 1));
+}
 // Entries of a record per lane: the diagonal block's row, the pivot's reciprocal, `k` blocks' rows.
 __host__ __device__ constexpr int run_entries(int b, int k) { return b + 1 + k * b; }
 

@@ -1364,6 +1364,7 @@ struct FvIlu0 {
     void* rec = nullptr;    // records, renewed by each factorisation
     int nlev = 0, nlev_fwd = 0, widest = 0;
     int k = 0;              // blocks in a record, at most
+    int most = 0;           // off-diagonal blocks of a row in a sweep, at most
   } run[2];
   bool fuse_fb = false;  // the last forward level's rows are the first backward level's (fused)
   cudaGraphExec_t apply_exec[2] = {nullptr, nullptr};  // forward / transposed solve
@@ -1446,6 +1447,7 @@ int build_run(FvIlu0* f, int t, const std::vector<int>& fwd, const std::vector<i
       rows.push_back(d);
       cols.push_back(make_int4(c[0], c[1], c[2], c[3]));
       run.k = std::max(run.k, std::min(d.y, kRunBlocks));
+      run.most = std::max(run.most, d.y);
     }
   std::vector<int> bounds(lv_fwd);
   for (int l = 1; l <= nb; ++l) bounds.push_back(f->n + lv_bwd[l]);
@@ -1466,6 +1468,7 @@ int pack_run(FvIlu0* f, int t, cudaStream_t s) {
   // fp32 rows of more blocks than the records hold go by k_ilu_sweep_w, which has all of them in
   // place (212 coarse rows of 20 to 40 blocks: 22 us a solve, 40 us by k_ilu_run)
   if (!run.row || !run_block_size(f->b, sizeof(V)) ||
+      (sizeof(V) == 8 && t && run.widest > run_widest_t64(f->b, run.most)) ||
       run_smem_bytes(f->n, f->b, run.nlev, sizeof(V)) > kRunSmem ||
       (sizeof(V) == 4 && f->row_cap > 2 * kRunBlocks + 1))
     return FV_OK;

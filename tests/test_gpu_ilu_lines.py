@@ -41,9 +41,10 @@ def _factor(a, b, precision, v):
                          precision=precision)
 
 
-def _layered(width, layers, links):
-    """`layers` level sets of `width` rows, each row coupled to `links` rows of the one before."""
-    n, off = width * layers, np.arange(links) * 7
+def _layered(width, layers, links, step=7):
+    """`layers` level sets of `width` rows, each row coupled to `links` rows of the one before, `step`
+    rows apart (a `step` that divides the width repeats some)."""
+    n, off = width * layers, np.arange(links) * step
     i = np.repeat(np.arange(width, n), links)
     j = (i // width - 1) * width + (i % width + np.tile(off, n - width)) % width
     a = sp.coo_matrix((np.ones(2 * i.size + n), (np.r_[i, j, np.arange(n)], np.r_[j, i, np.arange(n)])),
@@ -104,3 +105,36 @@ def test_a_factor_is_the_same_at_every_width(b, links, precision):
     for k in (7, 12, 24):  # 3,500, 6,000 and 12,000 rows a level set
         got = _factor(_copies(a, k), b, precision, v.repeat(k)).factor_values()
         assert torch.equal(got, want.repeat(k)), k
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("b,links", [(2, 1), (2, 8), (3, 2), (3, 4), (3, 20), (4, 1), (4, 2), (4, 8), (4, 20)])
+def test_a_solve_of_narrow_levels_is_not_the_slower_one(b, links, transpose):
+    """fp64, 60 level sets of 16 to 97 rows, in one launch or one a level: no width takes more than 1.15
+    times what a larger one takes."""
+    times = []
+    for width in (16, 32, 40, 48, 56, 64, 80, 96, 97):
+        a = _layered(width, 60, links, 1)
+        f = _factor(a, b, 64, _blocks(a, b, torch.float64))
+        r = torch.rand(width * 60 * b, device="cuda", dtype=torch.float64)
+        x = torch.empty_like(r)
+        times.append(_time(lambda: f.solve(r, transpose=transpose, out=x)))
+    for k, t in enumerate(times):
+        assert t <= 1.15 * min(times[k:]), (k, times)
+
+
+@pytest.mark.parametrize("b,links", [(2, 1), (2, 8), (3, 2), (3, 8), (4, 2), (4, 20)])
+def test_a_narrow_solve_is_the_same_at_every_width(b, links):
+    """Copies side by side, fp64: level sets of 20 to 100 rows, in one launch or one a level.  The
+    transposed solve bitwise; the forward one to the rounding of its reordered sums (at most
+    links * b + b terms a row of well-conditioned blocks: 100 units in the last place)."""
+    a = _layered(20, 30, links, 1)
+    v = _blocks(a, b, torch.float64, seed=b)
+    r = torch.rand(600 * b, device="cuda", dtype=torch.float64) - 0.5
+    f = _factor(a, b, 64, v)
+    x, xt = f.solve(r), f.solve(r, transpose=True)
+    for k in (2, 3, 4, 5):
+        g = _factor(_copies(a, k), b, 64, v.repeat(k))
+        assert torch.equal(g.solve(r.repeat(k), transpose=True), xt.repeat(k)), k
+        d = float((g.solve(r.repeat(k)) - x.repeat(k)).abs().max())
+        assert d <= 100 * 2.3e-16 * float(x.abs().max()), (k, d)
