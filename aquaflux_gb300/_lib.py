@@ -86,6 +86,7 @@ SIGNATURES = {
     "fv_ilu0_factor": (c_int, [P, P, c_int, P]),
     "fv_ilu0_factor_start": (c_int, [P, P, c_int, c_int, P]),
     "fv_ilu0_factor_finish": (c_int, [P, P]),
+    "fv_ilu0_set_streamed": (c_int, [P, c_int]),
     "fv_ilu0_apply": (c_int, [P, P, P, c_int, P]),
     "fv_ilu0_factor_values": (c_int, [P, P, P]),
     "fv_dot_f64": (c_int, [c_long, P, P, P, P]),

@@ -33,15 +33,20 @@ __host__ __device__ constexpr bool run_block_size(int b, size_t vs) {
 }
 // Rows a level may hold: one per lane group of the block.
 inline int run_capacity(int b) { return kRunThreads / run_lanes(b); }
-// ... and of the fp64 transposed solve, `most` blocks in a row: its operations, twice the fused forward
-// solve's, bind one block where a launch per level spreads them over the SMs.  us a solve of 60 level
-// sets, one launch / a launch per level, by rows and blocks a row (the forward solve in one launch is
-// the faster one throughout but for 4 blocks of b = 4 in 96 rows, 514 / 475):
-//   b = 4   48 rows  4: 457 / 473, 8: 696 / 658, 20: 1,313 / 1,164   96 rows  1: 373 / 372, 2: 509 / 375, 4: 883 / 475
-//   b = 3   56 rows  4: 370 / 415, 8: 611 / 570, 20: 1,169 / 989     96 rows  2: 381 / 332, 4: 598 / 415
-//   b = 2   64 rows  4: 292 / 356, 8: 488 / 487, 20: 971 / 871       96 rows  2: 257 / 296, 4: 398 / 361, 8: 627 / 498
-inline int run_widest_t64(int b, int most) {
-  return 48 - 2 * b + (450 - 62 * b) / (b * std::max(most, 1));
+// ... and in fp64 the rows they may hold in the mean, `most` blocks in a row, for one block's fp64 units not
+// to take longer than a launch per level: soonest in the transposed solve, with twice the operations of
+// the fused forward one.  Time in one launch over that of a launch per level (60 level sets; the launches
+// take 0.34 ms for 2 blocks a row of b = 3, 0.62 for 8), by rows:
+//   transposed, b = 3   2 blocks  64: 0.80, 88: 1.03   4: 48: 0.92, 56: 1.03   8: 40: 0.99, 48: 1.07   20: 24: 1.08
+//               b = 4   2 blocks  64: 0.97, 72: 1.09   4: 40: 0.98, 48: 1.09   8: 32: 0.94, 40: 1.05   20: 24: 1.05
+//               b = 2   2 blocks  96: 0.90             4: 64: 0.96, 72: 1.03   8: 48: 0.92, 56: 1.05   20: 24: 1.03
+//   forward,    b = 4   2 blocks  96: 0.71             4: 80: 1.00, 88: 1.09   8: 80: 0.97, 88: 1.04   20: 88: 0.97
+//   and below 1 for b = 2 and 3 throughout
+// (in the mean: 90 x 90 cells, level sets of 1 to 90 rows, b = 3 615 us transposed, 991 by launches).
+inline int run_mean64(int b, int most, bool transposed) {
+  if (!transposed) return b == 4 && most >= 4 ? 80 : run_capacity(b);
+  constexpr int few[5] = {240, 240, 200, 152, 104};
+  return 16 + (most <= 4 ? few[most] : std::max(0, 120 - 5 * most)) / b;
 }
 // Entries of a record per lane: the diagonal block's row, the pivot's reciprocal, `k` blocks' rows.
 __host__ __device__ constexpr int run_entries(int b, int k) { return b + 1 + k * b; }

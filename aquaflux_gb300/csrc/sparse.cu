@@ -12,6 +12,7 @@
 // reproduce the sequential algorithm's dependencies exactly.  With b = 1 this is the reference's
 // scalar CSR ILU(0).
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <type_traits>
 #include <memory>
@@ -826,10 +827,18 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
   for (int k = lane; k < nb * BB; k += 32) row[k] = blk[k];
 }
 
+// How the lane groups of a level read their rows (launch_apply_levels chooses):
+//   kPlain   a launch after the other; the compiler's unrolling reads a few blocks ahead
+//   kEarly   the same, launched before the level before has ended
+//   kDeep    so too, two blocks at a time, the columns of eight by the group's lanes at once
+//   kStream  a launch after the other, one block at a time: the fewest registers, the most warps
+// Each asks the L2 cache for the row's first lines, or all of them (`ask` bytes), before its first read.
+enum Read { kPlain, kEarly, kDeep, kStream };
+__host__ __device__ constexpr bool early(int m) { return m == kEarly || m == kDeep; }
+
 // acc minus the products of `count` blocks (positions q0, q0 + STEP, ...) with their columns' entries
-// of x, in that order (and, STEP = -1, each block's entries from the last).  U > 1: U blocks are
-// read at a time, the columns of eight by the group's lanes at once.
-template <class V, int B, int STEP, int U>
+// of x, in that order (and, STEP = -1, each block's entries from the last).
+template <class V, int B, int STEP, int M>
 __device__ __forceinline__ V subtract_blocks(V acc, const V* val, const int* idx, const V* x, int q0,
                                              int count, int a, bool live, unsigned mask) {
   constexpr long BB = (long)B * B;
@@ -840,52 +849,60 @@ __device__ __forceinline__ V subtract_blocks(V acc, const V* val, const int* idx
       acc -= L[e] * xj[e];
     }
   };
-  if constexpr (U == 1) {
-    if (live)
-#pragma unroll 1
-      for (int k = 0; k < count; ++k) {
-        const int q = q0 + STEP * k;
-        V L[B], xj[B];
-        load_seg<B>(val + (long)q * BB + (long)a * B, L);
-        load_seg<B>(x + (long)idx[q] * B, xj);
-        block(L, xj);
-      }
-  } else {
+  auto one = [&](int q) {
+    V L[B], xj[B];
+    load_seg<B>(val + (long)q * BB + (long)a * B, L);
+    load_seg<B>(x + (long)idx[q] * B, xj);
+    block(L, xj);
+  };
+  if constexpr (M == kDeep) {
     for (int k0 = 0; k0 < count; k0 += FV_LG) {
       const int col = k0 + a < count ? idx[q0 + STEP * (k0 + a)] : 0;
-      for (int k = k0; k < count && k < k0 + FV_LG; k += U) {
-        V L[U][B], xj[U][B];
+      for (int k = k0; k < count && k < k0 + FV_LG; k += 2) {
+        V L[2][B], xj[2][B];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < 2; ++u)
           if (live && k + u < count)
             load_seg<B>(val + (long)(q0 + STEP * (k + u)) * BB + (long)a * B, L[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
+        for (int u = 0; u < 2; ++u) {
           const int j = __shfl_sync(mask, col, k - k0 + u, FV_LG);
           if (live && k + u < count) load_seg<B>(x + (long)j * B, xj[u]);
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < 2; ++u)
           if (live && k + u < count) block(L[u], xj[u]);
       }
+    }
+  } else if constexpr (M == kStream) {
+    if (live)
+#pragma unroll 1
+      for (int k = 0; k < count; ++k) one(q0 + STEP * k);
+  } else {
+    if (live) {
+      if (STEP > 0)
+        for (int q = q0; q < q0 + count; ++q) one(q);
+      else
+        for (int q = q0; q > q0 - count; --q) one(q);
     }
   }
   return acc;
 }
 
 template <class V, int B>
-__device__ __forceinline__ void ask_blocks(const V* val, int q0, int count, int a) {
-  // lane a asks for the lines at a, a + 8, ... of the blocks' contiguous range
+__device__ __forceinline__ void ask_blocks(const V* val, int q0, int count, int a, int ask) {
+  // lane a asks for the lines at a, a + 8, ... of the blocks' contiguous range, of its first `ask` bytes
   const char* p = (const char*)(val + (long)q0 * B * B);
-  const long bytes = (long)count * B * B * (long)sizeof(V);
-  for (long o = 128L * a; o < bytes; o += 128L * FV_LG)
+  const long end = min((long)count * B * B * (long)sizeof(V), (long)ask);
+  for (long o = 128L * a; o < end; o += 128L * FV_LG)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
 }
 
 // Forward sweep of one level, a group of FV_LG lanes per block row (lane a = row a of the block).
-template <class V, int B, int U>
-__global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, const V* r, V* y) {
-  if (U > 1) next_level_may_start();
+template <class V, int B, int M>
+__global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, int ask, const V* r,
+                               V* y) {
+  if (early(M)) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -894,10 +911,10 @@ __global__ void k_ilu_lower_lg(IluView<V> F, const int* rows, int count, const V
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = F.ptr[i], di = F.diag[i];
-  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a);
-  if (U > 1) wait_level_before();
+  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a, ask);
+  if (early(M)) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
-  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
+  acc = subtract_blocks<V, B, 1, M>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
   if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
 #pragma unroll
@@ -944,9 +961,9 @@ __device__ __forceinline__ V upper_block_solve(V acc, const V (&D)[B], int a, bo
 }
 
 // Backward sweep of one level (U x = y).
-template <class V, int B, int U>
-__global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
-  if (U > 1) next_level_may_start();
+template <class V, int B, int M>
+__global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, int ask, V* x) {
+  if (early(M)) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -955,10 +972,10 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int di = F.diag[i], re = F.ptr[i + 1];
-  ask_blocks<V, B>(F.val, di, re - di, a);
-  if (U > 1) wait_level_before();
+  ask_blocks<V, B>(F.val, di, re - di, a, ask);
+  if (early(M)) wait_level_before();
   V acc = live ? x[(long)i * B + a] : V(0);
-  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, x, di + 1, re - di - 1, a, live, mask);
+  acc = subtract_blocks<V, B, 1, M>(acc, F.val, F.idx, x, di + 1, re - di - 1, a, live, mask);
   V D[B];
   if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
   acc = upper_block_solve<V, B>(acc, D, a, live, mask);
@@ -969,9 +986,10 @@ __global__ void k_ilu_upper_lg(IluView<V> F, const int* rows, int count, V* x) {
 // those rows own no upper blocks (the second colour of a two-colour order), a row's backward step
 // is the in-block upper solve of its own forward result, with the diagonal block already in
 // registers.  The same operations in the same order as the two separate sweeps.
-template <class V, int B, int U>
-__global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, const V* r, V* y) {
-  if (U > 1) next_level_may_start();
+template <class V, int B, int M>
+__global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, int ask, const V* r,
+                                     V* y) {
+  if (early(M)) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -980,10 +998,10 @@ __global__ void k_ilu_lower_upper_lg(IluView<V> F, const int* rows, int count, c
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = F.ptr[i], di = F.diag[i];
-  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a);
-  if (U > 1) wait_level_before();
+  ask_blocks<V, B>(F.val, q0, di - q0 + 1, a, ask);
+  if (early(M)) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
-  acc = subtract_blocks<V, B, 1, U>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
+  acc = subtract_blocks<V, B, 1, M>(acc, F.val, F.idx, y, q0, di - q0, a, live, mask);
   V D[B];
   if (live) load_seg<B>(F.val + (long)di * BB + (long)a * B, D);
 #pragma unroll
@@ -1029,10 +1047,11 @@ __device__ __forceinline__ V lower_t_block_solve(V acc, const V (&Dc)[B], int a,
 // blocks (j, i) of U, j < i (positions tptr[i] .. tdiag[i] of the transpose, ascending j), row a
 // of each transposed block (column a of the block of U) for lane a, then the in-block lower solve
 // with D^T -- the operations and their order of the reference's transposed solve.
-template <class V, int B, int U>
+template <class V, int B, int M>
 __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx, const int* tdiag,
-                                 const V* tval, const int* rows, int count, const V* r, V* z) {
-  if (U > 1) next_level_may_start();
+                                 const V* tval, const int* rows, int count, int ask, const V* r,
+                                 V* z) {
+  if (early(M)) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -1041,10 +1060,10 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int q0 = tptr[i], di = tdiag[i];
-  ask_blocks<V, B>(tval, q0, di - q0 + 1, a);
-  if (U > 1) wait_level_before();
+  ask_blocks<V, B>(tval, q0, di - q0 + 1, a, ask);
+  if (early(M)) wait_level_before();
   V acc = live ? r[(long)i * B + a] : V(0);
-  acc = subtract_blocks<V, B, 1, U>(acc, tval, tidx, z, q0, di - q0, a, live, mask);
+  acc = subtract_blocks<V, B, 1, M>(acc, tval, tidx, z, q0, di - q0, a, live, mask);
   V Dc[B];  // Dc[c] = D(c, a): row a of D^T
   if (live) load_seg<B>(tval + (long)di * BB + (long)a * B, Dc);
   else
@@ -1057,10 +1076,10 @@ __global__ void k_ilu_upper_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // Backward sweep of one level of the transposed solve, L^T x = z (unit diagonal): the blocks
 // (k, i) of L, k > i (positions tptr[i + 1] - 1 down to tdiag[i] + 1), then the in-block unit
 // upper solve.
-template <class V, int B, int U>
+template <class V, int B, int M>
 __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx, const int* tdiag,
-                                 const V* tval, const int* rows, int count, V* x) {
-  if (U > 1) next_level_may_start();
+                                 const V* tval, const int* rows, int count, int ask, V* x) {
+  if (early(M)) next_level_may_start();
   const int gid = (blockIdx.x * blockDim.x + threadIdx.x) / FV_LG;
   const int a = threadIdx.x & (FV_LG - 1);
   if (gid >= count) return;
@@ -1069,10 +1088,10 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   const bool live = a < B;
   constexpr long BB = (long)B * B;
   const int di = tdiag[i], last = tptr[i + 1] - 1;
-  ask_blocks<V, B>(tval, di, last - di + 1, a);
-  if (U > 1) wait_level_before();
+  ask_blocks<V, B>(tval, di, last - di + 1, a, ask);
+  if (early(M)) wait_level_before();
   V acc = live ? x[(long)i * B + a] : V(0);
-  acc = subtract_blocks<V, B, -1, U>(acc, tval, tidx, x, last, last - di, a, live, mask);
+  acc = subtract_blocks<V, B, -1, M>(acc, tval, tidx, x, last, last - di, a, live, mask);
   V Dc[B];
   if (live) load_seg<B>(tval + (long)di * BB + (long)a * B, Dc);
   else
@@ -1086,18 +1105,23 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
   if (live) x[(long)i * B + a] = acc;
 }
 
-// ---- fp32 levels of fewer than kDeepRows rows: a warp per block row, its blocks in shared memory.
-// Such a level's time is its longest row's chain, and a coarse Galerkin row holds 20 to 40 blocks:
-// with 8 lanes reading four blocks at a time from L2 the chain paid a memory latency or two every
-// four blocks (10 level sets of 720 rows: 6 us each).  Here a row's columns, blocks, diagonal block
-// and, going forward, right-hand side are in place before the level before is waited for; all its x
-// entries then come in one round of loads, a block's by a lane, and what is left is the subtractions
-// one after the other: 2 us a level set.  fp32 V-cycle of the 128 x 96 x 96 channel 2083 -> 1868 us,
-// of 40^3 cells 607 -> 345; from kDeepRows on, where the lanes and not a row's chain run out, the
-// lane groups are faster (levels of 26,000 rows: 1943 us with a warp a row).
+// ---- fp32 levels of few rows: a warp per block row, its blocks in shared memory.
+// Such a level's time is its longest row's chain, and a coarse Galerkin row holds 15 to 40 blocks:
+// with 8 lanes a row the chain paid a memory latency or two every few blocks (10 level sets of 720
+// rows: 6 us each).  Here a row's columns, blocks, diagonal block and, going forward, right-hand side
+// are in place before the level before is waited for; all its x entries then come in one round of
+// loads, a block's by a lane, and what is left is the subtractions one after the other: 2 us a level
+// set.  fp32 V-cycle of the 128 x 96 x 96 channel 2083 -> 1868 us, of 40^3 cells 607 -> 345.
+// The line (sweep_rows) lies where the lanes run out instead of a row's chain.  Blocks that come from
+// memory, as in a cycle over several hundred MB, hide that up to more rows: 64^3 cells 590 us a cycle,
+// 688 with lane groups from 3,072 rows on (b = 5 597 / 645, b = 4 420 / 471); but from L2 levels of
+// 4,000 rows gain 3 to 13 % (1,000 rows 13 to 28 %) and 8,191 lose 3 to 48 % to the lane groups.
 // The operations and their order are the lane-group kernels'.
 enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
-constexpr int kDeepRows = 8192;
+constexpr int sweep_rows(int b, bool streamed) {
+  if (b == 7 || b == 8) return 2048;  // 21 to 37 KB a block of four warps: few of them on an SM
+  return streamed ? 8192 : b == 5 ? 2048 : 3072;
+}
 
 constexpr int kSweepBlocks = 32;  // blocks in shared memory at a time: a column a lane
 template <int B>
@@ -1356,6 +1380,7 @@ struct FvIlu0 {
   int* rows_tbwd = nullptr;  // L^T order
   std::vector<int> lv_fwd, lv_bwd, lv_tfwd, lv_tbwd;
   void* work = nullptr;                      // (n * b) vector the captured sweeps run on
+  bool streamed = false;  // the blocks come from memory at each solve
   // (b > 1) narrow level sets: the forward / transposed solve as one launch (ilu_narrow.inc.cuh)
   struct Run {
     int4* row = nullptr;    // 2n rows in level order, forward sweep then backward
@@ -1402,6 +1427,11 @@ void levels(int n, bool ascending, DepFn deps, std::vector<int>* rows, std::vect
   rows->assign(n, 0);
   std::vector<int> fill(bounds->begin(), bounds->end() - 1);
   for (int i = 0; i < n; ++i) (*rows)[fill[lev[i]]++] = i;
+}
+
+// A factor larger than the L2 cache (126 MB).
+inline bool beyond_l2(long nnzb, int b, int precision) {
+  return nnzb * b * b * (precision / 8) >= 126000000;
 }
 
 template <class V>
@@ -1468,7 +1498,7 @@ int pack_run(FvIlu0* f, int t, cudaStream_t s) {
   // fp32 rows of more blocks than the records hold go by k_ilu_sweep_w, which has all of them in
   // place (212 coarse rows of 20 to 40 blocks: 22 us a solve, 40 us by k_ilu_run)
   if (!run.row || !run_block_size(f->b, sizeof(V)) ||
-      (sizeof(V) == 8 && t && run.widest > run_widest_t64(f->b, run.most)) ||
+      (sizeof(V) == 8 && 2L * f->n > (long)run_mean64(f->b, run.most, t != 0) * run.nlev) ||
       run_smem_bytes(f->n, f->b, run.nlev, sizeof(V)) > kRunSmem ||
       (sizeof(V) == 4 && f->row_cap > 2 * kRunBlocks + 1))
     return FV_OK;
@@ -1560,16 +1590,38 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   }
 }
 
-// The widest levels (590,000 rows: 120 us) are bound by bytes and want warps in flight: one block at
-// a time, a launch after the other (the registers of a deeper read made them 180-220 us), and all
-// lines of a row asked of the L2 cache first (125 -> 120 us, a 1.2M-row V-cycle 1870 -> 1844).  Below
-// kWideRows a row's chain of latencies is the level's time: blocks are read two at a time and the
-// next level is launched early (16 levels of 26,000 rows 176 -> 156 us); fp32 below kDeepRows takes
-// a warp a row.
-// fp64 levels of kDeep64 rows and more are bound by fp64 issue and read like the widest: a solve in
-// 3D with b = 6, 48^3 (levels of up to 1,728 rows) 2.34 -> 1.75 ms; 24^3 (432 rows) 671 us two
-// blocks at a time with an early launch, 686 one at a time.
-constexpr int kWideRows = 65536, kDeep64 = 512;
+// How a level's lane groups read, by rows and block size, and (streamed) whether the blocks come from
+// memory: a hierarchy's factors, or one larger than the L2 cache.
+// * A level of few rows is its rows' chain of latencies: the next one is launched early.  fp64 to 1,024
+//   rows (above, its blocks would be placed around a level that fp64 issue still binds: 6,000 rows 1.1 to
+//   1.4 times the time), fp32 to 32,768, odd block sizes, whose loads are scalar, to 8,192.
+//   kEarly / kPlain / the form with neither request nor early launch, 6 level sets, fp64 us: 512 rows, 14
+//   blocks, b = 3 92 / 99 / 99.5, b = 6 134 / 146 / 144; 97 rows, 2 blocks, b = 4 58 / 64 / 65.
+// * streamed: two blocks at a time and all of a row's lines asked for (V-cycle of 64^3 cells, fp64,
+//   b = 6, its small levels 3,240 -> 3,150 us; 80^3 fp32, levels of 14,000 rows 966 -> 943; but
+//   128 x 96 x 96, 30,000 rows 1,747 / 1,740, and from L2 4 to 28 % slower for b of 2, 3, 5 and 7).
+//   So, too, the transposed fp64 levels of few short rows of b = 2 and 3 (300 x 200 cells, b = 3, a
+//   transposed V-cycle 6,016 -> 5,830 us; 29 blocks a row, b = 3, 511 rows 97 us, kEarly 86).
+// * The cache is asked for a row's first KB, a line a lane; for all of a row where it is long in bytes and
+//   from memory or early (V-cycles, fp64, b = 6: 50^3 2,067 -> 2,024 us, 24^3 680 -> 661; late and from L2
+//   6,000 rows of 14 blocks 1 to 9 % slower).
+// * The widest are bound by bytes and want warps in flight (590,000 rows, b = 6: 120 us one block at a
+//   time, 180-220 with the registers of a deeper read; 500,000 rows, b = 4 0.78 of kPlain's time, b = 6
+//   0.92), but for the block sizes with scalar or 8-byte loads, which the compiler's unrolling serves
+//   better (b = 2, 16 blocks 71 / 83 us at 131,072 rows).
+inline int level_read(bool fp32, int b, int rows, int longest, bool streamed, bool transposed) {
+  const bool wide_loads = b % 2 == 0 && b > 2;
+  if (!fp32) {
+    if (rows < 512 && (wide_loads ? streamed : transposed && b <= 3 && longest <= 16))
+      return kDeep;
+    return rows <= 1024 ? kEarly : kPlain;
+  }
+  if (rows < 8192) return kEarly;
+  if (rows >= 65536) return wide_loads ? kStream : kPlain;
+  if (b % 2 != 0) return kPlain;
+  if (streamed && wide_loads && rows < 24576) return kDeep;
+  return rows < 32768 ? kEarly : wide_loads ? kStream : kPlain;
+}
 
 template <class V>
 void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_t s) {
@@ -1581,21 +1633,27 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
       const int cnt = lv[l + 1] - lv[l];
       if (!cnt) continue;
       one(l, order + lv[l], cnt);
-      after = cnt < kWideRows;
+      after = true;
     }
   };
-  // the lane-group kernels of a level, by block size and depth
+  // the lane-group kernels of a level, by block size and reading
   auto lane_groups = [&](int cnt, auto&& launch) {
     const int grid = fv_blocks((long)cnt * FV_LG, 128);
+    const int read = level_read(sizeof(V) == 4, f->b, cnt, f->row_cap, f->streamed, transpose != 0);
+    const int ask = read == kDeep || (sizeof(V) == 8 && (read == kEarly || f->streamed)) ? INT_MAX : 1024;
     with_block_size(f->b, [&](auto B) {
-      if (cnt >= (sizeof(V) == 4 ? kWideRows : kDeep64)) launch(B, std::integral_constant<int, 1>{}, grid);
-      else launch(B, std::integral_constant<int, 2>{}, grid);
+      if (read == kPlain) launch(B, std::integral_constant<int, kPlain>{}, grid, ask);
+      if (read == kEarly) launch(B, std::integral_constant<int, kEarly>{}, grid, ask);
+      if constexpr ((B() % 2 == 0 && B() > 2) || (sizeof(V) == 8 && B() <= 3))
+        if (read == kDeep) launch(B, std::integral_constant<int, kDeep>{}, grid, ask);
+      if constexpr (B() % 2 == 0 && B() > 2 && sizeof(V) == 4)
+        if (read == kStream) launch(B, std::integral_constant<int, kStream>{}, grid, ask);
     });
   };
   // an fp32 level of few rows by k_ilu_sweep_w; false: not one
   auto warp_rows = [&](auto mode, const int* rows, int cnt) {
     if constexpr (sizeof(V) == 4) {
-      if (cnt >= kDeepRows) return false;
+      if (cnt >= sweep_rows(f->b, f->streamed)) return false;
       const bool T = mode() == kUpperT || mode() == kLowerT;
       const int cap = std::max(1, std::min(f->row_cap - 1, kSweepBlocks));
       with_block_size(f->b, [&](auto B) {
@@ -1620,11 +1678,13 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
       if (f->fuse_fb && l == last ? warp_rows(std::integral_constant<int, kLowerUpper>{}, rows, cnt)
                                   : warp_rows(std::integral_constant<int, kLower>{}, rows, cnt))
         return;
-      lane_groups(cnt, [&](auto B, auto U, int grid) {
+      lane_groups(cnt, [&](auto B, auto M, int grid, int ask) {
         if (f->fuse_fb && l == last)
-          launch_level(k_ilu_lower_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, r, x);
+          launch_level(k_ilu_lower_upper_lg<V, B(), M()>, grid, s, after && early(M()), 128, 0,
+                       F, rows, cnt, ask, r, x);
         else
-          launch_level(k_ilu_lower_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, r, x);
+          launch_level(k_ilu_lower_lg<V, B(), M()>, grid, s, after && early(M()), 128, 0,
+                       F, rows, cnt, ask, r, x);
       });
     });
     levels_of(f->lv_bwd, f->rows_bwd, f->fuse_fb ? 1 : 0, [&](size_t, const int* rows, int cnt) {
@@ -1633,8 +1693,9 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
         return;
       }
       if (warp_rows(std::integral_constant<int, kUpper>{}, rows, cnt)) return;
-      lane_groups(cnt, [&](auto B, auto U, int grid) {
-        launch_level(k_ilu_upper_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, rows, cnt, x);
+      lane_groups(cnt, [&](auto B, auto M, int grid, int ask) {
+        launch_level(k_ilu_upper_lg<V, B(), M()>, grid, s, after && early(M()), 128, 0,
+                     F, rows, cnt, ask, x);
       });
     });
   } else {
@@ -1645,9 +1706,9 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
         return;
       }
       if (warp_rows(std::integral_constant<int, kUpperT>{}, rows, cnt)) return;
-      lane_groups(cnt, [&](auto B, auto U, int grid) {
-        launch_level(k_ilu_upper_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
-                     tval, rows, cnt, r, x);
+      lane_groups(cnt, [&](auto B, auto M, int grid, int ask) {
+        launch_level(k_ilu_upper_t_lg<V, B(), M()>, grid, s, after && early(M()), 128, 0,
+                     F, f->tptr, f->tidx, f->tdiag, tval, rows, cnt, ask, r, x);
       });
     });
     levels_of(f->lv_tbwd, f->rows_tbwd, 0, [&](size_t, const int* rows, int cnt) {
@@ -1657,9 +1718,9 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
         return;
       }
       if (warp_rows(std::integral_constant<int, kLowerT>{}, rows, cnt)) return;
-      lane_groups(cnt, [&](auto B, auto U, int grid) {
-        launch_level(k_ilu_lower_t_lg<V, B(), U()>, grid, s, after && U() > 1, 128, 0, F, f->tptr, f->tidx, f->tdiag,
-                     tval, rows, cnt, x);
+      lane_groups(cnt, [&](auto B, auto M, int grid, int ask) {
+        launch_level(k_ilu_lower_t_lg<V, B(), M()>, grid, s, after && early(M()), 128, 0,
+                     F, f->tptr, f->tidx, f->tdiag, tval, rows, cnt, ask, x);
       });
     });
   }
@@ -1867,6 +1928,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   f->b = b;
   f->nnzb = nnzb;
   f->precision = precision;
+  f->streamed = beyond_l2(nnzb, b, precision);
   for (int i = 0; i < n; ++i) f->row_cap = std::max(f->row_cap, indptr[i + 1] - indptr[i]);
   std::vector<int> rows;
   levels(n, true, [&](int i, auto&& use) {
@@ -1972,6 +2034,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->nnzb = src->nnzb;
   f->precision = precision;
   f->row_cap = src->row_cap;
+  f->streamed = beyond_l2(src->nnzb, src->b, precision);
   f->lv_cap = src->lv_cap;
   f->lv_low = src->lv_low;
   f->lv_sum = src->lv_sum;
@@ -2111,6 +2174,20 @@ extern "C" int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, v
   cudaStream_t s = (cudaStream_t)stream;
   if (f->precision == 64) return ilu_apply<double>(f, (const double*)r, (double*)x, transpose, s);
   return ilu_apply<float>(f, (const float*)r, (float*)x, transpose, s);
+}
+
+extern "C" int fv_ilu0_set_streamed(FvIlu0* f, int streamed) {
+  if (!f) {
+    fv_set_error("fv_ilu0_set_streamed: null factor");
+    return FV_ERR_ARG;
+  }
+  if (f->streamed == (streamed != 0)) return FV_OK;
+  f->streamed = streamed != 0;
+  for (cudaGraphExec_t& e : f->apply_exec) {  // captured with the other kernels
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
+  }
+  return FV_OK;
 }
 
 extern "C" int fv_ilu0_factor_values(const FvIlu0* f, void* out, void* stream) {

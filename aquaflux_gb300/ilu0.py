@@ -140,6 +140,11 @@ class Ilu0:
             v = v.to(torch.float64)
         return v
 
+    def set_streamed(self, streamed: bool) -> None:
+        """Say that a solve finds the factor's blocks in memory, not in the L2 cache (by default: a
+        factor larger than the cache does); the results are the same."""
+        check(lib().fv_ilu0_set_streamed(self._h, int(bool(streamed))))
+
     def factor_values(self) -> torch.Tensor:
         out = torch.empty(self._nvals, dtype=self._dtype, device="cuda")
         check(lib().fv_ilu0_factor_values(self._h, ptr(out), _stream()))

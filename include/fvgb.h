@@ -374,6 +374,10 @@ int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
  * 16-byte aligned: FV_ERR_ARG otherwise); a transposed solve needs one uncaptured transposed solve
  * first. */
 int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, void* stream);
+/* Whether the factor's blocks come from memory rather than the L2 cache at each solve, as in a cycle over
+ * more than the cache holds: it chooses between kernels of the same results.  By default a factor larger
+ * than the cache is taken to. */
+int fv_ilu0_set_streamed(FvIlu0* f, int streamed);
 /* Copy the factor (device, nnzb * b * b, `precision`) -- combined L (unit diagonal) and U. */
 int fv_ilu0_factor_values(const FvIlu0* f, void* out, void* stream);
 

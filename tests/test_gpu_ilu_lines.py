@@ -138,3 +138,41 @@ def test_a_narrow_solve_is_the_same_at_every_width(b, links):
         assert torch.equal(g.solve(r.repeat(k), transpose=True), xt.repeat(k)), k
         d = float((g.solve(r.repeat(k)) - x.repeat(k)).abs().max())
         assert d <= 100 * 2.3e-16 * float(x.abs().max()), (k, d)
+
+
+# rows of 14 blocks beside the diagonal one: their reading is most of a level's time
+@pytest.mark.parametrize("b,precision", [(2, 64), (3, 64), (4, 64), (5, 64), (2, 32), (3, 32), (4, 32), (5, 32), (7, 32)])
+@pytest.mark.parametrize("transpose", [False, True])
+def test_a_solve_of_narrower_levels_is_not_the_slower_one(b, precision, transpose):
+    """Six level sets of 511 to 12,000 rows: no width takes more than 1.12 times what a larger one does."""
+    dtype = torch.float64 if precision == 64 else torch.float32
+    times = []
+    for width in (511, 512, 1024, 1025, 2047, 2049, 3073, 5000, 8191, 8192, 12000):
+        a = _layered(width, 6, 14)
+        f = _factor(a, b, precision, _blocks(a, b, dtype))
+        r = torch.rand(a.shape[0] * b, device="cuda", dtype=dtype)
+        x = torch.empty_like(r)
+        times.append(_time(lambda: f.solve(r, transpose=transpose, out=x), 25))
+    for k, t in enumerate(times):
+        assert t <= 1.12 * min(times[k:]), (k, times)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("b,links", [(2, 3), (3, 14), (4, 16), (5, 9), (6, 3), (6, 12), (7, 6), (8, 10)])
+def test_a_solve_is_the_same_at_every_width(b, links, precision):
+    """Copies side by side and blocks said to come from memory or not, so that a row's level takes every
+    form of reading (from 100 rows, more than one launch a solve takes, to 72,000): bitwise."""
+    dtype = torch.float64 if precision == 64 else torch.float32
+    a = _layered(100, 3, links)
+    v = _blocks(a, b, dtype, seed=b)
+    r = torch.rand(300 * b, device="cuda", dtype=dtype) - 0.5
+    f = _factor(a, b, precision, v)
+    want = [f.solve(r, transpose=t) for t in (False, True)]
+    for k in (1, 5, 6, 11, 20, 31, 50, 90, 200, 400, 720):
+        if precision == 64 and k > 20:
+            break
+        g = _factor(_copies(a, k), b, precision, v.repeat(k))
+        for streamed in (False, True):
+            g.set_streamed(streamed)
+            for t in (False, True):
+                assert torch.equal(g.solve(r.repeat(k), transpose=t), want[t].repeat(k)), (k, streamed, t)
