@@ -79,6 +79,8 @@ SIGNATURES = {
     "fv_bsr_spmv_f32": (c_int, [c_int, c_int, P, P, P, P, P, c_int, P]),
     "fv_bsr_residual_f64": (c_int, [c_int, c_int, P, P, P, P, P, P, P]),
     "fv_bsr_residual_f32": (c_int, [c_int, c_int, P, P, P, P, P, P, P]),
+    "fv_bsr_product_f64": (c_int, [c_int, c_int, c_long, c_int, P, P, P, P, P, P, P]),
+    "fv_bsr_product_f32": (c_int, [c_int, c_int, c_long, c_int, P, P, P, P, P, P, P]),
     "fv_bsr_spmv_t_f64_noalloc": (c_int, [c_int, c_long, c_int, P, P, P, P, P, P]),
     "fv_ilu0_create": (c_int, [c_int, c_int, P, P, c_int, P, P]),
     "fv_ilu0_clone": (c_int, [P, c_int, P, P]),

@@ -41,6 +41,7 @@ class _Level:
         self.indptr = np.ascontiguousarray(indptr, dtype=np.int32)
         self.indices = np.ascontiguousarray(indices, dtype=np.int32)
         self.nnzb = int(self.indptr[-1])
+        self.longest = self.longest_t = int(np.diff(self.indptr).max())  # blocks in a row
         if kept:
             self.d_indptr, self.d_indices = kept["d_indptr"], kept["d_indices"]
             self.ilu = kept["ilu"].clone(precision)
@@ -82,20 +83,20 @@ class _Level:
             check(lib().fv_bsr_transpose_map(self.n, ptr(self.indptr), ptr(self.indices), ptr(tp),
                                              ptr(ti), ptr(tb)))
             self._tmap = [torch.tensor(a, device="cuda") for a in (tp, ti, tb)]
+            self.longest_t = int(np.diff(tp).max())
             self._tvals = torch.empty_like(self.values)
             self.transpose_values()
         return self._tmap[0], self._tmap[1], self._tvals
 
     def spmv(self, x, y, transpose: bool = False):
-        ip, ix, values = self._operator(transpose)
-        check(getattr(lib(), "fv_bsr_spmv_" + self.sfx)(
-            self.n, self.b, ptr(ip), ptr(ix), ptr(values), ptr(x), ptr(y), 0, _stream()))
+        self.residual(None, x, y, transpose)
 
     def residual(self, rhs, x, r, transpose: bool = False):
-        """``r = rhs - A x`` (``A^T x``)."""
+        """``r = rhs - A x`` (``A^T x``), or the product alone."""
         ip, ix, values = self._operator(transpose)
-        check(getattr(lib(), "fv_bsr_residual_" + self.sfx)(
-            self.n, self.b, ptr(ip), ptr(ix), ptr(values), ptr(x), ptr(rhs), ptr(r), _stream()))
+        check(getattr(lib(), "fv_bsr_product_" + self.sfx)(
+            self.n, self.b, self.nnzb, self.longest_t if transpose else self.longest, ptr(ip), ptr(ix),
+            ptr(values), ptr(x), ptr(rhs), ptr(r), _stream()))
 
 
 def plan_hierarchy(n, indptr, indices, *, min_cells: int = 4000, max_levels: int = 10,

@@ -1242,13 +1242,23 @@ __global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* 
   if (lane < B) x[(long)i * B + lane] = acc;
 }
 
-// fp32 y = A x or, RES, rhs - A x of fewer than kWarpProduct block rows: a warp per row as above,
-// which pays the memory's latency once a row instead of once a block; k_bsr_spmv_b's operations in
-// its order.  b = 6, coarse Galerkin rows: 5,370 of them 15.0 -> 8.3 us (7.5 -> 6.5 from L2), 212 of
-// them 13.6 -> 4.3 (6.0 -> 2.8).  The line: rows of a few blocks gain from one round of loads only
-// where the chip is not full of them (7 blocks, b = 6: 1,000 rows 2.6 -> 2.3 us, 8,000 rows 3.4 ->
-// 4.9; 5 blocks, b = 3: 4,096 rows 2.4 either way).
-constexpr int kWarpProduct = 6144;
+// fp32 y = A x or, RES, rhs - A x of few block rows: a warp per row as above, which pays the memory's
+// latency once a row instead of once a block; k_bsr_spmv_b's operations in its order.  b = 6, coarse
+// Galerkin rows: 5,370 of them, 17 blocks a row, 26 at most, 15.0 -> 8.3 us (7.5 -> 6.5 from L2), 212 of
+// them 13.6 -> 4.3 (6.0 -> 2.8).
+// The other kernel's time is its longest row's chain, this one's the warps' work as soon as they no longer
+// run side by side: its line is in rows of the longest's length (warp_product).  From L2, us a thread a
+// scalar row / a warp a row:
+//   b = 6   7 blocks  2,000 rows 3.08 / 2.79, 4,096 3.24 / 3.44, 6,143 3.20 / 4.46   20: 3,000 5.41 / 4.66, 5,000 5.48 / 6.58
+//   b = 4   7 blocks  2,000 rows 2.63 / 2.49, 4,096 2.67 / 2.83                      20: 3,000 4.06 / 3.60, 5,000 4.17 / 4.66
+//   b = 8   7 blocks  1,000 rows 2.99 / 2.84, 2,000 3.02 / 3.29                      20: 2,000 5.27 / 5.24, 5,000 6.14 / 9.34
+// and of fewer than 7 blocks a row, which have little latency to hide, 600 to 2,500 rows.
+inline bool warp_product(int rows, int b, long nnzb, int longest) {
+  if (longest <= 0) longest = (int)(nnzb / rows);  // (unknown)
+  if (longest < 7) return rows < 512;
+  constexpr int line[9] = {0, 0, 4600, 3600, 2900, 3200, 3600, 1500, 1500};
+  return nnzb < (long)line[b] * longest;
+}
 template <int B, bool RES>
 __global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restrict__ ptr,
                                                     const int* __restrict__ idx,
@@ -1296,13 +1306,14 @@ __global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restri
   if (lane < B) y[(long)i * B + lane] = RES ? own - acc : acc;
 }
 
-// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8)
+// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8); nnzb blocks,
+// `longest` in a row
 template <class V, bool RES>
-void launch_spmv_b(int nbr, int b, const int* indptr, const int* indices, const V* values,
+void launch_spmv_b(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices, const V* values,
                    const V* x, const V* rhs, V* y, cudaStream_t s) {
   with_block_size(b, [&](auto B) {
     if constexpr (sizeof(V) == 4) {
-      if (nbr < kWarpProduct) {
+      if (warp_product(nbr, b, nnzb, longest)) {
         k_bsr_spmv_w<B(), RES><<<fv_blocks(nbr, 4), 128, 0, s>>>(nbr, indptr, indices, values, x,
                                                                  rhs, y);
         return;
@@ -2306,7 +2317,7 @@ int spmv(int nbr, int b, const int* indptr, const int* indices, const V* values,
   if (!transpose) {
     const bool aligned = ((uintptr_t)values % 16 == 0) && ((uintptr_t)x % 16 == 0);
     if (aligned && b >= 2 && b <= 8)
-      launch_spmv_b<V, false>(nbr, b, indptr, indices, values, x, (const V*)nullptr, y, s);
+      launch_spmv_b<V, false>(nbr, b, 0, 0, indptr, indices, values, x, (const V*)nullptr, y, s);
     else
       k_bsr_spmv<V><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
                                                                    values, x, nullptr, y);
@@ -2420,30 +2431,57 @@ extern "C" int fv_bsr_spmv_f32(int nbr, int b, const int* indptr, const int* ind
 
 namespace {
 template <class V>
-int bsr_residual(int nbr, int b, const int* indptr, const int* indices, const V* values, const V* x,
-                 const V* rhs, V* r, cudaStream_t s) {
-  if (nbr <= 0 || b <= 0 || !indptr || !indices || !values || !x || !rhs || !r) {
-    fv_set_error("fv_bsr_residual: bad arguments");
-    return FV_ERR_ARG;
+int bsr_product(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices,
+                const V* values, const V* x, const V* rhs, V* y, cudaStream_t s) {
+  if (((uintptr_t)values | (uintptr_t)x) % 16 == 0 && b >= 2 && b <= 8) {
+    if (rhs)
+      launch_spmv_b<V, true>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y, s);
+    else
+      launch_spmv_b<V, false>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y, s);
+  } else {
+    k_bsr_spmv<V><<<fv_blocks((long)nbr * b, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
+                                                                         values, x, rhs, y);
   }
-  if (((uintptr_t)values | (uintptr_t)x) % 16 == 0 && b >= 2 && b <= 8)
-    launch_spmv_b<V, true>(nbr, b, indptr, indices, values, x, rhs, r, s);
-  else
-    k_bsr_spmv<V><<<fv_blocks((long)nbr * b, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices, values, x, rhs, r);
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
+}
+template <class V>
+int bsr_product_checked(const char* name, bool need_rhs, int nbr, int b, long nnzb, int longest,
+                        const int* indptr, const int* indices, const V* values, const V* x,
+                        const V* rhs, V* y, void* stream) {
+  if (nbr <= 0 || b <= 0 || nnzb < 0 || !indptr || !indices || !values || !x || !y ||
+      (need_rhs && !rhs)) {
+    fv_set_error("%s: bad arguments", name);
+    return FV_ERR_ARG;
+  }
+  return bsr_product<V>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y,
+                        (cudaStream_t)stream);
 }
 }  // namespace
 
 extern "C" int fv_bsr_residual_f64(int nbr, int b, const int* indptr, const int* indices,
                                    const double* values, const double* x, const double* rhs,
                                    double* r, void* stream) {
-  return bsr_residual<double>(nbr, b, indptr, indices, values, x, rhs, r, (cudaStream_t)stream);
+  return bsr_product_checked<double>("fv_bsr_residual", true, nbr, b, 0, 0, indptr, indices, values,
+                                     x, rhs, r, stream);
 }
 extern "C" int fv_bsr_residual_f32(int nbr, int b, const int* indptr, const int* indices,
                                    const float* values, const float* x, const float* rhs, float* r,
                                    void* stream) {
-  return bsr_residual<float>(nbr, b, indptr, indices, values, x, rhs, r, (cudaStream_t)stream);
+  return bsr_product_checked<float>("fv_bsr_residual", true, nbr, b, 0, 0, indptr, indices, values,
+                                    x, rhs, r, stream);
+}
+extern "C" int fv_bsr_product_f64(int nbr, int b, long nnzb, int longest, const int* indptr,
+                                  const int* indices, const double* values, const double* x,
+                                  const double* rhs, double* y, void* stream) {
+  return bsr_product_checked<double>("fv_bsr_product", false, nbr, b, nnzb, longest, indptr, indices,
+                                     values, x, rhs, y, stream);
+}
+extern "C" int fv_bsr_product_f32(int nbr, int b, long nnzb, int longest, const int* indptr,
+                                  const int* indices, const float* values, const float* x,
+                                  const float* rhs, float* y, void* stream) {
+  return bsr_product_checked<float>("fv_bsr_product", false, nbr, b, nnzb, longest, indptr, indices,
+                                    values, x, rhs, y, stream);
 }
 
 // out[i] = sum over fields q and cells c in [seg[i], seg[i + 1]) of a[q nc + c] b[q nc + c]: one

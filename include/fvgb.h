@@ -322,6 +322,14 @@ int fv_bsr_residual_f64(int n_block_rows, int b, const int* indptr, const int* i
 int fv_bsr_residual_f32(int n_block_rows, int b, const int* indptr, const int* indices,
                         const float* values, const float* x, const float* rhs, float* r,
                         void* stream);
+/* y = A x, or rhs - A x unless rhs is NULL (bitwise the two above), the kernel chosen knowing the
+ * pattern's nnzb blocks and its longest row's (0: not known). */
+int fv_bsr_product_f64(int n_block_rows, int b, long nnzb, int longest, const int* indptr,
+                       const int* indices, const double* values, const double* x,
+                       const double* rhs, double* y, void* stream);
+int fv_bsr_product_f32(int n_block_rows, int b, long nnzb, int longest, const int* indptr,
+                       const int* indices, const float* values, const float* x, const float* rhs,
+                       float* y, void* stream);
 /* Transpose map of a square BSR pattern (host): tptr (n + 1) / tidx (nnzb) list, for block row j
  * of A^T, the rows i of A holding a block (i, j); tblk (nnzb) that block's index in A. */
 int fv_bsr_transpose_map(int n, const int* indptr, const int* indices, int* tptr, int* tidx,
