@@ -993,9 +993,10 @@ __device__ __forceinline__ void k_apcoef_at(const int f, MeshView m, CaseView cv
 template <class T, int DIM, bool TURB>
 __global__ void __launch_bounds__(128) k_apcoef(MeshView m, CaseView cv, Src<T> st, Par<T> par,
                                                 const T* G, const T* cl, T* ac_own, T* ac_nb,
-                                                T* me, int face0 = 0) {
+                                                T* me) {
   stage_begin();
-  k_apcoef_at<T, DIM, TURB>(face0 + blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, ac_own, ac_nb, me);
+  k_apcoef_at<T, DIM, TURB>(blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, ac_own,
+                            ac_nb, me);
 }
 
 // ---------------------------------------------------------------- k_dcoeff
@@ -1227,10 +1228,10 @@ __device__ __forceinline__ void k_flux_at(const int f, MeshView m, CaseView cv, 
 template <class T, int DIM, bool TURB>
 __global__ void __launch_bounds__(128) k_flux(MeshView m, CaseView cv, Src<T> st, Par<T> par,
                                               const T* G, const T* cl, const T* dco, const T* me,
-                                              const T* psi, bool recompute_me, T* FL, double* aux,
-                                              int face0 = 0) {
+                                              const T* psi, bool recompute_me, T* FL, double* aux) {
   stage_begin();
-  k_flux_at<T, DIM, TURB>(face0 + blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, dco, me, psi, recompute_me, FL, aux);
+  k_flux_at<T, DIM, TURB>(blockIdx.x * blockDim.x + threadIdx.x, m, cv, st, par, G, cl, dco, me, psi,
+                          recompute_me, FL, aux);
 }
 
 // ---------------------------------------------------------------- k_sum
@@ -1369,7 +1370,7 @@ int run(FvCase* cs, Src<T> st, Par<T> par, double* R, double* JV, cudaStream_t s
   fv_prof_mark(cs, 1, s);
   if (TURB) stage(k_closure<T, DIM>, bc(1), tb[1], s, m, cv, st, par, w.G, w.cl, w.Gwi);
   fv_prof_mark(cs, 2, s);
-  stage(k_apcoef<T, DIM, TURB>, bf(2), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me, 0);
+  stage(k_apcoef<T, DIM, TURB>, bf(2), tb[2], s, m, cv, st, par, w.G, w.cl, w.acown, w.acnb, w.me);
   fv_prof_mark(cs, 3, s);
   stage(k_dcoeff<T>, bc(3), tb[3], s, m, w.acown, w.acnb, w.dco);
   const long npsi = psi_count<DIM, TURB>(cs);
@@ -1379,7 +1380,7 @@ int run(FvCase* cs, Src<T> st, Par<T> par, double* R, double* JV, cudaStream_t s
   if (frozen) freeze<T>(w.G, (long)(w.psi + npsi - w.G), s);
   fv_prof_mark(cs, 4, s);
   stage(k_flux<T, DIM, TURB>, bf(4), tb[4], s, m, cv, st, par, w.G, w.cl, w.dco, w.me,
-        npsi ? w.psi : nullptr, frozen, w.FL, aux, 0);
+        npsi ? w.psi : nullptr, frozen, w.FL, aux);
   fv_prof_mark(cs, 5, s);
   stage(k_sum<T, DIM, TURB>, bc(5), tb[5], s, m, cv, st, par, w.FL, w.cl, w.G, w.Gwi, R, JV);
   fv_prof_mark(cs, 6, s);
@@ -1711,8 +1712,9 @@ int linearise(FvCase* cs, const double* state, double* R, cudaStream_t s) {
   };
   if ((!cs->lin_aux && cudaMalloc(&cs->lin_aux, fv_aux_bytes(DIM, TURB, nf)) != cudaSuccess) ||
       !ensure(&cs->lin_me, nf) || !ensure(&cs->lin_d, nc) || !ensure(&cs->lin_g, NF * DIM * nc) ||
-      !ensure(&cs->lin_r, NF * nc) || !ensure(&cs->lin_cl, 7 * nc) ||
-      (TURB && (!ensure(&cs->lin_cc, LIN_NCOEF * nc) || !ensure(&cs->lin_src, 2 * nc)))) {
+      !ensure(&cs->lin_r, NF * nc) ||
+      (TURB && (!ensure(&cs->lin_cl, 7 * nc) || !ensure(&cs->lin_cc, LIN_NCOEF * nc) ||
+                !ensure(&cs->lin_src, 2 * nc)))) {
     fv_set_error("fv_case_linearise: %s", cudaGetErrorString(cudaGetLastError()));
     return FV_ERR_CUDA;
   }
@@ -1734,7 +1736,7 @@ int linearise(FvCase* cs, const double* state, double* R, cudaStream_t s) {
   // the pass writes what is held where it stays
   Work<double> w = work_layout<double, DIM, TURB>(cs->work, nc, nf, psi_count<DIM, TURB>(cs));
   w.G = cs->lin_g;
-  w.cl = cs->lin_cl;
+  if (TURB) w.cl = cs->lin_cl;
   w.me = cs->lin_me;
   w.dco = cs->lin_d;
   int rc = run<double, DIM, TURB>(cs, Src<double>{state},
