@@ -176,3 +176,29 @@ def test_a_solve_is_the_same_at_every_width(b, links, precision):
             g.set_streamed(streamed)
             for t in (False, True):
                 assert torch.equal(g.solve(r.repeat(k), transpose=t), want[t].repeat(k)), (k, streamed, t)
+
+
+# the widths at which fp64 levels change their reading, rows of 11 and 22 blocks on a side (read two at a
+# time, with a remainder, or as the compiler unrolls them)
+@pytest.mark.parametrize("b,links", [(2, 11), (3, 11), (4, 11), (3, 22)])
+@pytest.mark.parametrize("width", [511, 512, 1024, 1025])
+def test_long_rows_on_both_sides_of_a_reading_match_the_oracle(width, b, links):
+    """The factor and the transposed solve bitwise; the forward solve to the rounding of its reordered
+    sums (at most links * b + b terms a row of well-conditioned blocks: 100 units in the last place)."""
+    from tests.ilu_helpers import oracle_factor_solve
+
+    a = _layered(width, 3, links)
+    v = _blocks(a, b, torch.float64, seed=width)
+    full = sp.bsr_matrix((v.cpu().numpy().reshape(-1, b, b), a.indices, a.indptr)).tocsr()
+    full.sort_indices()
+    rhs = np.random.default_rng(width).uniform(-1, 1, a.shape[0] * b)
+    _, data, x, xt = oracle_factor_solve(full.indptr, full.indices, full.data, rhs)
+    f = _factor(a, b, 64, v)
+    got = sp.bsr_matrix((f.factor_values().cpu().numpy().reshape(-1, b, b), a.indices, a.indptr)).tocsr()
+    got.sort_indices()
+    assert np.array_equal(got.data, data)
+    r = torch.tensor(rhs, device="cuda")
+    for streamed in (False, True):
+        f.set_streamed(streamed)
+        assert np.array_equal(f.solve(r, transpose=True).cpu().numpy(), xt)
+        np.testing.assert_allclose(f.solve(r).cpu().numpy(), x, rtol=0, atol=100 * 2.3e-16 * np.abs(x).max())
