@@ -208,10 +208,10 @@ class AmgHierarchy:
                     kf["coarse"] = dict(fine.coarse)
             self.levels.append(_Level(step["n_coarse"], b, step["indptr"], step["indices"],
                                       precision, kl(i + 1)))
-        # A cycle over more than the L2 cache (126 MB; it keeps part of a little more) finds every level's
-        # blocks in memory, the small ones' too.  V-cycles with the solves of small levels told so or not:
-        # 64^3 cells, b = 3 (166 MB) 420 / 443 us, 56^3, b = 4 (196) 363 / 378, 50^3, b = 5 (216) 431 /
-        # 479; 40^3, b = 6 (161) 331 / 329, 50^3, b = 4 (140) 322 / 316.
+        # A cycle over more than the L2 cache (126 MB; it keeps part of a little more) finds every
+        # level's blocks in memory, the small ones' too.  V-cycles with the solves of small levels
+        # told so or not: 64^3 cells, b = 3 (166 MB) 420 / 443 us, 56^3, b = 4 (196) 363 / 378,
+        # 50^3, b = 5 (216) 431 / 479; 40^3, b = 6 (161) 331 / 329, 50^3, b = 4 (140) 322 / 316.
         if 2 * sum(lv.values.numel() * lv.values.element_size() for lv in self.levels) >= 160_000_000:
             for lv in self.levels:
                 lv.ilu.set_streamed(True)

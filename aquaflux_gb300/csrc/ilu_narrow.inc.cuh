@@ -33,14 +33,14 @@ __host__ __device__ constexpr bool run_block_size(int b, size_t vs) {
 }
 // Rows a level may hold: one per lane group of the block.
 inline int run_capacity(int b) { return kRunThreads / run_lanes(b); }
-// ... and in fp64 the rows they may hold in the mean, `most` blocks in a row, for one block's fp64 units not
-// to take longer than a launch per level: soonest in the transposed solve, with twice the operations of
-// the fused forward one.  Time in one launch over that of a launch per level (60 level sets; the launches
-// take 0.34 ms for 2 blocks a row of b = 3, 0.62 for 8), by rows:
-//   transposed, b = 3   2 blocks  64: 0.80, 88: 1.03   4: 48: 0.92, 56: 1.03   8: 40: 0.99, 48: 1.07   20: 24: 1.08
-//               b = 4   2 blocks  64: 0.97, 72: 1.09   4: 40: 0.98, 48: 1.09   8: 32: 0.94, 40: 1.05   20: 24: 1.05
-//               b = 2   2 blocks  96: 0.90             4: 64: 0.96, 72: 1.03   8: 48: 0.92, 56: 1.05   20: 24: 1.03
-//   forward,    b = 4   2 blocks  96: 0.71             4: 80: 1.00, 88: 1.09   8: 80: 0.97, 88: 1.04   20: 88: 0.97
+// ... and in fp64 the rows they may hold in the mean, `most` blocks in a row, for one block's fp64
+// units not to take longer than a launch per level: soonest in the transposed solve, with twice the
+// operations of the fused forward one.  Time in one launch over that of a launch per level (60 level
+// sets; the launches take 0.34 ms for 2 blocks a row of b = 3, 0.62 for 8), by blocks a row and rows:
+//   transposed  b = 3    2: 64 0.80, 88 1.03    4: 48 0.92, 56 1.03    8: 40 0.99, 48 1.07   20: 24 1.08
+//               b = 4    2: 64 0.97, 72 1.09    4: 40 0.98, 48 1.09    8: 32 0.94, 40 1.05   20: 24 1.05
+//               b = 2    2: 96 0.90             4: 64 0.96, 72 1.03    8: 48 0.92, 56 1.05   20: 24 1.03
+//   forward     b = 4    2: 96 0.71             4: 80 1.00, 88 1.09    8: 80 0.97, 88 1.04   20: 88 0.97
 //   and below 1 for b = 2 and 3 throughout
 // (in the mean: 90 x 90 cells, level sets of 1 to 90 rows, b = 3 615 us transposed, 991 by launches).
 inline int run_mean64(int b, int most, bool transposed) {
@@ -92,10 +92,10 @@ __device__ __forceinline__ bool finite_hi(double x) {  // no fp64 comparison
 }
 
 // The records of a solve from the factor's blocks (val: transposed blocks for the transposed solve,
-// whose backward sweep takes a row's blocks from the last one down).  A row of the fp64 forward
-// solve whose pivot's reciprocal or scaled entries would be large or small enough for a product with
-// them to leave the range of doubles stays as it is, marked by a NaN for the reciprocal, and is
-// divided last.
+// whose backward sweep takes a row's blocks from the last one down). A row of the fp64 forward
+// solve whose pivot's reciprocal or scaled entries would be large or small enough for a product
+// with them to leave the range of doubles stays as it is, marked by a NaN for the reciprocal, and
+// is divided last.
 template <class V>
 __global__ void k_run_pack(int n, int b, int k, bool transposed, const int4* row, const V* val,
                            V* rec) {

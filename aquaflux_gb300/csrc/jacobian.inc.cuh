@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(128) k_jac_rows(MeshView m, CaseView cv, const
 }
 
 // The fp64 blocks of J_direct; `src` holds 4 nc doubles.
-// Measured (80 x 63 x 51 SST channel): 6.73 -> 1.13 ms, 0.62 of it k_jac_rows.
+// Measured (80 x 63 x 51 SST channel): 6.73 -> 1.09 ms, 0.6 of it k_jac_rows.
 template <int DIM, bool TURB>
 int assemble_frozen64(FvCase* cs, const double* state, const int* indptr, const int* indices,
                       double* values, double* src, cudaStream_t s) {

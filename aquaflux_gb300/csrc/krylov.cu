@@ -13,9 +13,10 @@
 // Every reduction is a grid of kRedBlocks blocks, or one per tile of a shorter vector, over a
 // grid-stride loop, block partials summed in a fixed order by the last block to finish (a ticket
 // counter), so results are bitwise identical run to run (and the same for either grid: a block
-// without a tile would add zeros.  On 12,288 unknowns those 560 blocks' partials were most of a
-// column's time: 10-20 us a kernel, 5-15 without them).  Up to kChunk basis vectors are handled per launch; a longer basis is
-// processed chunk by chunk with the update and the projection in separate passes.
+// without a tile would add zeros. On 12,288 unknowns those 560 blocks' partials were most of a
+// column's time: 10-20 us a kernel, 5-15 without them). Up to kChunk basis vectors are handled per
+// launch; a longer basis is processed chunk by chunk with the update and the projection in separate
+// passes.
 #include <algorithm>
 #include <cmath>
 

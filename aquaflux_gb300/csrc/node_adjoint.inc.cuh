@@ -720,8 +720,9 @@ __global__ void k_nadj_wd_numerator(MeshView m, CaseView cv, double* num) {
 
 // Wall cells: the closure's wall-distance inputs and the wall faces' areas by seeded evaluations,
 // one per thread (blockIdx.y picks the input; a cell's seven seeded closures in one thread were one
-// serial chain: 385 us of the 48^3 channel's node VJP against 141 us).  Off the wall only 1/d and 1/d^2 enter, through c1 = sqrt(k) / (beta* w d), vt = 500 nu / (d^2 w)
-// and c2 = 4 sigma_w2 k / (cd d^2): the reverse of F1 = tanh(min(max(c1, vt), c2)^4) and
+// serial chain: 385 us of the 48^3 channel's node VJP against 141 us).  Off the wall only 1/d and
+// 1/d^2 enter, through c1 = sqrt(k) / (beta* w d), vt = 500 nu / (d^2 w) and
+// c2 = 4 sigma_w2 k / (cd d^2): the reverse of F1 = tanh(min(max(c1, vt), c2)^4) and
 // nu_t = A1 k / max(A1 w, S tanh(max(2 c1, vt)^2)), as in a_closure.
 template <int DIM>
 __global__ void __launch_bounds__(128) k_nadj_closure(MeshView m, CaseView cv, const double* state,

@@ -1605,11 +1605,14 @@ int run_vjp(FvCase* cs, const double* state, const double* W, double* R, double*
   const bool lim = psi_count<DIM, TURB>(cs) > 0;
   if (lim) aw.psi = fw.psi;
   if (aw.FLx && lim)
-    stage(a_flux<DIM, TURB, true, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me, cs->aux, aw);
+    stage(a_flux<DIM, TURB, true, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me,
+          cs->aux, aw);
   else if (aw.FLx)
-    stage(a_flux<DIM, TURB, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me, cs->aux, aw);
+    stage(a_flux<DIM, TURB, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me, cs->aux,
+          aw);
   else if (lim)
-    stage(a_flux<DIM, TURB, false, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me, cs->aux, aw);
+    stage(a_flux<DIM, TURB, false, true>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me,
+          cs->aux, aw);
   else
     stage(a_flux<DIM, TURB>, bc(7), tb[7], s, m, cv, st, par, G, cl, dco, fw.me, cs->aux, aw);
   if (lim && (cv.lim_km > 0.0 || cv.lim_ks > 0.0)) {
@@ -1628,7 +1631,8 @@ int run_vjp(FvCase* cs, const double* state, const double* W, double* R, double*
     FV_CUDA_TRY(cudaMemcpyAsync(gb_save, aw.Gb, sizeof(double) * L::NFLD * DIM * nc,
                                 cudaMemcpyDeviceToDevice, s));
   if (sweeps >= 2) gb0 = gg_sweeps_adjoint<DIM, L::NFLD>(m, sweeps, rel, aw, fw.FL, s);
-  stage(a_grad_face<DIM, TURB>, fv_blocks(nf, tb[10]), tb[10], s, m, cv, aw, gb0, sweeps >= 2 ? aw.Bb : nullptr, rel, fw.FL);
+  stage(a_grad_face<DIM, TURB>, fv_blocks(nf, tb[10]), tb[10], s, m, cv, aw, gb0,
+        sweeps >= 2 ? aw.Bb : nullptr, rel, fw.FL);
   stage(a_grad<DIM, TURB>, bc(10), tb[10], s, m, cv, aw, fw.FL, out);
   fv_prof_mark(cs, 11, s);
   fv_prof_end_run(cs);

@@ -551,30 +551,31 @@ __device__ __forceinline__ double quotient(double x, double piv, double rpiv) {
 __device__ __forceinline__ float quotient(float x, float piv, float) { return x / piv; }
 
 // Levels of at least this many rows take 8 lanes a row, whose time is a chain along a row's lower
-// blocks while the lanes last; a warp a row shortens the chain and takes four times the lanes, so the
-// line lies higher the longer the rows (`lower`: most lower blocks of a row in the level), and in a level
-// of uneven rows, whose longest is the lanes' chain and whose mean the warps' work, by their ratio.
-// fp32, us a factor of four level sets, lane groups / warps, by lower blocks and rows:
-//   b = 6   3:  5,000  98 /  99   6:  5,000 142 / 129,  8,191 162 / 187   16:  8,191 448 / 411, 12,000 490 / 562
-//   b = 4   3:  5,000  78 /  81   6:  5,000 112 / 113,  8,191 116 / 125   16: 12,000 345 / 347
-//   b = 2   3:  3,000  63 /  65   6:  8,192  97 / 100                     16: 12,000 270 / 255
+// blocks while the lanes last; a warp a row shortens the chain and takes four times the lanes, so
+// the line lies higher the longer the rows (`lower`: most lower blocks of a row in the level), and
+// in a level of uneven rows, whose longest is the lanes' chain and whose mean the warps' work, by
+// their ratio. fp32, us a factor of four level sets, lane groups / warps, by lower blocks and rows:
+//   b = 6    3:  5,000  98 /  99    6: 5,000 142 / 129, 8,191 162 / 187
+//           16:  8,191 448 / 411, 12,000 490 / 562
+//   b = 4    3:  5,000  78 /  81    6: 5,000 112 / 113, 8,191 116 / 125   16: 12,000 345 / 347
+//   b = 2    3:  3,000  63 /  65    6: 8,192  97 / 100                    16: 12,000 270 / 255
 // and at 65,535 rows of 6 lower blocks 622 / 1,171, 342 / 737, 184 / 484.
 constexpr int factor_wide(int b, int lower) {
   return b <= 4 ? 512 * lower + 2048 : 256 * lower + 3072;
 }
 // fp64 issue is four times scarcer for a warp a row than for four rows a warp, so there the line is
-// where the warps' rows fill the SMs' fp64 units; with a lane an entry (b <= 4) it lies higher
-// (3D 48^3, 142 level sets of up to 1,728 rows: b = 6 lane groups 6.55 ms, warps 5.9 ms, warps below
-// 1,024 rows 5.15; b = 4 3.91, 2.46, 2.79.  80^3, up to 4,800 rows, b = 6: 13.0, 20.7 and 11.6).
-// And a level launched early is placed where it finds room, not where fp64 units are free: it pays
-// only while a level has no more rows than there are SMs (64 x 64 cavity 793 us, 1026 without; the
-// 48^3 b = 6 factor 8.4 ms with every level early, 6.2 with none).
+// where the warps' rows fill the SMs' fp64 units; with a lane an entry (b <= 4) it lies higher (3D
+// 48^3, 142 level sets of up to 1,728 rows: b = 6 lane groups 6.55 ms, warps 5.9 ms, warps below
+// 1,024 rows 5.15; b = 4 3.91, 2.46, 2.79. 80^3, up to 4,800 rows, b = 6: 13.0, 20.7 and 11.6). And
+// a level launched early is placed where it finds room, not where fp64 units are free: it pays only
+// while a level has no more rows than there are SMs (64 x 64 cavity 793 us, 1026 without; the 48^3
+// b = 6 factor 8.4 ms with every level early, 6.2 with none).
 constexpr int kFactorWide64(int b) { return b <= 4 ? 2048 : 1024; }
 constexpr int kEarly64 = 152;
 constexpr size_t kFactorSmem = 96 * 1024;
 
-// Shared memory of one warp: the matches of one lower block, the row's columns (padded to a multiple
-// of four), the pivot row's diagonal block and reciprocals, the row's blocks.
+// Shared memory of one warp: the matches of one lower block, the row's columns (padded to a
+// multiple of four), the pivot row's diagonal block and reciprocals, the row's blocks.
 template <class V>
 __host__ __device__ constexpr size_t factor_warp_bytes(int cap, int bb) {
   return (32 * 8 + (size_t)(cap + 7) / 4 * 16 + 72 * sizeof(V) + (size_t)cap * bb * sizeof(V) + 15) /
@@ -832,12 +833,13 @@ __global__ void __launch_bounds__(128) k_ilu_factor_w(IluView<V> F, const int* r
 //   kEarly   the same, launched before the level before has ended
 //   kDeep    so too, two blocks at a time, the columns of eight by the group's lanes at once
 //   kStream  a launch after the other, one block at a time: the fewest registers, the most warps
-// Each asks the L2 cache for the row's first lines, or all of them (`ask` bytes), before its first read.
+// Each asks the L2 cache for the row's first lines, or all of them (`ask` bytes), before its first
+// read.
 enum Read { kPlain, kEarly, kDeep, kStream };
 __host__ __device__ constexpr bool early(int m) { return m == kEarly || m == kDeep; }
 
-// acc minus the products of `count` blocks (positions q0, q0 + STEP, ...) with their columns' entries
-// of x, in that order (and, STEP = -1, each block's entries from the last).
+// acc minus the products of `count` blocks (positions q0, q0 + STEP, ...) with their columns'
+// entries of x, in that order (and, STEP = -1, each block's entries from the last).
 template <class V, int B, int STEP, int M>
 __device__ __forceinline__ V subtract_blocks(V acc, const V* val, const int* idx, const V* x, int q0,
                                              int count, int a, bool live, unsigned mask) {
@@ -891,7 +893,8 @@ __device__ __forceinline__ V subtract_blocks(V acc, const V* val, const int* idx
 
 template <class V, int B>
 __device__ __forceinline__ void ask_blocks(const V* val, int q0, int count, int a, int ask) {
-  // lane a asks for the lines at a, a + 8, ... of the blocks' contiguous range, of its first `ask` bytes
+  // lane a asks for the lines at a, a + 8, ... of the blocks' contiguous range, of its first `ask`
+  // bytes
   const char* p = (const char*)(val + (long)q0 * B * B);
   const long end = min((long)count * B * B * (long)sizeof(V), (long)ask);
   for (long o = 128L * a; o < end; o += 128L * FV_LG)
@@ -1242,16 +1245,19 @@ __global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* 
   if (lane < B) x[(long)i * B + lane] = acc;
 }
 
-// fp32 y = A x or, RES, rhs - A x of few block rows: a warp per row as above, which pays the memory's
-// latency once a row instead of once a block; k_bsr_spmv_b's operations in its order.  b = 6, coarse
-// Galerkin rows: 5,370 of them, 17 blocks a row, 26 at most, 15.0 -> 8.3 us (7.5 -> 6.5 from L2), 212 of
-// them 13.6 -> 4.3 (6.0 -> 2.8).
-// The other kernel's time is its longest row's chain, this one's the warps' work as soon as they no longer
-// run side by side: its line is in rows of the longest's length (warp_product).  From L2, us a thread a
-// scalar row / a warp a row:
-//   b = 6   7 blocks  2,000 rows 3.08 / 2.79, 4,096 3.24 / 3.44, 6,143 3.20 / 4.46   20: 3,000 5.41 / 4.66, 5,000 5.48 / 6.58
-//   b = 4   7 blocks  2,000 rows 2.63 / 2.49, 4,096 2.67 / 2.83                      20: 3,000 4.06 / 3.60, 5,000 4.17 / 4.66
-//   b = 8   7 blocks  1,000 rows 2.99 / 2.84, 2,000 3.02 / 3.29                      20: 2,000 5.27 / 5.24, 5,000 6.14 / 9.34
+// fp32 y = A x or, RES, rhs - A x of few block rows: a warp per row as above, which pays the
+// memory's latency once a row instead of once a block; k_bsr_spmv_b's operations in its order.
+// b = 6, coarse Galerkin rows: 5,370 of them, 17 blocks a row, 26 at most, 15.0 -> 8.3 us (7.5 ->
+// 6.5 from L2), 212 of them 13.6 -> 4.3 (6.0 -> 2.8).
+// The other kernel's time is its longest row's chain, this one's the warps' work as soon as they no
+// longer run side by side: its line is in rows of the longest's length (warp_product).  From L2, us
+// a thread a scalar row / a warp a row:
+//   b = 6    7 blocks  2,000 rows 3.08 / 2.79, 4,096 3.24 / 3.44, 6,143 3.20 / 4.46
+//           20 blocks  3,000 rows 5.41 / 4.66, 5,000 5.48 / 6.58
+//   b = 4    7 blocks  2,000 rows 2.63 / 2.49, 4,096 2.67 / 2.83
+//           20 blocks  3,000 rows 4.06 / 3.60, 5,000 4.17 / 4.66
+//   b = 8    7 blocks  1,000 rows 2.99 / 2.84, 2,000 3.02 / 3.29
+//           20 blocks  2,000 rows 5.27 / 5.24, 5,000 6.14 / 9.34
 // and of fewer than 7 blocks a row, which have little latency to hide, 600 to 2,500 rows.
 inline bool warp_product(int rows, int b, long nnzb, int longest) {
   if (longest <= 0) longest = (int)(nnzb / rows);  // (unknown)
@@ -1306,11 +1312,11 @@ __global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restri
   if (lane < B) y[(long)i * B + lane] = RES ? own - acc : acc;
 }
 
-// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8); nnzb blocks,
-// `longest` in a row
+// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8); nnzb
+// blocks, `longest` in a row
 template <class V, bool RES>
-void launch_spmv_b(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices, const V* values,
-                   const V* x, const V* rhs, V* y, cudaStream_t s) {
+void launch_spmv_b(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices,
+                   const V* values, const V* x, const V* rhs, V* y, cudaStream_t s) {
   with_block_size(b, [&](auto B) {
     if constexpr (sizeof(V) == 4) {
       if (warp_product(nbr, b, nnzb, longest)) {
@@ -1577,9 +1583,9 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
                                                                 f->zero_flag);
       continue;
     }
-    // a level with a row of hundreds of blocks takes lane groups too, which hold no row, and keeps the
-    // other levels to itself (96 x 96 grid, fp64: b = 6 3.1 ms, 4.1 with the first cell coupled to 400
-    // more and 34.9 with every level at a thread a row then; b = 8 4.8, 6.5, 87)
+    // a level with a row of hundreds of blocks takes lane groups too, which hold no row, and keeps
+    // the other levels to itself (96 x 96 grid, fp64: b = 6 3.1 ms, 4.1 with the first cell coupled
+    // to 400 more and 34.9 with every level at a thread a row then; b = 8 4.8, 6.5, 87)
     if (lane_groups(l)) {
       with_block_size(f->b, [&](auto B) {
         k_ilu_factor_lgb<V, B()><<<fv_blocks((long)cnt * FV_LG, 128), 128, 0, s>>>(
@@ -1601,25 +1607,26 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   }
 }
 
-// How a level's lane groups read, by rows and block size, and (streamed) whether the blocks come from
-// memory: a hierarchy's factors, or one larger than the L2 cache.
-// * A level of few rows is its rows' chain of latencies: the next one is launched early.  fp64 to 1,024
-//   rows (above, its blocks would be placed around a level that fp64 issue still binds: 6,000 rows 1.1 to
-//   1.4 times the time), fp32 to 32,768, odd block sizes, whose loads are scalar, to 8,192.
-//   kEarly / kPlain / the form with neither request nor early launch, 6 level sets, fp64 us: 512 rows, 14
-//   blocks, b = 3 92 / 99 / 99.5, b = 6 134 / 146 / 144; 97 rows, 2 blocks, b = 4 58 / 64 / 65.
+// How a level's lane groups read, by rows and block size, and (streamed) whether the blocks come
+// from memory: a hierarchy's factors, or one larger than the L2 cache.
+// * A level of few rows is its rows' chain of latencies: the next one is launched early.  fp64 to
+//   1,024 rows (above, its blocks would be placed around a level that fp64 issue still binds: 6,000
+//   rows 1.1 to 1.4 times the time), fp32 to 32,768, odd block sizes, whose loads are scalar, to
+//   8,192.  kEarly / kPlain / the form with neither request nor early launch, 6 level sets, fp64,
+//   us: 512 rows, 14 blocks, b = 3 92 / 99 / 99.5, b = 6 134 / 146 / 144; 97 rows, 2 blocks, b = 4
+//   58 / 64 / 65.
 // * streamed: two blocks at a time and all of a row's lines asked for (V-cycle of 64^3 cells, fp64,
 //   b = 6, its small levels 3,240 -> 3,150 us; 80^3 fp32, levels of 14,000 rows 966 -> 943; but
 //   128 x 96 x 96, 30,000 rows 1,747 / 1,740, and from L2 4 to 28 % slower for b of 2, 3, 5 and 7).
 //   So, too, the transposed fp64 levels of few short rows of b = 2 and 3 (300 x 200 cells, b = 3, a
 //   transposed V-cycle 6,016 -> 5,830 us; 29 blocks a row, b = 3, 511 rows 97 us, kEarly 86).
-// * The cache is asked for a row's first KB, a line a lane; for all of a row where it is long in bytes and
-//   from memory or early (V-cycles, fp64, b = 6: 50^3 2,067 -> 2,024 us, 24^3 680 -> 661; late and from L2
-//   6,000 rows of 14 blocks 1 to 9 % slower).
-// * The widest are bound by bytes and want warps in flight (590,000 rows, b = 6: 120 us one block at a
-//   time, 180-220 with the registers of a deeper read; 500,000 rows, b = 4 0.78 of kPlain's time, b = 6
-//   0.92), but for the block sizes with scalar or 8-byte loads, which the compiler's unrolling serves
-//   better (b = 2, 16 blocks 71 / 83 us at 131,072 rows).
+// * The cache is asked for a row's first KB, a line a lane; for all of a row where it is long in
+//   bytes and from memory or early (V-cycles, fp64, b = 6: 50^3 2,067 -> 2,024 us, 24^3 680 -> 661;
+//   late and from L2 6,000 rows of 14 blocks 1 to 9 % slower).
+// * The widest are bound by bytes and want warps in flight (590,000 rows, b = 6: 120 us one block
+//   at a time, 180-220 with the registers of a deeper read; 500,000 rows, b = 4 0.78 of kPlain's
+//   time, b = 6 0.92), but for the block sizes with scalar or 8-byte loads, which the compiler's
+//   unrolling serves better (b = 2, 16 blocks 71 / 83 us at 131,072 rows).
 inline int level_read(bool fp32, int b, int rows, int longest, bool streamed, bool transposed) {
   const bool wide_loads = b % 2 == 0 && b > 2;
   if (!fp32) {
@@ -1651,7 +1658,8 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
   auto lane_groups = [&](int cnt, auto&& launch) {
     const int grid = fv_blocks((long)cnt * FV_LG, 128);
     const int read = level_read(sizeof(V) == 4, f->b, cnt, f->row_cap, f->streamed, transpose != 0);
-    const int ask = read == kDeep || (sizeof(V) == 8 && (read == kEarly || f->streamed)) ? INT_MAX : 1024;
+    const bool all = read == kDeep || (sizeof(V) == 8 && (read == kEarly || f->streamed));
+    const int ask = all ? INT_MAX : 1024;
     with_block_size(f->b, [&](auto B) {
       if (read == kPlain) launch(B, std::integral_constant<int, kPlain>{}, grid, ask);
       if (read == kEarly) launch(B, std::integral_constant<int, kEarly>{}, grid, ask);

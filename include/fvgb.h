@@ -314,8 +314,9 @@ int fv_bsr_spmv_t_f64_noalloc(int n_block_rows, long nnzb, int b, const int* ind
 /* fp32 values and vectors. */
 int fv_bsr_spmv_f32(int n_block_rows, int b, const int* indptr, const int* indices,
                     const float* values, const float* x, float* y, int transpose, void* stream);
-/* r = rhs - A x in one pass (device; r overlaps no input): bitwise the difference of rhs and the product of
- * fv_bsr_spmv (the defect of a V-cycle's smoother, aquaflux/solve/multigrid.py:1510-1864). */
+/* r = rhs - A x in one pass (device; r overlaps no input): bitwise the difference of rhs and the
+ * product of fv_bsr_spmv (the defect of a V-cycle's smoother,
+ * aquaflux/solve/multigrid.py:1510-1864). */
 int fv_bsr_residual_f64(int n_block_rows, int b, const int* indptr, const int* indices,
                         const double* values, const double* x, const double* rhs, double* r,
                         void* stream);
@@ -371,10 +372,10 @@ int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvIlu0** out);
 int fv_ilu0_factor(FvIlu0* f, const void* values, int values_f64, void* stream);
 /* Its two halves, to factor several matrices side by side: start enqueues the factorization on a
  * stream of the factor's own (of higher priority if `urgent`; fixed by the first call) behind what
- * `stream` holds by then; finish waits for it, also on `stream`, and reports a zero pivot.  In between
- * `values` stay untouched, and the factor's other calls but clone and destroy, which waits, are refused
- * (FV_ERR_ARG).  A start that fails has waited for what it queued and needs no finish.  Not under stream
- * capture. */
+ * `stream` holds by then; finish waits for it, also on `stream`, and reports a zero pivot.  In
+ * between `values` stay untouched, and the factor's other calls but clone and destroy, which waits,
+ * are refused (FV_ERR_ARG).  A start that fails has waited for what it queued and needs no finish.
+ * Not under stream capture. */
 int fv_ilu0_factor_start(FvIlu0* f, const void* values, int values_f64, int urgent, void* stream);
 int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
 /* x = (LU)^-1 r, or (LU)^-T r when transpose != 0.  Device vectors of `precision`.  On a stream
@@ -382,9 +383,9 @@ int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
  * 16-byte aligned: FV_ERR_ARG otherwise); a transposed solve needs one uncaptured transposed solve
  * first. */
 int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, void* stream);
-/* Whether the factor's blocks come from memory rather than the L2 cache at each solve, as in a cycle over
- * more than the cache holds: it chooses between kernels of the same results.  By default a factor larger
- * than the cache is taken to. */
+/* Whether the factor's blocks come from memory rather than the L2 cache at each solve, as in a cycle
+ * over more than the cache holds: it chooses between kernels of the same results.  By default a
+ * factor larger than the cache is taken to. */
 int fv_ilu0_set_streamed(FvIlu0* f, int streamed);
 /* Copy the factor (device, nnzb * b * b, `precision`) -- combined L (unit diagonal) and U. */
 int fv_ilu0_factor_values(const FvIlu0* f, void* out, void* stream);
