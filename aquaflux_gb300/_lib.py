@@ -79,8 +79,8 @@ SIGNATURES = {
     "fv_bsr_spmv_f32": (c_int, [c_int, c_int, P, P, P, P, P, c_int, P]),
     "fv_bsr_residual_f64": (c_int, [c_int, c_int, P, P, P, P, P, P, P]),
     "fv_bsr_residual_f32": (c_int, [c_int, c_int, P, P, P, P, P, P, P]),
-    "fv_bsr_product_f64": (c_int, [c_int, c_int, c_long, c_int, P, P, P, P, P, P, P]),
-    "fv_bsr_product_f32": (c_int, [c_int, c_int, c_long, c_int, P, P, P, P, P, P, P]),
+    "fv_bsr_product_f64": (c_int, [c_int, c_int, c_long, c_int, c_long, P, P, P, P, P, P, P]),
+    "fv_bsr_product_f32": (c_int, [c_int, c_int, c_long, c_int, c_long, P, P, P, P, P, P, P]),
     "fv_bsr_spmv_t_f64_noalloc": (c_int, [c_int, c_long, c_int, P, P, P, P, P, P]),
     "fv_ilu0_create": (c_int, [c_int, c_int, P, P, c_int, P, P]),
     "fv_ilu0_clone": (c_int, [P, c_int, P, P]),
@@ -88,7 +88,7 @@ SIGNATURES = {
     "fv_ilu0_factor": (c_int, [P, P, c_int, P]),
     "fv_ilu0_factor_start": (c_int, [P, P, c_int, c_int, P]),
     "fv_ilu0_factor_finish": (c_int, [P, P]),
-    "fv_ilu0_set_streamed": (c_int, [P, c_int]),
+    "fv_ilu0_set_traffic": (c_int, [P, c_long]),
     "fv_ilu0_apply": (c_int, [P, P, P, c_int, P]),
     "fv_ilu0_factor_values": (c_int, [P, P, P]),
     "fv_dot_f64": (c_int, [c_long, P, P, P, P]),

@@ -42,6 +42,7 @@ class _Level:
         self.indices = np.ascontiguousarray(indices, dtype=np.int32)
         self.nnzb = int(self.indptr[-1])
         self.longest = self.longest_t = int(np.diff(self.indptr).max())  # blocks in a row
+        self.traffic = 0  # bytes between two products (set_traffic)
         if kept:
             self.d_indptr, self.d_indices = kept["d_indptr"], kept["d_indices"]
             self.ilu = kept["ilu"].clone(precision)
@@ -95,8 +96,13 @@ class _Level:
         """``r = rhs - A x`` (``A^T x``), or the product alone."""
         ip, ix, values = self._operator(transpose)
         check(getattr(lib(), "fv_bsr_product_" + self.sfx)(
-            self.n, self.b, self.nnzb, self.longest_t if transpose else self.longest, ptr(ip), ptr(ix),
-            ptr(values), ptr(x), ptr(rhs), ptr(r), _stream()))
+            self.n, self.b, self.nnzb, self.longest_t if transpose else self.longest, self.traffic,
+            ptr(ip), ptr(ix), ptr(values), ptr(x), ptr(rhs), ptr(r), _stream()))
+
+    def set_traffic(self, n_bytes: int) -> None:
+        """The bytes that pass between two uses of this level's blocks."""
+        self.traffic = n_bytes
+        self.ilu.set_traffic(n_bytes)
 
 
 def plan_hierarchy(n, indptr, indices, *, min_cells: int = 4000, max_levels: int = 10,
@@ -208,13 +214,13 @@ class AmgHierarchy:
                     kf["coarse"] = dict(fine.coarse)
             self.levels.append(_Level(step["n_coarse"], b, step["indptr"], step["indices"],
                                       precision, kl(i + 1)))
-        # A cycle over more than the L2 cache (126 MB; it keeps part of a little more) finds every
-        # level's blocks in memory, the small ones' too.  V-cycles with the solves of small levels
-        # told so or not: 64^3 cells, b = 3 (166 MB) 420 / 443 us, 56^3, b = 4 (196) 363 / 378,
-        # 50^3, b = 5 (216) 431 / 479; 40^3, b = 6 (161) 331 / 329, 50^3, b = 4 (140) 322 / 316.
-        if 2 * sum(lv.values.numel() * lv.values.element_size() for lv in self.levels) >= 160_000_000:
-            for lv in self.levels:
-                lv.ilu.set_streamed(True)
+        # What a cycle reads of all levels passes between two uses of each (operators and factors).
+        # Over about the L2 cache's 126 MB the small levels' blocks come from memory too: V-cycles
+        # with their solves told so or not, 64^3 cells, b = 3 (166 MB) 420 / 443 us, 56^3, b = 4
+        # (196) 363 / 378, 50^3, b = 5 (216) 431 / 479; 40^3, b = 6 (161) 331 / 329.
+        traffic = 2 * sum(lv.values.numel() * lv.values.element_size() for lv in self.levels)
+        for lv in self.levels:
+            lv.set_traffic(traffic)
         last = self.levels[-1]
         nd = last.n * b
         self.dense = None

@@ -1121,9 +1121,9 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // 4,000 rows gain 3 to 13 % (1,000 rows 13 to 28 %) and 8,191 lose 3 to 48 % to the lane groups.
 // The operations and their order are the lane-group kernels'.
 enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
-constexpr int sweep_rows(int b, bool streamed) {
+constexpr int sweep_rows(int b, long traffic) {
   if (b == 7 || b == 8) return 2048;  // 21 to 37 KB a block of four warps: few of them on an SM
-  return streamed ? 8192 : b == 5 ? 2048 : 3072;
+  return traffic >= 160000000 ? 8192 : b == 5 ? 2048 : 3072;
 }
 
 constexpr int kSweepBlocks = 32;  // blocks in shared memory at a time: a column a lane
@@ -1258,10 +1258,13 @@ __global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* 
 //           20 blocks  3,000 rows 4.06 / 3.60, 5,000 4.17 / 4.66
 //   b = 8    7 blocks  1,000 rows 2.99 / 2.84, 2,000 3.02 / 3.29
 //           20 blocks  2,000 rows 5.27 / 5.24, 5,000 6.14 / 9.34
-// and of fewer than 7 blocks a row, which have little latency to hide, 600 to 2,500 rows.
-inline bool warp_product(int rows, int b, long nnzb, int longest) {
+// and of fewer than 7 blocks a row, which have little latency to hide, 600 to 2,500 rows.  From memory
+// (traffic, the bytes between two products) more rows gain: V-cycles of 42,000 cells, b = 6, 5,000
+// coarse rows of 14 blocks, 16 at most, 283 / 279 us.
+inline bool warp_product(int rows, int b, long nnzb, int longest, long traffic) {
   if (longest <= 0) longest = (int)(nnzb / rows);  // (unknown)
   if (longest < 7) return rows < 512;
+  if (traffic >= 100000000 && longest > 9) return rows < 6144;
   constexpr int line[9] = {0, 0, 4600, 3600, 2900, 3200, 3600, 1500, 1500};
   return nnzb < (long)line[b] * longest;
 }
@@ -1312,14 +1315,21 @@ __global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restri
   if (lane < B) y[(long)i * B + lane] = RES ? own - acc : acc;
 }
 
-// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8); nnzb
-// blocks, `longest` in a row
+// What a caller knows of a product's pattern and use: its blocks, the longest row's, and the bytes
+// that pass between two products (0: not known).
+struct ProductHint {
+  long nnzb = 0;
+  int longest = 0;
+  long traffic = 0;
+};
+
+// y = A x, or rhs - A x with RES, where the alignment allows vector loads (2 <= b <= 8)
 template <class V, bool RES>
-void launch_spmv_b(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices,
+void launch_spmv_b(int nbr, int b, const ProductHint& hint, const int* indptr, const int* indices,
                    const V* values, const V* x, const V* rhs, V* y, cudaStream_t s) {
   with_block_size(b, [&](auto B) {
     if constexpr (sizeof(V) == 4) {
-      if (warp_product(nbr, b, nnzb, longest)) {
+      if (warp_product(nbr, b, hint.nnzb, hint.longest, hint.traffic)) {
         k_bsr_spmv_w<B(), RES><<<fv_blocks(nbr, 4), 128, 0, s>>>(nbr, indptr, indices, values, x,
                                                                  rhs, y);
         return;
@@ -1397,7 +1407,7 @@ struct FvIlu0 {
   int* rows_tbwd = nullptr;  // L^T order
   std::vector<int> lv_fwd, lv_bwd, lv_tfwd, lv_tbwd;
   void* work = nullptr;                      // (n * b) vector the captured sweeps run on
-  bool streamed = false;  // the blocks come from memory at each solve
+  long traffic = 0;  // bytes read between two reads of a block (fv_ilu0_set_traffic)
   // (b > 1) narrow level sets: the forward / transposed solve as one launch (ilu_narrow.inc.cuh)
   struct Run {
     int4* row = nullptr;    // 2n rows in level order, forward sweep then backward
@@ -1444,11 +1454,6 @@ void levels(int n, bool ascending, DepFn deps, std::vector<int>* rows, std::vect
   rows->assign(n, 0);
   std::vector<int> fill(bounds->begin(), bounds->end() - 1);
   for (int i = 0; i < n; ++i) (*rows)[fill[lev[i]]++] = i;
-}
-
-// A factor larger than the L2 cache (126 MB).
-inline bool beyond_l2(long nnzb, int b, int precision) {
-  return nnzb * b * b * (precision / 8) >= 126000000;
 }
 
 template <class V>
@@ -1607,17 +1612,18 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   }
 }
 
-// How a level's lane groups read, by rows and block size, and (streamed) whether the blocks come
-// from memory: a hierarchy's factors, or one larger than the L2 cache.
+// How a level's lane groups read, by rows and block size, and by the bytes that pass between two
+// solves (traffic): from about the L2 cache's 126 MB on, its blocks come from memory.
 // * A level of few rows is its rows' chain of latencies: the next one is launched early.  fp64 to
 //   1,024 rows (above, its blocks would be placed around a level that fp64 issue still binds: 6,000
 //   rows 1.1 to 1.4 times the time), fp32 to 32,768, odd block sizes, whose loads are scalar, to
 //   8,192.  kEarly / kPlain / the form with neither request nor early launch, 6 level sets, fp64,
 //   us: 512 rows, 14 blocks, b = 3 92 / 99 / 99.5, b = 6 134 / 146 / 144; 97 rows, 2 blocks, b = 4
 //   58 / 64 / 65.
-// * streamed: two blocks at a time and all of a row's lines asked for (V-cycle of 64^3 cells, fp64,
-//   b = 6, its small levels 3,240 -> 3,150 us; 80^3 fp32, levels of 14,000 rows 966 -> 943; but
-//   128 x 96 x 96, 30,000 rows 1,747 / 1,740, and from L2 4 to 28 % slower for b of 2, 3, 5 and 7).
+// * From memory: two blocks at a time and all of a row's lines asked for (V-cycle of 64^3 cells,
+//   fp64, b = 6, its small levels 3,240 -> 3,150 us; fp32 80^3, levels of 14,000 rows 966 -> 943,
+//   22 x 96 x 21, a cycle of 113 MB, levels of 22,000 289 -> 283; but 128 x 96 x 96, 30,000 rows
+//   1,747 / 1,740, and from L2 4 to 28 % slower for b of 2, 3, 5 and 7).
 //   So, too, the transposed fp64 levels of few short rows of b = 2 and 3 (300 x 200 cells, b = 3, a
 //   transposed V-cycle 6,016 -> 5,830 us; 29 blocks a row, b = 3, 511 rows 97 us, kEarly 86).
 // * The cache is asked for a row's first KB, a line a lane; for all of a row where it is long in
@@ -1627,17 +1633,17 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
 //   at a time, 180-220 with the registers of a deeper read; 500,000 rows, b = 4 0.78 of kPlain's
 //   time, b = 6 0.92), but for the block sizes with scalar or 8-byte loads, which the compiler's
 //   unrolling serves better (b = 2, 16 blocks 71 / 83 us at 131,072 rows).
-inline int level_read(bool fp32, int b, int rows, int longest, bool streamed, bool transposed) {
+inline int level_read(bool fp32, int b, int rows, int longest, long traffic, bool transposed) {
   const bool wide_loads = b % 2 == 0 && b > 2;
   if (!fp32) {
-    if (rows < 512 && (wide_loads ? streamed : transposed && b <= 3 && longest <= 16))
+    if (rows < 512 && (wide_loads ? traffic >= 160000000 : transposed && b <= 3 && longest <= 16))
       return kDeep;
     return rows <= 1024 ? kEarly : kPlain;
   }
   if (rows < 8192) return kEarly;
   if (rows >= 65536) return wide_loads ? kStream : kPlain;
   if (b % 2 != 0) return kPlain;
-  if (streamed && wide_loads && rows < 24576) return kDeep;
+  if (traffic >= 100000000 && wide_loads && rows < 24576) return kDeep;
   return rows < 32768 ? kEarly : wide_loads ? kStream : kPlain;
 }
 
@@ -1657,8 +1663,9 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
   // the lane-group kernels of a level, by block size and reading
   auto lane_groups = [&](int cnt, auto&& launch) {
     const int grid = fv_blocks((long)cnt * FV_LG, 128);
-    const int read = level_read(sizeof(V) == 4, f->b, cnt, f->row_cap, f->streamed, transpose != 0);
-    const bool all = read == kDeep || (sizeof(V) == 8 && (read == kEarly || f->streamed));
+    const int read = level_read(sizeof(V) == 4, f->b, cnt, f->row_cap, f->traffic, transpose != 0);
+    const bool all = read == kDeep ||
+                     (sizeof(V) == 8 && (read == kEarly || f->traffic >= 160000000));
     const int ask = all ? INT_MAX : 1024;
     with_block_size(f->b, [&](auto B) {
       if (read == kPlain) launch(B, std::integral_constant<int, kPlain>{}, grid, ask);
@@ -1672,7 +1679,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
   // an fp32 level of few rows by k_ilu_sweep_w; false: not one
   auto warp_rows = [&](auto mode, const int* rows, int cnt) {
     if constexpr (sizeof(V) == 4) {
-      if (cnt >= sweep_rows(f->b, f->streamed)) return false;
+      if (cnt >= sweep_rows(f->b, f->traffic)) return false;
       const bool T = mode() == kUpperT || mode() == kLowerT;
       const int cap = std::max(1, std::min(f->row_cap - 1, kSweepBlocks));
       with_block_size(f->b, [&](auto B) {
@@ -1947,7 +1954,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   f->b = b;
   f->nnzb = nnzb;
   f->precision = precision;
-  f->streamed = beyond_l2(nnzb, b, precision);
+  f->traffic = (long)nnzb * b * b * (precision / 8);
   for (int i = 0; i < n; ++i) f->row_cap = std::max(f->row_cap, indptr[i + 1] - indptr[i]);
   std::vector<int> rows;
   levels(n, true, [&](int i, auto&& use) {
@@ -2053,7 +2060,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->nnzb = src->nnzb;
   f->precision = precision;
   f->row_cap = src->row_cap;
-  f->streamed = beyond_l2(src->nnzb, src->b, precision);
+  f->traffic = (long)src->nnzb * src->b * src->b * (precision / 8);
   f->lv_cap = src->lv_cap;
   f->lv_low = src->lv_low;
   f->lv_sum = src->lv_sum;
@@ -2195,13 +2202,13 @@ extern "C" int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, v
   return ilu_apply<float>(f, (const float*)r, (float*)x, transpose, s);
 }
 
-extern "C" int fv_ilu0_set_streamed(FvIlu0* f, int streamed) {
-  if (!f) {
-    fv_set_error("fv_ilu0_set_streamed: null factor");
+extern "C" int fv_ilu0_set_traffic(FvIlu0* f, long bytes) {
+  if (!f || bytes < 0) {
+    fv_set_error("fv_ilu0_set_traffic: bad arguments");
     return FV_ERR_ARG;
   }
-  if (f->streamed == (streamed != 0)) return FV_OK;
-  f->streamed = streamed != 0;
+  if (f->traffic == bytes) return FV_OK;
+  f->traffic = bytes;
   for (cudaGraphExec_t& e : f->apply_exec) {  // captured with the other kernels
     if (e) cudaGraphExecDestroy(e);
     e = nullptr;
@@ -2325,7 +2332,7 @@ int spmv(int nbr, int b, const int* indptr, const int* indices, const V* values,
   if (!transpose) {
     const bool aligned = ((uintptr_t)values % 16 == 0) && ((uintptr_t)x % 16 == 0);
     if (aligned && b >= 2 && b <= 8)
-      launch_spmv_b<V, false>(nbr, b, 0, 0, indptr, indices, values, x, (const V*)nullptr, y, s);
+      launch_spmv_b<V, false>(nbr, b, {}, indptr, indices, values, x, (const V*)nullptr, y, s);
     else
       k_bsr_spmv<V><<<fv_blocks(rows, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
                                                                    values, x, nullptr, y);
@@ -2439,13 +2446,20 @@ extern "C" int fv_bsr_spmv_f32(int nbr, int b, const int* indptr, const int* ind
 
 namespace {
 template <class V>
-int bsr_product(int nbr, int b, long nnzb, int longest, const int* indptr, const int* indices,
-                const V* values, const V* x, const V* rhs, V* y, cudaStream_t s) {
+int bsr_product(const char* name, bool need_rhs, int nbr, int b, const ProductHint& hint,
+                const int* indptr, const int* indices, const V* values, const V* x, const V* rhs,
+                V* y, void* stream) {
+  if (nbr <= 0 || b <= 0 || hint.nnzb < 0 || !indptr || !indices || !values || !x || !y ||
+      (need_rhs && !rhs)) {
+    fv_set_error("%s: bad arguments", name);
+    return FV_ERR_ARG;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
   if (((uintptr_t)values | (uintptr_t)x) % 16 == 0 && b >= 2 && b <= 8) {
     if (rhs)
-      launch_spmv_b<V, true>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y, s);
+      launch_spmv_b<V, true>(nbr, b, hint, indptr, indices, values, x, rhs, y, s);
     else
-      launch_spmv_b<V, false>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y, s);
+      launch_spmv_b<V, false>(nbr, b, hint, indptr, indices, values, x, rhs, y, s);
   } else {
     k_bsr_spmv<V><<<fv_blocks((long)nbr * b, kThreads), kThreads, 0, s>>>(nbr, b, indptr, indices,
                                                                          values, x, rhs, y);
@@ -2453,43 +2467,31 @@ int bsr_product(int nbr, int b, long nnzb, int longest, const int* indptr, const
   FV_CUDA_TRY(cudaGetLastError());
   return FV_OK;
 }
-template <class V>
-int bsr_product_checked(const char* name, bool need_rhs, int nbr, int b, long nnzb, int longest,
-                        const int* indptr, const int* indices, const V* values, const V* x,
-                        const V* rhs, V* y, void* stream) {
-  if (nbr <= 0 || b <= 0 || nnzb < 0 || !indptr || !indices || !values || !x || !y ||
-      (need_rhs && !rhs)) {
-    fv_set_error("%s: bad arguments", name);
-    return FV_ERR_ARG;
-  }
-  return bsr_product<V>(nbr, b, nnzb, longest, indptr, indices, values, x, rhs, y,
-                        (cudaStream_t)stream);
-}
 }  // namespace
 
 extern "C" int fv_bsr_residual_f64(int nbr, int b, const int* indptr, const int* indices,
                                    const double* values, const double* x, const double* rhs,
                                    double* r, void* stream) {
-  return bsr_product_checked<double>("fv_bsr_residual", true, nbr, b, 0, 0, indptr, indices, values,
-                                     x, rhs, r, stream);
+  return bsr_product<double>("fv_bsr_residual", true, nbr, b, {}, indptr, indices, values, x, rhs, r,
+                             stream);
 }
 extern "C" int fv_bsr_residual_f32(int nbr, int b, const int* indptr, const int* indices,
                                    const float* values, const float* x, const float* rhs, float* r,
                                    void* stream) {
-  return bsr_product_checked<float>("fv_bsr_residual", true, nbr, b, 0, 0, indptr, indices, values,
-                                    x, rhs, r, stream);
+  return bsr_product<float>("fv_bsr_residual", true, nbr, b, {}, indptr, indices, values, x, rhs, r,
+                            stream);
 }
-extern "C" int fv_bsr_product_f64(int nbr, int b, long nnzb, int longest, const int* indptr,
-                                  const int* indices, const double* values, const double* x,
-                                  const double* rhs, double* y, void* stream) {
-  return bsr_product_checked<double>("fv_bsr_product", false, nbr, b, nnzb, longest, indptr, indices,
-                                     values, x, rhs, y, stream);
+extern "C" int fv_bsr_product_f64(int nbr, int b, long nnzb, int longest, long traffic,
+                                  const int* indptr, const int* indices, const double* values,
+                                  const double* x, const double* rhs, double* y, void* stream) {
+  return bsr_product<double>("fv_bsr_product", false, nbr, b, {nnzb, longest, traffic}, indptr,
+                             indices, values, x, rhs, y, stream);
 }
-extern "C" int fv_bsr_product_f32(int nbr, int b, long nnzb, int longest, const int* indptr,
-                                  const int* indices, const float* values, const float* x,
-                                  const float* rhs, float* y, void* stream) {
-  return bsr_product_checked<float>("fv_bsr_product", false, nbr, b, nnzb, longest, indptr, indices,
-                                    values, x, rhs, y, stream);
+extern "C" int fv_bsr_product_f32(int nbr, int b, long nnzb, int longest, long traffic,
+                                  const int* indptr, const int* indices, const float* values,
+                                  const float* x, const float* rhs, float* y, void* stream) {
+  return bsr_product<float>("fv_bsr_product", false, nbr, b, {nnzb, longest, traffic}, indptr,
+                            indices, values, x, rhs, y, stream);
 }
 
 // out[i] = sum over fields q and cells c in [seg[i], seg[i + 1]) of a[q nc + c] b[q nc + c]: one

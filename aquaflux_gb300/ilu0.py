@@ -140,10 +140,10 @@ class Ilu0:
             v = v.to(torch.float64)
         return v
 
-    def set_streamed(self, streamed: bool) -> None:
-        """Say that a solve finds the factor's blocks in memory, not in the L2 cache (by default: a
-        factor larger than the cache does); the results are the same."""
-        check(lib().fv_ilu0_set_streamed(self._h, int(bool(streamed))))
+    def set_traffic(self, n_bytes: int) -> None:
+        """The bytes that pass between two solves with this factor, its own among them (by default
+        those alone): whether its blocks are then in the L2 cache.  The results are the same."""
+        check(lib().fv_ilu0_set_traffic(self._h, int(n_bytes)))
 
     def factor_values(self) -> torch.Tensor:
         out = torch.empty(self._nvals, dtype=self._dtype, device="cuda")

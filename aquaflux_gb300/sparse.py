@@ -32,7 +32,7 @@ def bsr_spmv(indptr, indices, values, block_size: int, x, *, transpose: bool = F
     nbr = ip.numel() - 1
     y = torch.empty(nbr * block_size, dtype=dtype, device="cuda") if out is None else out
     if dtype == torch.float32 and not transpose:  # whose kernel depends on the blocks a row
-        check(lib().fv_bsr_product_f32(nbr, block_size, ix.numel(), 0, ptr(ip), ptr(ix), ptr(v),
+        check(lib().fv_bsr_product_f32(nbr, block_size, ix.numel(), 0, 0, ptr(ip), ptr(ix), ptr(v),
                                        ptr(xv), None, ptr(y), _stream()))
         return y
     fn = lib().fv_bsr_spmv_f64 if dtype == torch.float64 else lib().fv_bsr_spmv_f32

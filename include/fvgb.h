@@ -324,13 +324,14 @@ int fv_bsr_residual_f32(int n_block_rows, int b, const int* indptr, const int* i
                         const float* values, const float* x, const float* rhs, float* r,
                         void* stream);
 /* y = A x, or rhs - A x unless rhs is NULL (bitwise the two above), the kernel chosen knowing the
- * pattern's nnzb blocks and its longest row's (0: not known). */
-int fv_bsr_product_f64(int n_block_rows, int b, long nnzb, int longest, const int* indptr,
-                       const int* indices, const double* values, const double* x,
-                       const double* rhs, double* y, void* stream);
-int fv_bsr_product_f32(int n_block_rows, int b, long nnzb, int longest, const int* indptr,
-                       const int* indices, const float* values, const float* x, const float* rhs,
-                       float* y, void* stream);
+ * pattern's nnzb blocks, its longest row's (0: not known) and the bytes that pass between two products
+ * with it (0: not known), which say whether its blocks come from the L2 cache or from memory. */
+int fv_bsr_product_f64(int n_block_rows, int b, long nnzb, int longest, long traffic,
+                       const int* indptr, const int* indices, const double* values,
+                       const double* x, const double* rhs, double* y, void* stream);
+int fv_bsr_product_f32(int n_block_rows, int b, long nnzb, int longest, long traffic,
+                       const int* indptr, const int* indices, const float* values, const float* x,
+                       const float* rhs, float* y, void* stream);
 /* Transpose map of a square BSR pattern (host): tptr (n + 1) / tidx (nnzb) list, for block row j
  * of A^T, the rows i of A holding a block (i, j); tblk (nnzb) that block's index in A. */
 int fv_bsr_transpose_map(int n, const int* indptr, const int* indices, int* tptr, int* tidx,
@@ -383,10 +384,10 @@ int fv_ilu0_factor_finish(FvIlu0* f, void* stream);
  * 16-byte aligned: FV_ERR_ARG otherwise); a transposed solve needs one uncaptured transposed solve
  * first. */
 int fv_ilu0_apply(FvIlu0* f, const void* r, void* x, int transpose, void* stream);
-/* Whether the factor's blocks come from memory rather than the L2 cache at each solve, as in a cycle
- * over more than the cache holds: it chooses between kernels of the same results.  By default a
- * factor larger than the cache is taken to. */
-int fv_ilu0_set_streamed(FvIlu0* f, int streamed);
+/* The bytes that pass between two solves with this factor, its own among them (by default: those
+ * alone).  Whether its blocks are then found in the L2 cache or in memory chooses between kernels of
+ * the same results. */
+int fv_ilu0_set_traffic(FvIlu0* f, long bytes);
 /* Copy the factor (device, nnzb * b * b, `precision`) -- combined L (unit diagonal) and U. */
 int fv_ilu0_factor_values(const FvIlu0* f, void* out, void* stream);
 

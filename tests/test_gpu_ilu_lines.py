@@ -172,10 +172,10 @@ def test_a_solve_is_the_same_at_every_width(b, links, precision):
         if precision == 64 and k > 20:
             break
         g = _factor(_copies(a, k), b, precision, v.repeat(k))
-        for streamed in (False, True):
-            g.set_streamed(streamed)
+        for traffic in (0, 120_000_000, 10**9):
+            g.set_traffic(traffic)
             for t in (False, True):
-                assert torch.equal(g.solve(r.repeat(k), transpose=t), want[t].repeat(k)), (k, streamed, t)
+                assert torch.equal(g.solve(r.repeat(k), transpose=t), want[t].repeat(k)), (k, traffic, t)
 
 
 # the widths at which fp64 levels change their reading, rows of 11 and 22 blocks on a side (read two at a
@@ -198,7 +198,7 @@ def test_long_rows_on_both_sides_of_a_reading_match_the_oracle(width, b, links):
     got.sort_indices()
     assert np.array_equal(got.data, data)
     r = torch.tensor(rhs, device="cuda")
-    for streamed in (False, True):
-        f.set_streamed(streamed)
+    for traffic in (0, 10**9):
+        f.set_traffic(traffic)
         assert np.array_equal(f.solve(r, transpose=True).cpu().numpy(), xt)
         np.testing.assert_allclose(f.solve(r).cpu().numpy(), x, rtol=0, atol=100 * 2.3e-16 * np.abs(x).max())

@@ -41,8 +41,9 @@ def test_products_are_the_operations_in_turn(b, n, counts):
     d = [torch.tensor(v, device="cuda") for v in (indptr, indices, a.reshape(-1), x, rhs)]
     ip, ix, av, xv, rv = map(ptr, d)
     y = torch.empty(n * b, device="cuda")
-    calls = [lambda r: lib().fv_bsr_product_f32(n, b, indices.size, int(nq.max()), ip, ix, av, xv, r, ptr(y), 0),
-             lambda r: lib().fv_bsr_product_f32(n, b, indices.size, 0, ip, ix, av, xv, r, ptr(y), 0),
+    calls = [lambda r: lib().fv_bsr_product_f32(n, b, indices.size, int(nq.max()), 0, ip, ix, av, xv, r, ptr(y), 0),
+             lambda r: lib().fv_bsr_product_f32(n, b, indices.size, int(nq.max()), 10**9, ip, ix, av, xv, r, ptr(y), 0),
+             lambda r: lib().fv_bsr_product_f32(n, b, indices.size, 0, 0, ip, ix, av, xv, r, ptr(y), 0),
              lambda r: (lib().fv_bsr_residual_f32(n, b, ip, ix, av, xv, r, ptr(y), 0) if r else
                         lib().fv_bsr_spmv_f32(n, b, ip, ix, av, xv, ptr(y), 0, 0))]
     for call in calls:
