@@ -196,8 +196,8 @@ int fv_case_run(FvCase* c, const double* state, const double* tangent, int tange
                 double* residual, double* jv, cudaStream_t s);
 int fv_case_vjp_run(FvCase* c, const double* state, const double* w, double* residual, double* out,
                     cudaStream_t s);
-// The residual at a (physical) state with its face intermediates and primal face fluxes kept for
-// the linearised JVP (residual.cu); refuses limited reconstruction.
+// The residual at a (physical) state with its face intermediates, gradients and closure kept for the
+// linearised JVP (residual.cu); refuses limited reconstruction.
 int fv_case_linearise(FvCase* c, const double* state, double* residual, cudaStream_t s);
 // The VJP's forward pass at a (physical) state, held in the workspace for fv_case_vjp_held, which
 // runs only the adjoint stages (residual.cu).  Any other evaluation drops the hold.

@@ -528,8 +528,8 @@ __global__ void k_ilu_factor_lgb(IluView<V> F, const int* rows, int count,
 // columns of row j come in one load, each lane counting row i's columns below its own to find its
 // place; what the pattern alone gives is found before the level before is waited for; the next row
 // j is fetched and the matching blocks' columns are read before the chain of quotients, which hides
-// them; and the matching blocks are updated side by side.  Pivots of finished rows come with their reciprocals
-// (`rp`): a quotient is a product and a correction, not a division on the chain (fp64: 192 cycles
+// them; and the matching blocks are updated side by side.  Pivots of finished rows come with their
+// reciprocals (`rp`): a quotient is a product and a correction, not a division on the chain (fp64: 192 cycles
 // for 321).
 // Lanes: for b <= 4 one per block entry (16 to a block, two blocks at a time), which keeps the
 // number of fp64 instructions, 64 cycles each, at one per elimination step; above, one per column
@@ -554,23 +554,46 @@ __device__ __forceinline__ float quotient(float x, float piv, float) { return x 
 // blocks while the lanes last; a warp a row shortens the chain and takes four times the lanes, so
 // the line lies higher the longer the rows (`lower`: most lower blocks of a row in the level), and
 // in a level of uneven rows, whose longest is the lanes' chain and whose mean the warps' work, by
-// their ratio. fp32, us a factor of four level sets, lane groups / warps, by lower blocks and rows:
+// their ratio.  fp32, us a factor of four level sets, lane groups / warps, by lower blocks and rows:
 //   b = 6    3:  5,000  98 /  99    6: 5,000 142 / 129, 8,191 162 / 187
 //           16:  8,191 448 / 411, 12,000 490 / 562
 //   b = 4    3:  5,000  78 /  81    6: 5,000 112 / 113, 8,191 116 / 125   16: 12,000 345 / 347
 //   b = 2    3:  3,000  63 /  65    6: 8,192  97 / 100                    16: 12,000 270 / 255
-// and at 65,535 rows of 6 lower blocks 622 / 1,171, 342 / 737, 184 / 484.
-constexpr int factor_wide(int b, int lower) {
-  return b <= 4 ? 512 * lower + 2048 : 256 * lower + 3072;
+//   b = 8   10:  8,191 306 / 354   16: 8,191 510 / 545
+// and at 65,535 rows of 6 lower blocks 622 / 1,171, 342 / 737, 184 / 484 (80^3 grid in reverse
+// Cuthill-McKee order, level sets of up to 4,800 rows of 3: b = 2 1,438 / 1,223, b = 4 1,979 / 1,714,
+// b = 6 2,571 / 2,514; 96^3, 6,900 rows: 1,923 / 1,913, 2,619 / 2,715, 3,560 / 3,627).
+// Rows scattered over the matrix (a grid's own order, where a level set is a diagonal) cost the lane
+// groups' short reads more than the warps' long ones: 80^3 grid, level sets of up to 4,800 rows, us
+// a factor with the line at 4,000 / 6,144: b = 2 1,466 / 1,216, b = 4 1,956 / 1,698, b = 6 2,614 /
+// 2,521; 112^3, 9,408 rows, at 6,144 / 8,192 / 12,288: b = 3 3,191 / 3,137 / 3,307, b = 6 4,721 /
+// 4,892 / 5,455.
+constexpr int factor_wide(int b, int lower, bool scattered) {
+  const int line = b <= 4   ? 512 * lower + 3400
+                   : b <= 6 ? 256 * lower + 4100
+                            : 128 * lower + 3600;
+  return scattered ? std::max(line, b <= 4 ? 8192 : 6144) : line;
 }
 // fp64 issue is four times scarcer for a warp a row than for four rows a warp, so there the line is
 // where the warps' rows fill the SMs' fp64 units; with a lane an entry (b <= 4) it lies higher (3D
 // 48^3, 142 level sets of up to 1,728 rows: b = 6 lane groups 6.55 ms, warps 5.9 ms, warps below
-// 1,024 rows 5.15; b = 4 3.91, 2.46, 2.79. 80^3, up to 4,800 rows, b = 6: 13.0, 20.7 and 11.6). And
-// a level launched early is placed where it finds room, not where fp64 units are free: it pays only
-// while a level has no more rows than there are SMs (64 x 64 cavity 793 us, 1026 without; the 48^3
-// b = 6 factor 8.4 ms with every level early, 6.2 with none).
-constexpr int kFactorWide64(int b) { return b <= 4 ? 2048 : 1024; }
+// 1,024 rows 5.15; b = 4 3.91, 2.46, 2.79.  80^3, up to 4,800 rows, b = 6: 13.0, 20.7 and 11.6).
+// And a level launched early is placed where it finds room, not where fp64 units are free: it pays
+// only while a level has no more rows than there are SMs (64 x 64 cavity 793 us, 1026 without; the
+// 48^3 b = 6 factor 8.4 ms with every level early, 6.2 with none).
+// The warps' time goes by rounds of one warp on each of the 608 quarters of an SM, the lane groups'
+// by the chain: with few lower blocks a round less.  Warps / lane groups, 12 level sets, by lower
+// blocks:
+//   b = 3   1,100 rows  2: 0.93, 3: 0.84   1,300  2: 1.09, 3: 1.08, 4: 0.95   1,900  4: 1.15, 6: 0.98
+//   b = 6     600 rows  1: 0.87, 3: 0.69     800  1: 1.25, 2: 1.16, 3: 1.06, 6: 0.92
+// (3: 48^3 grid in reverse Cuthill-McKee order, level sets of up to 1,728 rows, b = 4 2,522 us with
+// all of them by warps, 2,670 from 1,217 rows on by lane groups).  Scattered, the same grid's own
+// order, line at 1,024 / 2,048: b = 4 2,745 / 2,450.
+constexpr int factor_wide64(int b, int lower, bool scattered) {
+  constexpr int round = 4 * 152;
+  if (b > 4) return scattered || lower >= 3 ? 1024 : round + 1;
+  return scattered || lower >= 6 ? 2048 : (lower >= 3 ? 3 : 2) * round + 1;
+}
 constexpr int kEarly64 = 152;
 constexpr size_t kFactorSmem = 96 * 1024;
 
@@ -1122,7 +1145,7 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // The operations and their order are the lane-group kernels'.
 enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
 constexpr int sweep_rows(int b, long traffic) {
-  if (b == 7 || b == 8) return 2048;  // 21 to 37 KB a block of four warps: few of them on an SM
+  if (b >= 7) return b == 7 ? 1024 : 2048;  // scalar loads; up to 37 KB a block, few on an SM
   return traffic >= 160000000 ? 8192 : b == 5 ? 2048 : 3072;
 }
 
@@ -1395,6 +1418,7 @@ struct FvIlu0 {
   int row_cap = 0;        // most blocks in a row
   std::vector<int> lv_cap, lv_low;  // ... of each forward level, and most lower blocks
   std::vector<long> lv_sum;         // ... and its lower blocks together
+  std::vector<char> lv_scattered;   // ... and whether its rows do not lie beside each other
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
   bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
@@ -1572,8 +1596,10 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
   auto lane_groups = [&](size_t l) {
     const int cnt = f->lv_fwd[l + 1] - f->lv_fwd[l], low = f->lv_low[l];
     if (factor_warp_bytes<V>(f->lv_cap[l], bb) > kFactorSmem) return true;
-    if (sizeof(V) == 8) return cnt >= kFactorWide64(f->b);
-    return low ? f->lv_sum[l] >= (long)factor_wide(f->b, low) * low : cnt >= factor_wide(f->b, 0);
+    const bool far = f->lv_scattered[l];
+    if (sizeof(V) == 8) return cnt >= factor_wide64(f->b, low, far);
+    const long line = factor_wide(f->b, low, far);
+    return low ? f->lv_sum[l] >= line * low : cnt >= line;
   };
   bool warps = false;  // a level takes warps, which read the pivots' reciprocals
   for (size_t l = 0; l + 1 < f->lv_fwd.size(); ++l) warps = warps || !lane_groups(l);
@@ -1966,13 +1992,18 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   f->lv_cap.assign(nf - 1, 0);
   f->lv_low.assign(nf - 1, 0);
   f->lv_sum.assign(nf - 1, 0);
-  for (size_t l = 0; l + 1 < nf; ++l)
+  f->lv_scattered.assign(nf - 1, 0);
+  for (size_t l = 0; l + 1 < nf; ++l) {
+    int jumps = 0;
     for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k) {
       const int i = rows[k];
+      jumps += k > f->lv_fwd[l] && rows[k - 1] != i - 1;
       f->lv_cap[l] = std::max(f->lv_cap[l], indptr[i + 1] - indptr[i]);
       f->lv_low[l] = std::max(f->lv_low[l], diag[i] - indptr[i]);
       f->lv_sum[l] += diag[i] - indptr[i];
     }
+    f->lv_scattered[l] = jumps > (f->lv_fwd[l + 1] - f->lv_fwd[l]) / 8;
+  }
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
     for (int q = diag[i] + 1; q < indptr[i + 1]; ++q) use(indices[q]);
@@ -2064,6 +2095,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->lv_cap = src->lv_cap;
   f->lv_low = src->lv_low;
   f->lv_sum = src->lv_sum;
+  f->lv_scattered = src->lv_scattered;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;

@@ -186,14 +186,14 @@ int fv_jvp(FvCase* c, const double* state, const double* v, double* residual, do
 /* The linearised Jacobian-vector product (jax.linearize's split of the reference's
  * jax.jvp(residual_fn, (phi,), (v,)), aquaflux/solve/newton.py:110-111): fv_linearise evaluates the
  * residual at `state` (into `residual`, device, may be NULL) and holds that evaluation's face
- * intermediates, primal face fluxes, gradients, residual and (SST) the off-wall cells' closure and
- * source tangents as linear forms in (k', omega', S', (grad k . grad omega)'); fv_jvp_linearised then
- * gives J(state) v (and, when `residual` is not NULL, the held residual) with the interior faces'
- * flux, coefficient and compact-gradient stages, the off-wall closure and the face sums computed as
- * tangents only, every other stage as fv_jvp does.  `state` must be the linearised one.  A change of parameters, of the
- * viscosity field, of the wall distance or of the geometry (fv_case_refresh_geometry) drops the
- * linearisation; fv_jvp_linearised then refuses until fv_linearise runs again.  First-order upwind
- * advection only (a limited reconstruction is refused by fv_linearise). */
+ * intermediates, mass-flux estimates, d, gradients, residual and (SST) closure fields, and the off-wall
+ * cells' closure and source tangents as linear forms in (k', omega', S', (grad k . grad omega)');
+ * fv_jvp_linearised then gives J(state) v (and, when `residual` is not NULL, the held residual) as
+ * tangents only, boundary faces and wall cells by the formulas of fv_jvp.  `state` must be the
+ * linearised one.  A change of parameters, of the viscosity field, of the wall distance or of the
+ * geometry (fv_case_refresh_geometry) drops the linearisation; fv_jvp_linearised then refuses until
+ * fv_linearise runs again.  First-order upwind advection only (a limited reconstruction is refused
+ * by fv_linearise). */
 int fv_linearise(FvCase* c, const double* state, double* residual, void* stream);
 int fv_jvp_linearised(FvCase* c, const double* state, const double* v, double* residual,
                       double* jv, void* stream);

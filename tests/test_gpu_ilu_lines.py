@@ -94,6 +94,19 @@ def test_a_factor_of_narrower_levels_is_not_the_slower_one(b, links):
         assert t <= 1.2 * min(times[k:]), (k, times)
 
 
+@pytest.mark.parametrize("b,links", [(2, 3), (3, 1), (3, 3), (4, 2), (4, 4), (4, 6), (5, 1), (6, 2), (8, 1)])
+def test_an_fp64_factor_of_narrower_levels_is_not_the_slower_one(b, links):
+    """Twelve level sets of 300 to 3,000 rows: no width takes more than 1.15 times what a larger one does."""
+    times = []
+    for width in (300, 608, 609, 900, 1023, 1024, 1216, 1217, 1500, 1824, 1825, 2047, 2048, 3000):
+        a = _layered(width, 12, links)
+        v = _blocks(a, b, torch.float64)
+        f = _factor(a, b, 64, v)
+        times.append(_time(lambda: f.refactor(v)))
+    for k, t in enumerate(times):
+        assert t <= 1.15 * min(times[k:]), (k, times)
+
+
 @pytest.mark.parametrize("precision", [32, 64])
 @pytest.mark.parametrize("b,links", [(2, 3), (3, 6), (4, 16), (5, 1), (6, 3), (6, 12), (7, 6), (8, 3)])
 def test_a_factor_is_the_same_at_every_width(b, links, precision):
@@ -102,9 +115,32 @@ def test_a_factor_is_the_same_at_every_width(b, links, precision):
     a = _layered(500, 3, links)
     v = _blocks(a, b, dtype, seed=b)
     want = _factor(a, b, precision, v).factor_values()
-    for k in (7, 12, 24):  # 3,500, 6,000 and 12,000 rows a level set
+    for k in (2, 3, 7, 12, 24):  # 1,000 to 12,000 rows a level set
         got = _factor(_copies(a, k), b, precision, v.repeat(k)).factor_values()
         assert torch.equal(got, want.repeat(k)), k
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("b", [2, 4, 6])
+def test_a_factor_is_the_same_for_scattered_rows(b, precision):
+    """A grid's own order, whose level sets are diagonals of up to 1,200 rows, and its reverse
+    Cuthill-McKee-like order by diagonals, whose level sets lie together: bitwise, block by block."""
+    dtype = torch.float64 if precision == 64 else torch.float32
+    nx, ny, nz = 40, 36, 32
+    e = [sp.diags([1.0, 1.0, 1.0], [-1, 0, 1], shape=(k, k)) for k in (nx, ny, nz)]
+    i = [sp.eye(k) for k in (nx, ny, nz)]
+    a = (sp.kron(sp.kron(e[2], i[1]), i[0]) + sp.kron(sp.kron(i[2], e[1]), i[0]) +
+         sp.kron(sp.kron(i[2], i[1]), e[0])).tocsr()
+    a.sort_indices()
+    q = np.arange(nx * ny * nz)
+    p = np.argsort(q // (nx * ny) + q // nx % ny + q % nx, kind="stable")  # ascending on a diagonal
+    where = sp.csr_matrix((np.arange(1, a.nnz + 1), a.indices, a.indptr))[p][:, p].tocsr()
+    where.sort_indices()
+    v = _blocks(a, b, dtype, seed=b)
+    block = torch.tensor(where.data - 1, device="cuda")
+    f = _factor(a, b, precision, v).factor_values().reshape(-1, b * b)
+    g = _factor(where, b, precision, v.reshape(-1, b * b)[block].reshape(-1)).factor_values()
+    assert torch.equal(g, f[block].reshape(-1))
 
 
 @pytest.mark.parametrize("transpose", [False, True])
