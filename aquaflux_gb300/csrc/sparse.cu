@@ -1138,15 +1138,28 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 // are in place before the level before is waited for; all its x entries then come in one round of
 // loads, a block's by a lane, and what is left is the subtractions one after the other: 2 us a level
 // set.  fp32 V-cycle of the 128 x 96 x 96 channel 2083 -> 1868 us, of 40^3 cells 607 -> 345.
-// The line (sweep_rows) lies where the lanes run out instead of a row's chain.  Blocks that come from
-// memory, as in a cycle over several hundred MB, hide that up to more rows: 64^3 cells 590 us a cycle,
-// 688 with lane groups from 3,072 rows on (b = 5 597 / 645, b = 4 420 / 471); but from L2 levels of
-// 4,000 rows gain 3 to 13 % (1,000 rows 13 to 28 %) and 8,191 lose 3 to 48 % to the lane groups.
+// The line (sweep_rows) lies where the lanes run out instead of a row's chain.  A warp's time over the
+// lane groups', level sets of rows of 2 / 13 blocks before the diagonal one, forward:
+//   from L2      b = 2  3,500 rows 0.86 / 0.85, 5,500 1.03 / 0.92, 8,000 1.44 / 1.25
+//                b = 4  3,500 rows 0.92 / 0.84, 5,500 1.03 / 0.78, 8,000 1.44
+//                b = 5  2,000 rows 0.88 / 0.92, 3,500 1.08 / 1.06
+//                b = 8  2,000 rows 0.94, 3,500 1.04, 5,500 0.99
+//   from memory  b = 4  3,500 rows 0.78 / 0.63, 5,500 0.98 / 0.76, 8,000 1.66 / 1.26
+//                b = 5  5,500 rows 1.03 / 1.06, 8,000 1.08 / 1.14, of scattered rows 0.79 / 0.89
+//                b = 7  3,500 rows 0.91 / 0.88, 5,500 1.09 / 1.04, 8,000 1.18 / 1.18, scattered 1.07 / 0.86
+//                b = 8  3,500 rows 0.94 / 0.86, 5,500 1.02 / 0.97, 8,000 1.45 / 1.40
+// Scattered rows (a grid's own order) cost the lane groups more: solves on a 96^3 grid, lines at 4,608
+// and at 8,192 rows, b = 2 1,216 / 1,105 us; at 6,144 and 8,192, b = 6 1,523 / 1,452, b = 4 1,382 / 1,407,
+// and at 5,120 and 8,192, b = 8 1,829 / 2,045.
 // The operations and their order are the lane-group kernels'.
 enum { kLower, kLowerUpper, kUpper, kUpperT, kLowerT };
-constexpr int sweep_rows(int b, long traffic) {
-  if (b >= 7) return b == 7 ? 1024 : 2048;  // scalar loads; up to 37 KB a block, few on an SM
-  return traffic >= 160000000 ? 8192 : b == 5 ? 2048 : 3072;
+constexpr int sweep_rows(int b, long traffic, bool scattered) {
+  constexpr int l2[9] = {0, 0, 4608, 4608, 5120, 2560, 5120, 1536, 4096};
+  constexpr int memory[9] = {0, 0, 6144, 8192, 6144, 8192, 6144, 7168, 5120};
+  constexpr int l2_far[9] = {0, 0, 7168, 7168, 6144, 3584, 7168, 3072, 4096};
+  constexpr int memory_far[9] = {0, 0, 7168, 8192, 6144, 8192, 7168, 8192, 5120};
+  if (scattered) return traffic >= 160000000 ? memory_far[b] : l2_far[b];
+  return traffic >= 160000000 ? memory[b] : l2[b];
 }
 
 constexpr int kSweepBlocks = 32;  // blocks in shared memory at a time: a column a lane
@@ -1419,6 +1432,7 @@ struct FvIlu0 {
   std::vector<int> lv_cap, lv_low;  // ... of each forward level, and most lower blocks
   std::vector<long> lv_sum;         // ... and its lower blocks together
   std::vector<char> lv_scattered;   // ... and whether its rows do not lie beside each other
+  bool scattered = false;           // most rows are in such a level
   cudaStream_t side = nullptr;  // of fv_ilu0_factor_start
   bool open = false;            // started, not finished: the factor belongs to `side`
   cudaEvent_t side_event = nullptr;
@@ -1650,6 +1664,10 @@ void launch_factor_levels(FvIlu0* f, cudaStream_t s) {
 //   fp64, b = 6, its small levels 3,240 -> 3,150 us; fp32 80^3, levels of 14,000 rows 966 -> 943,
 //   22 x 96 x 21, a cycle of 113 MB, levels of 22,000 289 -> 283; but 128 x 96 x 96, 30,000 rows
 //   1,747 / 1,740, and from L2 4 to 28 % slower for b of 2, 3, 5 and 7).
+//   fp32 of odd b so, over kPlain's time, from memory: 9,000 to 14,000 rows of 2 blocks before the
+//   diagonal one b = 3 0.79 to 0.90, b = 5 0.85 to 1.06, b = 7 0.97 to 1.09, of 13 blocks 0.99 to
+//   1.25; 20,000 rows 0.83 to 1.02; 28,000 0.83 to 1.28, 40,000 and 60,000 0.96 to 1.14 (solves on
+//   a 150^3 grid, b = 3, transposed, 3,008 -> 2,666 us, b = 5 3,593 -> 3,344).
 //   So, too, the transposed fp64 levels of few short rows of b = 2 and 3 (300 x 200 cells, b = 3, a
 //   transposed V-cycle 6,016 -> 5,830 us; 29 blocks a row, b = 3, 511 rows 97 us, kEarly 86).
 // * The cache is asked for a row's first KB, a line a lane; for all of a row where it is long in
@@ -1668,7 +1686,9 @@ inline int level_read(bool fp32, int b, int rows, int longest, long traffic, boo
   }
   if (rows < 8192) return kEarly;
   if (rows >= 65536) return wide_loads ? kStream : kPlain;
-  if (b % 2 != 0) return kPlain;
+  if (b % 2 != 0)
+    return traffic >= 160000000 && rows < 24576 && (rows >= 16384 || (b < 7 && longest <= 9))
+               ? kDeep : kPlain;
   if (traffic >= 100000000 && wide_loads && rows < 24576) return kDeep;
   return rows < 32768 ? kEarly : wide_loads ? kStream : kPlain;
 }
@@ -1696,7 +1716,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
     with_block_size(f->b, [&](auto B) {
       if (read == kPlain) launch(B, std::integral_constant<int, kPlain>{}, grid, ask);
       if (read == kEarly) launch(B, std::integral_constant<int, kEarly>{}, grid, ask);
-      if constexpr ((B() % 2 == 0 && B() > 2) || (sizeof(V) == 8 && B() <= 3))
+      if constexpr (sizeof(V) == 8 ? B() % 2 == 0 || B() == 3 : B() != 2)
         if (read == kDeep) launch(B, std::integral_constant<int, kDeep>{}, grid, ask);
       if constexpr (B() % 2 == 0 && B() > 2 && sizeof(V) == 4)
         if (read == kStream) launch(B, std::integral_constant<int, kStream>{}, grid, ask);
@@ -1705,7 +1725,7 @@ void launch_apply_levels(FvIlu0* f, int transpose, const V* r, V* x, cudaStream_
   // an fp32 level of few rows by k_ilu_sweep_w; false: not one
   auto warp_rows = [&](auto mode, const int* rows, int cnt) {
     if constexpr (sizeof(V) == 4) {
-      if (cnt >= sweep_rows(f->b, f->traffic)) return false;
+      if (cnt >= sweep_rows(f->b, f->traffic, f->scattered)) return false;
       const bool T = mode() == kUpperT || mode() == kLowerT;
       const int cap = std::max(1, std::min(f->row_cap - 1, kSweepBlocks));
       with_block_size(f->b, [&](auto B) {
@@ -1993,6 +2013,7 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
   f->lv_low.assign(nf - 1, 0);
   f->lv_sum.assign(nf - 1, 0);
   f->lv_scattered.assign(nf - 1, 0);
+  int far = 0;
   for (size_t l = 0; l + 1 < nf; ++l) {
     int jumps = 0;
     for (int k = f->lv_fwd[l]; k < f->lv_fwd[l + 1]; ++k) {
@@ -2003,7 +2024,9 @@ extern "C" int fv_ilu0_create(int n, int b, const int* indptr, const int* indice
       f->lv_sum[l] += diag[i] - indptr[i];
     }
     f->lv_scattered[l] = jumps > (f->lv_fwd[l + 1] - f->lv_fwd[l]) / 8;
+    if (f->lv_scattered[l]) far += f->lv_fwd[l + 1] - f->lv_fwd[l];
   }
+  f->scattered = far > n / 2;
   std::vector<int> fwd_last(rows.begin() + f->lv_fwd[nf - 2], rows.begin() + f->lv_fwd[nf - 1]);
   levels(n, false, [&](int i, auto&& use) {
     for (int q = diag[i] + 1; q < indptr[i + 1]; ++q) use(indices[q]);
@@ -2096,6 +2119,7 @@ extern "C" int fv_ilu0_clone(const FvIlu0* src, int precision, void* stream, FvI
   f->lv_low = src->lv_low;
   f->lv_sum = src->lv_sum;
   f->lv_scattered = src->lv_scattered;
+  f->scattered = src->scattered;
   f->lv_fwd = src->lv_fwd;
   f->lv_bwd = src->lv_bwd;
   f->lv_tfwd = src->lv_tfwd;

@@ -194,7 +194,7 @@ def test_a_solve_of_narrower_levels_is_not_the_slower_one(b, precision, transpos
 
 
 @pytest.mark.parametrize("precision", [32, 64])
-@pytest.mark.parametrize("b,links", [(2, 3), (3, 14), (4, 16), (5, 9), (6, 3), (6, 12), (7, 6), (8, 10)])
+@pytest.mark.parametrize("b,links", [(2, 3), (3, 3), (3, 14), (4, 16), (5, 3), (5, 9), (6, 3), (6, 12), (7, 6), (8, 10)])
 def test_a_solve_is_the_same_at_every_width(b, links, precision):
     """Copies side by side and blocks said to come from memory or not, so that a row's level takes every
     form of reading (from 100 rows, more than one launch a solve takes, to 72,000): bitwise."""
