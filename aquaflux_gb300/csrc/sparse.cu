@@ -1146,7 +1146,7 @@ __global__ void k_ilu_lower_t_lg(IluView<V> F, const int* tptr, const int* tidx,
 //                b = 8  2,000 rows 0.94, 3,500 1.04, 5,500 0.99
 //   from memory  b = 4  3,500 rows 0.78 / 0.63, 5,500 0.98 / 0.76, 8,000 1.66 / 1.26
 //                b = 5  5,500 rows 1.03 / 1.06, 8,000 1.08 / 1.14, of scattered rows 0.79 / 0.89
-//                b = 7  3,500 rows 0.91 / 0.88, 5,500 1.09 / 1.04, 8,000 1.18 / 1.18, scattered 1.07 / 0.86
+//                b = 7  3,500 rows 0.90 / 0.86, 5,500 1.06 / 1.00, 8,000 1.19 / 1.13, scattered 1.08 / 0.89
 //                b = 8  3,500 rows 0.94 / 0.86, 5,500 1.02 / 0.97, 8,000 1.45 / 1.40
 // Scattered rows (a grid's own order) cost the lane groups more: solves on a 96^3 grid, lines at 4,608
 // and at 8,192 rows, b = 2 1,216 / 1,105 us; at 6,144 and 8,192, b = 6 1,523 / 1,452, b = 4 1,382 / 1,407,
@@ -1286,23 +1286,29 @@ __global__ void __launch_bounds__(128) k_ilu_sweep_w(const int* ptr, const int* 
 // b = 6, coarse Galerkin rows: 5,370 of them, 17 blocks a row, 26 at most, 15.0 -> 8.3 us (7.5 ->
 // 6.5 from L2), 212 of them 13.6 -> 4.3 (6.0 -> 2.8).
 // The other kernel's time is its longest row's chain, this one's the warps' work as soon as they no
-// longer run side by side: its line is in rows of the longest's length (warp_product).  From L2, us
-// a thread a scalar row / a warp a row:
-//   b = 6    7 blocks  2,000 rows 3.08 / 2.79, 4,096 3.24 / 3.44, 6,143 3.20 / 4.46
-//           20 blocks  3,000 rows 5.41 / 4.66, 5,000 5.48 / 6.58
-//   b = 4    7 blocks  2,000 rows 2.63 / 2.49, 4,096 2.67 / 2.83
-//           20 blocks  3,000 rows 4.06 / 3.60, 5,000 4.17 / 4.66
-//   b = 8    7 blocks  1,000 rows 2.99 / 2.84, 2,000 3.02 / 3.29
-//           20 blocks  2,000 rows 5.27 / 5.24, 5,000 6.14 / 9.34
-// and of fewer than 7 blocks a row, which have little latency to hide, 600 to 2,500 rows.  From memory
-// (traffic, the bytes between two products) more rows gain: V-cycles of 42,000 cells, b = 6, 5,000
-// coarse rows of 14 blocks, 16 at most, 283 / 279 us.
+// longer run side by side: its line is in rows of the longest's length (warp_product).  This one's
+// time over the other's, from L2 / from memory:
+//   b = 2  grids of 5 blocks a row  3,025 rows 0.89 / 0.96, 5,184 0.95 / 0.98, 6,400 1.03 / 0.80
+//          7  3,375 rows 0.88 / 0.74, 5,832 0.96 / 0.92, 8,000 1.24 / 1.00;  27  8,000 1.00 / 0.79
+//   b = 4  5  2,025 rows 0.88 / 1.00, 4,096 0.98 / 1.00, 6,400 1.12 / 0.97
+//          7  2,744 rows 0.96 / 0.98, 4,096 1.05 / 0.80, 5,832 1.10 / 0.80
+//         27  4,096 rows 0.83 / 0.60, 5,832 0.96 / 0.74, 8,000 1.26 / 0.87
+//             (20, at random columns, from L2: 3,000 rows 0.89, 5,000 1.12)
+//   b = 6  5  2,025 rows 0.83 / 0.82, 4,096 1.01 / 0.80, 6,400 1.39 / 1.00
+//          7  2,744 rows 0.94 / 0.80, 4,096 1.08 / 0.81, 6,859 1.40 / 1.03
+//         27  3,375 rows 0.89 / 0.60, 4,913 1.11 / 0.70, 5,832 1.22 / 0.81
+//   b = 8  5  2,025 rows 0.95 / 0.80, 4,096 1.45 / 1.23;  7  2,197 rows 1.03 / 0.81, 4,096 1.52 / 1.20
+//         27  2,197 rows 0.97 / 0.66, 4,096 1.47 / 0.90, 4,913 1.91 / 1.09
+// traffic: the bytes between two products (0: not known, as from L2).
 inline bool warp_product(int rows, int b, long nnzb, int longest, long traffic) {
-  if (longest <= 0) longest = (int)(nnzb / rows);  // (unknown)
-  if (longest < 7) return rows < 512;
-  if (traffic >= 100000000 && longest > 9) return rows < 6144;
-  constexpr int line[9] = {0, 0, 4600, 3600, 2900, 3200, 3600, 1500, 1500};
-  return nnzb < (long)line[b] * longest;
+  if (traffic >= 100000000) return rows < (b == 8 ? 3584 : b == 7 ? 4608 : 6144);
+  constexpr int few[9] = {0, 0, 5000, 2500, 3000, 2500, 3000, 1800, 2000};  // blocks a row: below 7,
+  constexpr int some[9] = {0, 0, 6000, 3600, 3700, 3200, 3400, 2300, 1900};  // to 13,
+  constexpr int many[9] = {0, 0, 6500, 5500, 4600, 4400, 3900, 3000, 2000};  // more
+  if (nnzb <= 0) return rows < few[b];  // (unknown)
+  if (longest <= 0) longest = (int)((nnzb + rows - 1) / rows);
+  const int line = longest < 7 ? few[b] : longest < 14 ? some[b] : many[b];
+  return nnzb < (long)line * longest;
 }
 template <int B, bool RES>
 __global__ void __launch_bounds__(128) k_bsr_spmv_w(int nbr, const int* __restrict__ ptr,
